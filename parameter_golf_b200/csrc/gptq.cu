@@ -1,11 +1,19 @@
-// GPTQ row kernel: column-by-column quantisation with Hessian error feedback, one warp per weight row.
+// GPTQ row kernel: column-by-column quantisation with Hessian error feedback, GQ_ROWS weight rows per CTA.
 //
 // Inputs are what the host prepared once per matrix: the column-permuted weights Wp [rows, cols] (activation order),
 // the upper Cholesky factor U [cols, cols] of the inverse permuted Hessian, and one fixed scale per row (one clip
 // candidate; the caller loops over candidates and keeps the best per row).  Rows are independent, so the only serial
-// dimension is the column index; the row lives in shared memory and the current 128-column block in registers
-// (4 per lane), column values are broadcast with shuffles, the rank-1 feedback inside the block reads U from a shared
-// 128x128 tile and the feedback to the columns right of the block is a 128-term dot product per column.
+// dimension is the column index, and what bounds the kernel is the chain of dependent operations along it.
+//   * One warp per row walks a 128-column block (4 values per lane in registers, the current one broadcast with a shuffle,
+//     the rank-1 feedback reads U from a shared 128x128 tile). The two divisions of a column sit on the chain: each is a
+//     multiplication by a reciprocal and two fused corrections (`div_rn`) instead of the general routine.
+//   * The block's 128 errors must reach every column right of it. The next block needs them at once (`near`: all 16 warps,
+//     one column of one row per thread); the columns beyond are updated by the other 12 warps while the 4 row warps already
+//     walk the next block (`far`), so that phase and the fetch of the next diagonal tile are off the chain. An element of U is
+//     loaded once per CTA and used for all four rows.
+// Four rows per CTA spread 512 rows over 128 SMs. The form with eight rows per CTA, in which every warp also did the far
+// updates of its row by itself, took 2.42 ms at 512 x 1536 (6-bit); four rows with near and far update in one phase between two
+// blocks 0.53 ms; this one 0.35 ms.
 // The arithmetic inside a block is written with explicitly rounded operations (no fused multiply-add) so that the
 // codes match the float32 reference except where the two summation orders of the trailing update differ.
 //
@@ -19,79 +27,177 @@
 namespace pgb {
 
 namespace {
-constexpr int GQ_WARPS = 8;
+constexpr int GQ_ROWS = 4;
+constexpr int GQ_THREADS = 512;
+constexpr int GQ_FAR_THREADS = GQ_THREADS - 32 * GQ_ROWS;
 constexpr int GQ_BLOCK = 128;
+constexpr int GQ_TILE = GQ_BLOCK * GQ_BLOCK;
 
-__device__ __forceinline__ float round_half_away(float x) { return copysignf(floorf(fabsf(x) + 0.5f), x); }
+// sign(x) floor(|x| + 1/2). Codes are clamped to 8 bits, so larger magnitudes may stop at 1024; below 2^23 adding and
+// subtracting 2^23 with the first addition rounded down is a floor (two additions where `floorf` is a slower conversion).
+__device__ __forceinline__ float round_half_away(float x) {
+  const float t = fminf(__fadd_rn(fabsf(x), 0.5f), 1024.f);
+  return copysignf(__fsub_rn(__fadd_rd(t, 8388608.f), 8388608.f), x);
+}
 
-__global__ void __launch_bounds__(GQ_WARPS * 32)
+// a / b rounded to nearest, given r = 1 / b rounded to nearest: a first quotient, its exact remainder, one correction
+// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990, theorem on division
+// with a correctly rounded reciprocal). Holds away from overflow and underflow of the quotient and the remainder.
+__device__ __forceinline__ float div_rn(float a, float b, float r) {
+  const float q = __fmul_rn(a, r);
+  return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+}
+
+// One row's walk over a block of 128 columns (`WHOLE`) or the last nb < 128 columns: without the end test of the ragged form
+// the shared-memory reads of later columns move ahead of the dependency chain.
+template <bool WHOLE>
+__device__ __forceinline__ void walk_block(const float* __restrict__ tile, const float* __restrict__ sR, const float* w_row, int8_t* q_row, float* e_row,
+                                           int lane, int nb, float s, float rs, float qmin, float qmax) {
+  float reg[4];
+#pragma unroll
+  for (int ii = 0; ii < 4; ++ii) {
+    const int c = ii * 32 + lane;
+    reg[ii] = (WHOLE || c < nb) ? w_row[c] : 0.f;
+  }
+#pragma unroll
+  for (int ii = 0; ii < 4; ++ii) {
+    float my_q = 0.f, my_e = 0.f;
+#pragma unroll 8
+    for (int jj = 0; jj < 32; ++jj) {
+      const int j = ii * 32 + jj;
+      if (!WHOLE && j >= nb) break;                                        // uniform across the warp
+      const float* u_row = tile + j * GQ_BLOCK;
+      const float w = __shfl_sync(0xffffffffu, reg[ii], jj);
+      const float q = fminf(fmaxf(round_half_away(div_rn(w, s, rs)), qmin), qmax);
+      const float err = div_rn(__fsub_rn(w, __fmul_rn(q, s)), u_row[j], sR[j]);
+      if (lane == jj) {
+        my_q = q;
+        my_e = err;
+      }
+#pragma unroll
+      for (int i2 = 0; i2 < 4; ++i2)
+        if (i2 >= ii) {
+          // columns left of j are finished: what the upper triangle's zeros would subtract from them is never read again
+          const int c = i2 * 32 + lane;
+          reg[i2] = __fsub_rn(reg[i2], __fmul_rn(err, u_row[c]));
+        }
+    }
+    const int c = ii * 32 + lane;
+    if (WHOLE || c < nb) {
+      q_row[c] = (int8_t)my_q;
+      e_row[c] = my_e;
+    }
+  }
+}
+
+template <int BYTES>
+__device__ __forceinline__ void gq_copy(float* smem_dst, const float* gmem_src, bool valid) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(gmem_src), "n"(BYTES), "r"(valid ? BYTES : 0) : "memory");
+}
+
+__global__ void __launch_bounds__(GQ_THREADS)
 gptq_rows_kernel(const float* __restrict__ Wp, const float* __restrict__ U, const float* __restrict__ scales, int8_t* __restrict__ Q, int rows,
                  int cols, float qmin, float qmax) {
-  extern __shared__ float sm[];
-  float* sU = sm;                                   // [128][128] diagonal tile of U
-  float* sW = sU + GQ_BLOCK * GQ_BLOCK;             // [warps][cols] working rows
-  float* sE = sW + GQ_WARPS * cols;                 // [warps][128] scaled errors of the current block
+  extern __shared__ __align__(16) float sm[];
+  float* sU = sm;                                   // 2 diagonal tiles of U, [128][128] each
+  float* sR = sU + 2 * GQ_TILE;                     // [128] reciprocals of the current tile's diagonal
+  float* sE = sR + GQ_BLOCK;                        // 2 x [rows][128] scaled errors of a block
+  float* sW = sE + 2 * GQ_ROWS * GQ_BLOCK;          // [rows][cols] working rows
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * GQ_WARPS + warp;
-  const bool active = row < rows;
-  float* w_row = sW + warp * cols;
-  float* e_row = sE + warp * GQ_BLOCK;
-  if (active)
-    for (int c = lane; c < cols; c += 32) w_row[c] = Wp[(size_t)row * cols + c];
-  const float s = active ? scales[row] : 1.f;
+  const int row0 = blockIdx.x * GQ_ROWS;
+  const int live = min(GQ_ROWS, rows - row0);
+  const float* src = Wp + (size_t)row0 * cols;
+  for (int i = threadIdx.x; i < GQ_ROWS * cols; i += GQ_THREADS) sW[i] = i < live * cols ? src[i] : 0.f;
+  for (int i = threadIdx.x; i < 2 * GQ_ROWS * GQ_BLOCK; i += GQ_THREADS) sE[i] = 0.f;
+  const bool wide = (cols & 3) == 0 && (reinterpret_cast<uintptr_t>(U) & 15) == 0;      // rows of U start on 16-byte boundaries
+  auto load_tile = [&](int i1, int t, int threads) {     // elements outside the matrix read as zero
+    const int nb = min(GQ_BLOCK, cols - i1);
+    float* dst = sU + ((i1 / GQ_BLOCK) & 1) * GQ_TILE;
+    if (wide) {
+      for (int idx = t * 4; idx < GQ_TILE; idx += threads * 4) {
+        const int j = idx >> 7, c = idx & 127;
+        const bool in = j < nb && c < nb;
+        gq_copy<16>(dst + idx, in ? U + (size_t)(i1 + j) * cols + i1 + c : U, in);
+      }
+    } else {
+      for (int idx = t; idx < GQ_TILE; idx += threads) {
+        const int j = idx >> 7, c = idx & 127;
+        const bool in = j < nb && c < nb;
+        gq_copy<4>(dst + idx, in ? U + (size_t)(i1 + j) * cols + i1 + c : U, in);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load_tile(0, threadIdx.x, GQ_THREADS);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x < min(GQ_BLOCK, cols)) sR[threadIdx.x] = __frcp_rn(sU[threadIdx.x * (GQ_BLOCK + 1)]);
+  __syncthreads();
+  const float s = warp < live ? scales[row0 + warp] : 1.f;
+  const float rs = __frcp_rn(s);
   for (int i1 = 0; i1 < cols; i1 += GQ_BLOCK) {
     const int nb = min(GQ_BLOCK, cols - i1);
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < GQ_BLOCK * GQ_BLOCK; idx += blockDim.x) {
-      const int j = idx >> 7, c = idx & 127;
-      sU[idx] = (j < nb && c < nb) ? U[(size_t)(i1 + j) * cols + i1 + c] : 0.f;
-    }
-    __syncthreads();
-    if (!active) continue;
-    float reg[4];
+    const int buf = (i1 / GQ_BLOCK) & 1;
+    if (warp < GQ_ROWS) {
+      if (warp < live) {
+        const float* tile = sU + buf * GQ_TILE;
+        float* e_row = sE + (buf * GQ_ROWS + warp) * GQ_BLOCK;
+        const float* w_row = sW + warp * cols + i1;
+        int8_t* q_row = Q + (size_t)(row0 + warp) * cols + i1;
+        if (nb == GQ_BLOCK) walk_block<true>(tile, sR, w_row, q_row, e_row, lane, nb, s, rs, qmin, qmax);
+        else walk_block<false>(tile, sR, w_row, q_row, e_row, lane, nb, s, rs, qmin, qmax);
+      }
+    } else {
+      const int t = threadIdx.x - 32 * GQ_ROWS;
+      if (i1 + GQ_BLOCK < cols) load_tile(i1 + GQ_BLOCK, t, GQ_FAR_THREADS);
+      if (i1 > 0) {
+        // far: the previous block's errors into the columns beyond this block, w[r][c] -= sum_j err[r][j] * U[j][c]
+        const float* e_prev = sE + (buf ^ 1) * GQ_ROWS * GQ_BLOCK;
+        for (int c = i1 + GQ_BLOCK + t; c < cols; c += GQ_FAR_THREADS) {
+          float a[GQ_ROWS][4] = {};
+          const float* u = U + (size_t)(i1 - GQ_BLOCK) * cols + c;
+#pragma unroll 4
+          for (int j = 0; j < GQ_BLOCK; j += 4) {
+            const float u0 = __ldg(u + (size_t)j * cols), u1 = __ldg(u + (size_t)(j + 1) * cols), u2 = __ldg(u + (size_t)(j + 2) * cols),
+                        u3 = __ldg(u + (size_t)(j + 3) * cols);
 #pragma unroll
-    for (int ii = 0; ii < 4; ++ii) {
-      const int c = ii * 32 + lane;
-      reg[ii] = c < nb ? w_row[i1 + c] : 0.f;
-    }
-#pragma unroll
-    for (int ii = 0; ii < 4; ++ii) {
-      for (int jj = 0; jj < 32; ++jj) {
-        const int j = ii * 32 + jj;
-        if (j >= nb) break;                                            // uniform across the warp
-        const float w = __shfl_sync(0xffffffffu, reg[ii], jj);
-        const float q = fminf(fmaxf(round_half_away(__fdiv_rn(w, s)), qmin), qmax);
-        const float err = __fdiv_rn(__fsub_rn(w, __fmul_rn(q, s)), sU[j * GQ_BLOCK + j]);
-        if (lane == jj) {
-          Q[(size_t)row * cols + i1 + j] = (int8_t)q;
-          e_row[j] = err;
-        }
-        const float* u_row = sU + j * GQ_BLOCK;
-#pragma unroll
-        for (int i2 = 0; i2 < 4; ++i2) {
-          if (i2 >= ii) {
-            const int c = i2 * 32 + lane;
-            if (c >= j) reg[i2] = __fsub_rn(reg[i2], __fmul_rn(err, u_row[c]));
+            for (int r = 0; r < GQ_ROWS; ++r) {
+              const float4 e = *reinterpret_cast<const float4*>(e_prev + r * GQ_BLOCK + j);
+              a[r][0] = fmaf(e.x, u0, a[r][0]);
+              a[r][1] = fmaf(e.y, u1, a[r][1]);
+              a[r][2] = fmaf(e.z, u2, a[r][2]);
+              a[r][3] = fmaf(e.w, u3, a[r][3]);
+            }
           }
+#pragma unroll
+          for (int r = 0; r < GQ_ROWS; ++r) sW[r * cols + c] -= (a[r][0] + a[r][1]) + (a[r][2] + a[r][3]);
         }
       }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
-    __syncwarp();
-    // feedback to every column right of the block: w[c] -= sum_j err[j] * U[i1 + j][c]
-    for (int c = i1 + nb + lane; c < cols; c += 32) {
-      float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-      const float* u = U + (size_t)i1 * cols + c;
-      int j = 0;
-      for (; j + 4 <= nb; j += 4) {
-        a0 = fmaf(e_row[j], u[(size_t)j * cols], a0);
-        a1 = fmaf(e_row[j + 1], u[(size_t)(j + 1) * cols], a1);
-        a2 = fmaf(e_row[j + 2], u[(size_t)(j + 2) * cols], a2);
-        a3 = fmaf(e_row[j + 3], u[(size_t)(j + 3) * cols], a3);
+    __syncthreads();                                // this block's errors, the far updates and the next tile are visible
+    if (i1 + GQ_BLOCK >= cols) break;
+    {
+      // near: this (whole) block's errors into the next block's columns
+      const int r = threadIdx.x >> 7, cc = threadIdx.x & 127, c = i1 + GQ_BLOCK + cc;
+      if (r == 0 && c < cols) sR[cc] = __frcp_rn(sU[(buf ^ 1) * GQ_TILE + cc * (GQ_BLOCK + 1)]);
+      if (c < cols) {
+        const float* e_row = sE + (buf * GQ_ROWS + r) * GQ_BLOCK;
+        const float* u = U + (size_t)i1 * cols + c;
+        float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll 8
+        for (int j = 0; j < GQ_BLOCK; j += 4) {
+          const float4 e = *reinterpret_cast<const float4*>(e_row + j);
+          a0 = fmaf(e.x, __ldg(u + (size_t)j * cols), a0);
+          a1 = fmaf(e.y, __ldg(u + (size_t)(j + 1) * cols), a1);
+          a2 = fmaf(e.z, __ldg(u + (size_t)(j + 2) * cols), a2);
+          a3 = fmaf(e.w, __ldg(u + (size_t)(j + 3) * cols), a3);
+        }
+        sW[r * cols + c] -= (a0 + a1) + (a2 + a3);
       }
-      for (; j < nb; ++j) a0 = fmaf(e_row[j], u[(size_t)j * cols], a0);
-      w_row[c] -= (a0 + a1) + (a2 + a3);
     }
-    __syncwarp();
+    __syncthreads();
   }
 }
 }  // namespace
@@ -99,8 +205,9 @@ gptq_rows_kernel(const float* __restrict__ Wp, const float* __restrict__ U, cons
 void gptq_rows(const float* Wp, const float* U, const float* scales, int8_t* Q, int rows, int cols, int bits, cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return;
   if (bits < 2 || bits > 8) throw std::runtime_error("gptq_rows: bits must be in 2..8");
-  const size_t smem = ((size_t)GQ_BLOCK * GQ_BLOCK + (size_t)GQ_WARPS * cols + GQ_WARPS * GQ_BLOCK) * sizeof(float);
-  if (smem > 227 * 1024) throw std::runtime_error("gptq_rows: rows of more than " + std::to_string((227 * 1024 / 4 - GQ_BLOCK * GQ_BLOCK - GQ_WARPS * GQ_BLOCK) / GQ_WARPS) + " columns do not fit in shared memory");
+  constexpr size_t fixed = 2 * (size_t)GQ_TILE + GQ_BLOCK + 2 * GQ_ROWS * GQ_BLOCK;
+  const size_t smem = (fixed + (size_t)GQ_ROWS * cols) * sizeof(float);
+  if (smem > 227 * 1024) throw std::runtime_error("gptq_rows: rows of more than " + std::to_string((227 * 1024 / 4 - fixed) / GQ_ROWS) + " columns do not fit in shared memory");
   static size_t configured[64] = {};        // largest size set so far, per device (the attribute is a per-device property)
   int dev = 0;
   cudaGetDevice(&dev);
@@ -109,7 +216,7 @@ void gptq_rows(const float* Wp, const float* U, const float* scales, int8_t* Q, 
     if (dev >= 0 && dev < 64) configured[dev] = smem;
   }
   const float qmax = (float)((1 << (bits - 1)) - 1), qmin = -(float)(1 << (bits - 1));
-  gptq_rows_kernel<<<(rows + GQ_WARPS - 1) / GQ_WARPS, GQ_WARPS * 32, smem, st>>>(Wp, U, scales, Q, rows, cols, qmin, qmax);
+  gptq_rows_kernel<<<(rows + GQ_ROWS - 1) / GQ_ROWS, GQ_THREADS, smem, st>>>(Wp, U, scales, Q, rows, cols, qmin, qmax);
 }
 
 }  // namespace pgb

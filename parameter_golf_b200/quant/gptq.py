@@ -35,10 +35,13 @@ def gptq_prepare(H: torch.Tensor, damping: float = 0.01):
     """Return (perm, inv_perm, U) with ``U`` the upper Cholesky factor of ``inv(H[perm][:, perm])``."""
     Hd = damp_hessian(H, damping)
     perm = torch.argsort(torch.diagonal(Hd), descending=True)
-    Hp = Hd[perm][:, perm].double()
-    L = torch.linalg.cholesky(Hp)
-    Hinv = torch.cholesky_inverse(L)
-    U = torch.linalg.cholesky(Hinv, upper=True).float()
+    # inv(H) = U^T U with U upper means H = R R^T with R = inv(U) upper, and R is the Cholesky factor of H with its rows and
+    # columns in reverse order, reversed back. So one factorisation and one triangular inverse give the (unique) factor; neither
+    # inv(H) nor its own factorisation is needed.
+    rev = perm.flip(0)
+    L = torch.linalg.cholesky(Hd[rev][:, rev].double())
+    eye = torch.eye(L.shape[0], dtype=L.dtype, device=L.device)
+    U = torch.linalg.solve_triangular(L, eye, upper=False).flip(0, 1).float()
     return perm, torch.argsort(perm), U
 
 
@@ -93,7 +96,7 @@ def gptq_quantize(W: torch.Tensor, H: torch.Tensor, bits: int = 6, block: int = 
         better = err < best_err
         best_err = torch.where(better, err, best_err)
         best_s = torch.where(better, scale, best_s)
-        best_q[better] = Q[better]
+        best_q = torch.where(better[:, None], Q, best_q)
     return best_q[:, inv_perm].contiguous(), best_s
 
 

@@ -53,3 +53,29 @@ def test_gptq_quantize_uses_the_kernel_on_cuda_tensors():
     q_ref, s_ref = gptq_quantize(W, H, bits=6, rows_fn=gptq_rows_torch)
     assert torch.allclose(s, s_ref)
     assert ((q.int() - q_ref.int()).abs() > 0).float().mean() < 0.01
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 127), (5, 129), (4, 256), (6, 390), (9, 1288)])
+def test_gptq_rows_at_the_edges_of_its_blocks(rows, cols):
+    """Row counts around the four rows of a CTA and column counts around the 128-column blocks (one ragged block, a whole one, a
+    one-column rest, widths off 16 bytes): the codes of the float32 statement up to rounding-boundary flips, which the summation
+    order of the trailing update can cause and which then propagate through that row alone."""
+    from parameter_golf_b200.ops import native as n
+    from parameter_golf_b200.quant.gptq import gptq_prepare, gptq_rows_torch
+    W, H = _problem(rows, cols, 7 * rows + cols)
+    perm, _, U = gptq_prepare(H)
+    Wp = W[:, perm].contiguous()
+    scale = (Wp.abs().amax(1) / 31).clamp_min(1e-8)
+    want, got = gptq_rows_torch(Wp, U, scale, 6), n.gptq_rows(Wp, U, scale, 6)
+    diff = (got.int() - want.int()).abs()
+    assert diff.max() <= 1 and int((diff > 0).sum()) <= max(2, rows * cols // 100)
+
+
+def test_gptq_prepare_gives_the_upper_factor_of_the_inverse():
+    from parameter_golf_b200.quant.gptq import damp_hessian, gptq_prepare
+    _, H = _problem(4, 192, 11)
+    perm, inv_perm, U = gptq_prepare(H)
+    Hp = damp_hessian(H)[perm][:, perm].double()
+    want = torch.linalg.cholesky(torch.cholesky_inverse(torch.linalg.cholesky(Hp)), upper=True)
+    assert torch.equal(perm[inv_perm], torch.arange(192, device=perm.device)) and float(U.tril(-1).abs().max()) == 0.0
+    assert float((U.double() - want).norm() / want.norm()) < 1e-6          # one rounding to fp32: 2^-24 per element
