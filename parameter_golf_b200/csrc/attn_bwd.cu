@@ -136,7 +136,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   // the data-movement warpgroup hands most of its registers to the two softmax warpgroups (128 live values per thread)
   asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       long long tg = 0;                     // key tiles loaded by this CTA so far
       int il = 0;                           // items handled by this CTA so far
       bool ok = true;
@@ -163,7 +163,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     }
   } else if (warp == 1) {
     // scores: S(j) and dP(j) as soon as the previous tile's scores have been pulled into registers
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_S = make_idesc_bf16(128, 128, 0, 0);    // Q K^T, dO V^T
       long long tg = 0;
       int il = 0;
@@ -191,7 +191,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     }
   } else if (warp == 2) {
     // dQ += dS K once both softmax groups have stored their halves of dS
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_DQ = make_idesc_bf16(128, 64, 0, 1);    // dS (TMEM) x K, K read N(=hd)-contiguous
       long long tg = 0;
       int il = 0;
@@ -410,7 +410,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   // the data-movement warpgroup hands most of its registers to the two softmax warpgroups (128 live values per thread)
   asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       uint32_t item_par = 0;
       long long ubase = 0;
@@ -445,7 +445,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     }
   } else if (warp == 1) {
     // scores: S^T(u) and dP^T(u) as soon as the previous unit's scores have been pulled into registers
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_T = make_idesc_bf16(128, 128, 0, 0);    // K Q^T and V dO^T
       const uint32_t sk = smem_u32(sK), sv = smem_u32(sV);
       bool ok = true;
@@ -473,7 +473,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     }
   } else if (warp == 2) {
     // gradients: dV += P^T dO and dK += dS^T Q once both softmax groups have stored their halves of P^T / dS^T
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_A = make_idesc_bf16(128, 64, 0, 1);     // A from TMEM; B (dO, Q) read N(=hd)-contiguous
       bool ok = true;
       uint32_t item_par = 0;

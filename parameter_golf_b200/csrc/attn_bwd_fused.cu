@@ -218,7 +218,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     // the data-movement warpgroup hands most of its registers to the softmax warpgroups
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(F_REGS_MOVE));
     if (warp == 0) {
-      if (lane == 0) {
+      if (elect_one()) {
         bool ok = true;
         UnitPos up;
         int il = 0;
@@ -252,7 +252,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       }
     } else if (warp == 1) {
       // scores: S^T(u) and dP^T(u) as soon as the previous unit's scores have been pulled into registers
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t IDESC_T = make_idesc_bf16(128, 128, 0, 0);    // K Q^T and V dO^T
         bool ok = true;
         UnitPos up;
@@ -288,7 +288,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       }
     } else if (warp == 2) {
       // gradients, once every softmax group has stored its part of P^T (tensor memory) and dS^T (shared memory)
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t IDESC_DV = make_idesc_bf16(128, 64, 0, 1);    // A = P^T from TMEM; B = dO read N(=hd)-contiguous
         constexpr uint32_t IDESC_DK = make_idesc_bf16(128, 64, 0, 1);    // A = dS^T K-major (rows = keys); B = Q read N-contiguous
         constexpr uint32_t IDESC_DQ = make_idesc_bf16(128, 64, 1, 1);    // A = dS^T read MN-major (M = queries); B = K read N-contiguous

@@ -162,7 +162,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(A1_REG_ROLE));
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
       // ---- TMA producer ----
       int ks = 0, vs = 0;
       uint32_t kph = 0, vph = 0, ic = 0, q_issued = 0;
@@ -203,7 +203,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         for (int s = 0; s < A1_KST; ++s) mbar_drain(&k_full[s], (s < ks) ? kph : (kph ^ 1));
         for (int s = 0; s < A1_VST; ++s) mbar_drain(&v_full[s], (s < vs) ? vph : (vph ^ 1));
       }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
       // ---- score products: S = Q K^T as soon as K has landed and the previous scores have been pulled into registers ----
       constexpr uint32_t IDESC_S = make_idesc_bf16(128, 128, 0, 0);    // both operands K-major
       int ks = 0;
@@ -232,7 +232,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
         umma_commit(&q_empty[slot]);
       }
-    } else if (warp == 2 && lane == 0) {
+    } else if (warp == 2 && elect_one()) {
       // ---- O += P V: its own issuing thread, so that a score product never queues behind a wait for probabilities ----
       constexpr uint32_t IDESC_O = make_idesc_bf16(128, AT_HD, 0, 1);  // A from TMEM, V is N-contiguous
       int vs = 0;

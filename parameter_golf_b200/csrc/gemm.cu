@@ -386,7 +386,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -459,8 +459,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC = make_idesc_bf16(BM, BN, A_KMAJOR ? 0 : 1, B_KMAJOR ? 0 : 1);
+      // operand descriptors of stage 0; a stage or K step only adds to their address field
+      const uint64_t da0 = A_KMAJOR ? make_smem_desc(smem_u32(smem), 16, 1024) : make_smem_desc(smem_u32(smem), 8192, 1024);
+      const uint64_t db0 = B_KMAJOR ? make_smem_desc(smem_u32(smem) + S::A_BYTES, 16, 1024) : make_smem_desc(smem_u32(smem) + S::A_BYTES, 8192, 1024);
+      constexpr uint32_t A_STEP = (A_KMAJOR ? 32 : 2048) >> 4, B_STEP = (B_KMAJOR ? 32 : 2048) >> 4;
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -477,14 +481,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, ST_WAIT_FULL, kb)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * S::STAGE_BYTES);
-          const uint32_t sb = sa + S::A_BYTES;
+          const uint32_t at = (uint32_t)stage * (S::STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t da = A_KMAJOR ? make_smem_desc(sa + k * 32, 16, 1024) : make_smem_desc(sa + k * 2048, 8192, 1024);
-            const uint64_t db = B_KMAJOR ? make_smem_desc(sb + k * 32, 16, 1024) : make_smem_desc(sb + k * 2048, 8192, 1024);
-            umma_ss(tmem_d, da, db, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / 16; ++k) umma_ss(tmem_d, da0 + at + k * A_STEP, db0 + at + k * B_STEP, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
           umma_commit(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
