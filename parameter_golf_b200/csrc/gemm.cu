@@ -15,8 +15,8 @@
 // CTA = 10 warps: warp 0 issues TMA loads, warp 1 owns TMEM and issues the MMAs (one elected lane),
 // warps 2..9 read the accumulator back (tcgen05.ld, one row per thread) and run the epilogue. Two
 // accumulators (2 x BN TMEM columns) let the epilogue of tile i overlap the main loop of tile i+1.
-// Tile 128 x BN x 64, BN in {128, 256}; grid = min(#tiles, #SMs); tile index = n fastest so CTAs
-// working at the same time share the rows of the large operand in L2.
+// Tile 128 x BN x 64, BN in {64, 128, 256} (`pick_tile`); grid = min(#tiles, #SMs); tile index = n fastest so CTAs
+// working at the same time share the rows of the large operand in L2. The 64-column form has four epilogue warps (6 warps in all).
 #include "common.cuh"
 #include "pgb.h"
 #include "tma_host.h"
@@ -25,7 +25,9 @@ namespace pgb {
 
 constexpr int BM = 128;
 constexpr int BK = 64;
-constexpr int GEMM_THREADS = 320;     // TMA warp, MMA warp, 8 epilogue warps (two per TMEM lane quarter)
+// TMA warp, MMA warp, epilogue warps: two per TMEM lane quarter (one for 64 columns, so that a warp still owns whole heads)
+constexpr int epi_warps(int bn) { return bn == 64 ? 4 : 8; }
+constexpr int gemm_threads(int bn) { return 64 + 32 * epi_warps(bn); }
 
 struct GemmKernelParams {
   int M, N, K, batch;
@@ -62,9 +64,9 @@ struct GemmSmem {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN == 256) ? 4 : 6;
+  static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128) ? 6 : 8;
   static constexpr int TILE_BYTES = STAGES * STAGE_BYTES;
-  static constexpr int STG_BYTES = 8 * 2 * STG_WARP_BYTES;
+  static constexpr int STG_BYTES = epi_warps(BN) * 2 * STG_WARP_BYTES;
   static constexpr int TOTAL = TILE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + STG_BYTES;
 };
 
@@ -338,12 +340,12 @@ __device__ __forceinline__ void epilogue_qkv_head_staged(const GemmKernelParams&
 }
 
 template <int BN, bool A_KMAJOR, bool B_KMAJOR, int EPI>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(gemm_threads(BN), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_x, const GemmKernelParams p) {
   using S = GemmSmem<BN>;
   constexpr int STAGES = S::STAGES;
-  constexpr uint32_t TMEM_COLS = 2 * BN;            // 256 or 512: two accumulators
+  constexpr uint32_t TMEM_COLS = 2 * BN;            // 128, 256 or 512: two accumulators
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::TILE_BYTES);
@@ -363,7 +365,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 256);
+      mbar_init(&tempty_bar[a], 32 * epi_warps(BN));
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -493,7 +495,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..9)
+    // ------------------------------------------------------------------ epilogue (warps 2..9; 2..5 for 64 columns)
     const int quarter = warp & 3;                 // TMEM lane quarter this warp may access
     const int half = (warp - 2) >> 2;             // which half of the tile's columns
     uint8_t* slots = smem + S::TILE_BYTES + 256 + (warp - 2) * 2 * STG_WARP_BYTES;
@@ -504,7 +506,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint32_t acc_phase = 0;
     bool ok = true;
     constexpr bool HAS_AUX = (EPI == EPI_AXPBY_BF16 || EPI == EPI_RESID_BF16 || EPI == EPI_MUL_ACTGRAD);
-    constexpr int CH = BN / 64;                   // 32-column chunks per epilogue warp (the two warps of a quarter split the columns)
+    constexpr int CH = BN / 8 / epi_warps(BN);    // 32-column chunks per epilogue warp (the warps of a quarter split the columns)
     constexpr bool BF16_OUT = !(EPI == EPI_F32 || EPI == EPI_F32_ATOMIC);
     const int c_begin = half * CH;
     auto tile_coords = [&](int tile, int& b, int& tm, int& tn) {
@@ -665,7 +667,7 @@ static void launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const C
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  kern<<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL, stream>>>(ma, mb, mx, p);
+  kern<<<grid, gemm_threads(BN), GemmSmem<BN>::TOTAL, stream>>>(ma, mb, mx, p);
 }
 
 template <int BN, int EPI>
@@ -673,6 +675,7 @@ static void launch_major(const GemmArgs& a, const CUtensorMap& ma, const CUtenso
                          cudaStream_t stream) {
   if (a.a_kmajor && a.b_kmajor) launch_variant<BN, true, true, EPI>(ma, mb, mx, p, grid, stream);
   else if (a.a_kmajor && !a.b_kmajor) launch_variant<BN, true, false, EPI>(ma, mb, mx, p, grid, stream);
+  else if constexpr (BN == 64) throw std::runtime_error("gemm: 64-column tiles take row-major activations");
   else if (!a.a_kmajor && a.b_kmajor) launch_variant<BN, false, true, EPI>(ma, mb, mx, p, grid, stream);
   else launch_variant<BN, false, false, EPI>(ma, mb, mx, p, grid, stream);
 }
@@ -680,12 +683,17 @@ static void launch_major(const GemmArgs& a, const CUtensorMap& ma, const CUtenso
 template <int BN>
 static void launch_epi(const GemmArgs& a, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mx, const GemmKernelParams& p, int grid,
                        cudaStream_t stream) {
+  if constexpr (BN != 64) {
+    switch (a.epi) {
+      case EPI_F32: launch_major<BN, EPI_F32>(a, ma, mb, mx, p, grid, stream); return;
+      case EPI_F32_ATOMIC: launch_major<BN, EPI_F32_ATOMIC>(a, ma, mb, mx, p, grid, stream); return;
+      case EPI_RESID_BF16: launch_major<BN, EPI_RESID_BF16>(a, ma, mb, mx, p, grid, stream); return;
+      default: break;
+    }
+  }
   switch (a.epi) {
     case EPI_BF16: launch_major<BN, EPI_BF16>(a, ma, mb, mx, p, grid, stream); break;
-    case EPI_F32: launch_major<BN, EPI_F32>(a, ma, mb, mx, p, grid, stream); break;
-    case EPI_F32_ATOMIC: launch_major<BN, EPI_F32_ATOMIC>(a, ma, mb, mx, p, grid, stream); break;
     case EPI_AXPBY_BF16: launch_major<BN, EPI_AXPBY_BF16>(a, ma, mb, mx, p, grid, stream); break;
-    case EPI_RESID_BF16: launch_major<BN, EPI_RESID_BF16>(a, ma, mb, mx, p, grid, stream); break;
     case EPI_ACT_SQ: launch_major<BN, EPI_ACT_SQ>(a, ma, mb, mx, p, grid, stream); break;
     case EPI_MUL_ACTGRAD: launch_major<BN, EPI_MUL_ACTGRAD>(a, ma, mb, mx, p, grid, stream); break;
     case EPI_QKV_NORM_ROPE:
@@ -696,36 +704,59 @@ static void launch_epi(const GemmArgs& a, const CUtensorMap& ma, const CUtensorM
   }
 }
 
-void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
-  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.batch <= 0) throw std::runtime_error("gemm: empty problem");
-  if ((a.lda % 8) || (a.ldb % 8)) throw std::runtime_error("gemm: leading dimensions must be multiples of 8 elements");
-  const int bn = (a.N > 128) ? 256 : 128;
-  GemmKernelParams p;
-  p.M = a.M; p.N = a.N; p.K = a.K; p.batch = a.batch;
-  p.tiles_m = (a.M + BM - 1) / BM;
-  p.tiles_n = (a.N + bn - 1) / bn;
-  p.kb_total = (a.K + BK - 1) / BK;
-  int splits = a.splits;
-  if (splits <= 0) {
-    splits = 1;
-    if (a.epi == EPI_F32_ATOMIC) {
-      // Fill the machine when the output is small and K is long, in whole waves: with `base` output tiles, base * splits
-      // work items run in ceil(items / SMs) rounds, so 2 * SMs + a few items would cost a third round for nothing.
-      // Two rounds are preferred (the second tile's main loop hides the first one's epilogue), then one, then three.
-      const int base = p.tiles_m * p.tiles_n * a.batch, sms = num_sms();
-      const int max_splits = std::max(1, p.kb_total / 8);
-      double best_eff = 0.0;
-      for (int waves : {2, 1, 3}) {
-        const int sp = std::min(max_splits, std::max(1, waves * sms / base));
-        const int items = base * sp;
-        const double eff = (double)items / ((double)((items + sms - 1) / sms) * sms);
-        if (eff > best_eff + 0.02) {
-          best_eff = eff;
-          splits = sp;
-        }
+struct TilePlan {
+  int bn, splits;
+};
+
+// Tile width and number of K splits by estimated time, in SM clocks. An item (one tile, one K split) costs 540 / 285 / 245 clocks
+// per 64-deep K step of a 256 / 128 / 64 column tile (a 64-column MMA is bound by its operand reads) plus an epilogue; a round of
+// items beyond the first costs 0.8 of that, since a main loop overlaps the epilogue before it. The constants were fitted to
+// products of 1024 to 98,304 rows on the model's sites and order the widths as measured there (us, 256 / 128 / 64 columns):
+//   M = 2048,  N = 512,  K = 512   7.7 / 5.6 / 5.0       M = 4096, N = 512, K = 1536   12.5 / 8.9 / 11.0
+//   M = 5760,  N = 512,  K = 1536  12.8 / 13.5 / 14.3    M = 98304, N = 1024, K = 512  99 / 111 / 134
+// A narrower tile has to win by 8 %: it reads the activations from L2 more often than the model counts.
+// Weight gradients (fp32 adds): every split adds a whole tile to the output in L2 (~52 clocks per column), so one round with as many
+// splits as fill the SMs beats two rounds (512x1536 from 4096 rows: 3 splits of 128-column tiles 10.4 us, 6 splits 12.3; from
+// 98,304 rows 6 splits of 256 columns 118 us, 12 splits 122), and narrow tiles win while the sum is short.
+static TilePlan pick_tile(const GemmArgs& a, int tiles_m, int kb_total, int sms) {
+  TilePlan best{0, 1};
+  double best_cost = 0.0;
+  const bool atomic = a.epi == EPI_F32_ATOMIC;
+  for (int bn : {256, 128, 64}) {
+    if (a.tile_n > 0 && bn != a.tile_n) continue;
+    if (a.tile_n <= 0 && bn == 256 && a.N <= 128) continue;
+    if (bn == 64 && (!a.a_kmajor || a.epi == EPI_F32 || a.epi == EPI_RESID_BF16 || atomic)) continue;
+    const int base = tiles_m * ((a.N + bn - 1) / bn) * a.batch;
+    const double step = bn == 256 ? 540.0 : bn == 128 ? 285.0 : 245.0;
+    const double epi = atomic ? 52.0 * bn : bn == 256 ? 4900.0 : bn == 128 ? 2900.0 : 2000.0;
+    int last = 0;
+    for (int waves : {1, 2, 3}) {
+      int splits = std::max(1, a.splits);
+      if (atomic && a.splits <= 0) splits = std::min(std::max(1, kb_total / 4), std::max(1, waves * sms / base));
+      if (splits == last) continue;
+      last = splits;
+      const int rounds = (base * splits + sms - 1) / sms;
+      const double cost = (step * ((kb_total + splits - 1) / splits) + epi) * (1.0 + 0.8 * (rounds - 1));
+      if (best.bn == 0 || cost < 0.92 * best_cost) {
+        best = {bn, splits};
+        best_cost = cost;
       }
     }
   }
+  if (best.bn == 0) throw std::runtime_error("gemm: no tile of this width for this product");
+  return best;
+}
+
+void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
+  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.batch <= 0) throw std::runtime_error("gemm: empty problem");
+  if ((a.lda % 8) || (a.ldb % 8)) throw std::runtime_error("gemm: leading dimensions must be multiples of 8 elements");
+  GemmKernelParams p;
+  p.M = a.M; p.N = a.N; p.K = a.K; p.batch = a.batch;
+  p.tiles_m = (a.M + BM - 1) / BM;
+  p.kb_total = (a.K + BK - 1) / BK;
+  const TilePlan plan = pick_tile(a, p.tiles_m, p.kb_total, num_sms());
+  const int bn = plan.bn, splits = plan.splits;
+  p.tiles_n = (a.N + bn - 1) / bn;
   if (splits > 1 && a.epi != EPI_F32_ATOMIC) throw std::runtime_error("gemm: split-K needs the atomic fp32 epilogue");
   p.kb_per_split = (p.kb_total + splits - 1) / splits;
   p.splits = (p.kb_total + p.kb_per_split - 1) / p.kb_per_split;
@@ -769,7 +800,8 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
                        (reinterpret_cast<uintptr_t>(a.aux) & 15) == 0 && total > grid) ? 1 : 0;
   const CUtensorMap mx = p.aux_l2_prefetch ? operand_map(a.aux, true, a.M, a.N, a.ld_aux, a.stride_aux, a.batch, BM) : ma;
   if (bn == 256) launch_epi<256>(a, ma, mb, mx, p, grid, stream);
-  else launch_epi<128>(a, ma, mb, mx, p, grid, stream);
+  else if (bn == 128) launch_epi<128>(a, ma, mb, mx, p, grid, stream);
+  else launch_epi<64>(a, ma, mb, mx, p, grid, stream);
 }
 
 }  // namespace pgb

@@ -36,6 +36,7 @@ struct GemmArgs {
   long long stride_a = 0, stride_b = 0, stride_d = 0, stride_aux = 0; // batch strides in elements
   int epi = EPI_BF16;
   int splits = 0;            // 0 = automatic
+  int tile_n = 0;            // output tile columns (64, 128 or 256); 0 = automatic
   float alpha = 1.f, beta = 0.f, slope = 0.f;
   int* status = nullptr;     // device status word (4 ints) or null
   const int* wait_flag = nullptr;   // optional readiness counter for B (see comm.cu); polled with a bounded wait

@@ -183,3 +183,31 @@ def test_qkv_product_with_norm_rope_and_gain_in_its_output_stage(T, d, H, Hkv, r
         q_ref, k_ref = R.qk_norm_rope_gain(qf, kf, cos, sin, rope, gain, eps)
         _close(post[:, :H * hd], q_ref.reshape(T, H * hd))
         _close(post[:, H * hd:qk], k_ref.reshape(T, Hkv * hd))
+
+
+@pytest.mark.parametrize("tile_n", [64, 128, 256])
+@pytest.mark.parametrize("M,N,K", [(128, 64, 64), (129, 200, 72), (640, 512, 1536), (2500, 328, 136)])
+def test_every_tile_width_gives_the_same_product(tile_n, M, N, K):
+    """Each output tile width against fp32, for every epilogue it carries, on whole and ragged tiles. bf16 results: one rounding
+    (2^-9 relative) plus fp32 sums, within the 1e-2 of the other product tests."""
+    n = _n()
+    torch.manual_seed(M + N + K + tile_n)
+    A, W, Wt, aux = _rand(M, K), _rand(N, K, scale=K ** -0.5), _rand(K, N, scale=K ** -0.5), _rand(M, N)
+    ref, ref_t = _ref(A, W, True, True), _ref(A, Wt, True, False)
+    D, D2 = (torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    n.gemm(A, W, D, tile_n=tile_n)
+    _close(D, ref)
+    n.gemm(A, Wt, D, True, False, tile_n=tile_n)
+    _close(D, ref_t)
+    n.gemm(A, W, D, epi=n.EPI_AXPBY_BF16, alpha=0.5, beta=2.0, aux=aux, tile_n=tile_n)
+    _close(D, 0.5 * ref + 2.0 * aux.float())
+    n.gemm(A, W, D, epi=n.EPI_ACT_SQ, slope=0.5, D2=D2, tile_n=tile_n)
+    _close(D, ref)
+    _close(D2, torch.nn.functional.leaky_relu(D.float(), 0.5).square())
+    n.gemm(A, Wt, D, True, False, n.EPI_MUL_ACTGRAD, slope=0.5, aux=aux, tile_n=tile_n)
+    _close(D, ref_t * 2.0 * torch.where(aux.float() >= 0, aux.float(), 0.25 * aux.float()))
+    torch.cuda.synchronize()
+    n.check_status()
+    if tile_n == 64:
+        with pytest.raises(RuntimeError, match="no tile of this width"):
+            n.gemm(A, W, torch.empty(M, N, device="cuda"), epi=n.EPI_F32, tile_n=64)
