@@ -20,7 +20,12 @@
 // Scheduling: work items are (batch, KV head, key tile); key tiles j and n-1-j of one (batch, KV head) are handed to the
 // same CTA one after the other, so every CTA-level item has the same length, and items are numbered (batch, KV head)
 // first so that the CTAs running at any time add into a few MB of the accumulator, which therefore stays in L2 between
-// the contributions of different key tiles.
+// the contributions of different key tiles. Only whole rounds of items (one per SM) run that way. The items left over
+// would keep a few SMs busy for a whole item; their units (plus one per key tile for loading K/V and storing dK/dV) are cut into
+// equal contiguous ranges, one per CTA, at most two of whose key tiles are shared with a neighbour. A shared tile's dK/dV go to a
+// per-CTA fp32 slot and attn_bwd_merge_kernel adds the slots in CTA order, so dK and dV stay independent of timing.
+// Longest CTA in units (H = 8, Hkv = 4, S = 2048, 148 SMs), whole items against this split: B = 1 36 / 9, B = 2 36 / 17,
+// B = 8 72 / 64, B = 48 396 / 375.
 //
 // The per-query terms ride on the tensor core. P^T = exp2(c S^T - lse[q]) and dS^T = P^T (dP^T - D[q]) need one lse and one
 // D per query COLUMN of the transposed tiles, i.e. every thread would need every value: broadcast loads from shared memory
@@ -109,6 +114,10 @@ __device__ __forceinline__ int bias_row_off(int r) { return (r >> 3) * 256 + (r 
 struct FusedParams {
   int B, S, H, Hkv, n_qt, group;
   int n_pairs, n_super;          // key-tile pairs per (batch, KV head); CTA-level items
+  int whole;                     // rounds of whole items per CTA; the rest is split by units
+  int w_pair, w_bk;              // weight (units + 1 per key tile) of an ordinary pair and of all pairs of one (batch, KV head)
+  int rest_base, rest_w;         // position of item `rest0` and total weight of the rest (0: nothing is split)
+  float* part;                   // [2 * grid] slots of {dK, dV} partial tiles, each 16 x 128 x 4 floats: first and last tile of a CTA's range
   float scale, scale_log2;
   const float* lse;              // [B, H, S]  -(log2-domain log-sum-exp)
   const float* Dsum;             // [B, H, S]  -rowsum(dO * O)
@@ -120,20 +129,58 @@ struct FusedParams {
   int* status;
 };
 
-struct FItem { int j, b, kvh, nu, key0; };
+// key tile j of (b, kvh): units u0 .. u0 + nu - 1 of it, a unit being (query tile >= j, head of the group), heads fastest
+struct FItem { int j, b, kvh, nu, key0, u0, slot; };       // slot: where a shared tile's dK/dV go (-1: the tile is this CTA's alone)
 
-// The seq-th item of this CTA: 0 = valid, 1 = nothing at this position (odd tile count, middle tile already done), 2 = end.
+// Position of item `super` when the units of all items are laid out one after the other.
+__device__ __forceinline__ int f_pos(const FusedParams& p, int super) {
+  const int bk = super / p.n_pairs;
+  return bk * p.w_bk + (super - bk * p.n_pairs) * p.w_pair;
+}
+__device__ __forceinline__ int f_range_start(const FusedParams& p, int cta, int ctas) {
+  return p.rest_base + (int)((long long)cta * p.rest_w / ctas);
+}
+// item that position `pos` falls into
+__device__ __forceinline__ int f_super_at(const FusedParams& p, int pos) {
+  const int bk = pos / p.w_bk;
+  return bk * p.n_pairs + min((pos - bk * p.w_bk) / p.w_pair, p.n_pairs - 1);
+}
+
+// The seq-th item of this CTA: 0 = valid, 1 = nothing at this position, 2 = end.
 __device__ __forceinline__ int f_decode(const FusedParams& p, int seq, FItem& it) {
-  const int super = (int)blockIdx.x + (seq >> 1) * (int)gridDim.x;
-  if (super >= p.n_super) return 2;
+  const int round = seq >> 1;
+  int super, lo = 0, hi = 0;
+  const bool split = round >= p.whole;
+  if (!split) {
+    super = (int)blockIdx.x + round * (int)gridDim.x;
+    if (super >= p.n_super) return 2;
+  } else {
+    if (p.rest_w == 0) return 2;
+    lo = f_range_start(p, (int)blockIdx.x, (int)gridDim.x);
+    hi = f_range_start(p, (int)blockIdx.x + 1, (int)gridDim.x);
+    super = f_super_at(p, lo) + round - p.whole;
+    if (lo >= hi || super >= p.n_super || f_pos(p, super) >= hi) return 2;
+  }
   const int bk = super / p.n_pairs, pr = super - bk * p.n_pairs;
   const int j = (seq & 1) ? p.n_qt - 1 - pr : pr;
-  if ((seq & 1) && j == pr) return 1;
+  if ((seq & 1) && j == pr) return 1;                  // odd tile count, middle tile already done
+  const int nu = (p.n_qt - j) * p.group;
   it.j = j;
   it.b = bk / p.Hkv;
   it.kvh = bk - it.b * p.Hkv;
-  it.nu = (p.n_qt - j) * p.group;        // units: (query tile >= j, head of the group)
+  it.nu = nu;
+  it.u0 = 0;
+  it.slot = -1;
   it.key0 = it.b * p.S + j * 128;
+  if (split) {
+    const int first = f_pos(p, super) + ((seq & 1) ? (p.n_qt - pr) * p.group + 1 : 0) + 1;      // position of the tile's first unit
+    const int u0 = max(0, lo - first), u1 = min(nu, hi - first);
+    if (u1 <= u0) return 1;
+    it.u0 = u0;
+    it.nu = u1 - u0;
+    if (u0 > 0) it.slot = 2 * (int)blockIdx.x;
+    else if (u1 < nu) it.slot = 2 * (int)blockIdx.x + 1;
+  }
   return 0;
 }
 
@@ -233,7 +280,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
           mbar_expect_tx(&kv_full[kvb], 2 * F_TILE);
           f_tma2d(sk, &map_k, &kv_full[kvb], it.kvh * F_HD, it.key0);
           f_tma2d(sk + F_TILE, &map_v, &kv_full[kvb], it.kvh * F_HD, it.key0);
-          int head = it.kvh * p.group, qi = it.j, g = 0;
+          int g = it.u0 % p.group, head = it.kvh * p.group + g, qi = it.j + it.u0 / p.group;
           for (int u = 0; u < it.nu; ++u, up.next()) {
             const int stage = up.stage;
             if (!mbar_wait(&st_empty[stage], up.phase ^ 1, abort_flag, p.status, ST_WAIT_EMPTY, u, F_BACKOFF_NS)) { ok = false; break; }
@@ -345,7 +392,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const int rc = f_decode(p, seq, it);
         if (rc == 2) break;
         if (rc == 1) continue;
-        int head = it.kvh * p.group, qi = it.j, g = 0;
+        int g = it.u0 % p.group, head = it.kvh * p.group + g, qi = it.j + it.u0 / p.group;
         for (int u = 0; u < it.nu; ++u, up.next()) {
           const int stage = up.stage;
           const size_t vidx = ((size_t)it.b * p.H + head) * p.S + qi * 128 + lane * 4;
@@ -395,7 +442,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       if (rc == 2) break;
       if (rc == 1) continue;
       const int j = it.j, kvh = it.kvh, key0 = it.key0, nu = it.nu;
-      int head = kvh * p.group, qi = j, g = 0;
+      int g = it.u0 % p.group, head = kvh * p.group + g, qi = j + it.u0 / p.group;
       float* dq_blk = p.dq_acc + (((size_t)it.b * p.H + head) * p.n_qt + qi) * 8192;
       for (int u = 0; u < nu; ++u, up.next()) {
         const int stage = up.stage;
@@ -488,6 +535,14 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_empty);     // the values are in registers: the next key tile may start accumulating
+        if (it.slot >= 0) {
+          float4* dst = reinterpret_cast<float4*>(p.part) + ((size_t)it.slot * 2 + (is_dk ? 0 : 1)) * 2048 + (col0 / 4) * 128 + kk;
+#pragma unroll
+          for (int c = 0; c < EC; c += 4)
+            dst[(c / 4) * 128] = make_float4(__uint_as_float(v[c]), __uint_as_float(v[c + 1]), __uint_as_float(v[c + 2]), __uint_as_float(v[c + 3]));
+          ++il;
+          continue;
+        }
 #pragma unroll
         for (int c = 0; c < EC; c += 8) {
           float f[8];
@@ -523,6 +578,50 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// dK/dV of the key tiles whose units two or more CTAs shared: CTA c handles the tile in which range c starts, if range c is the
+// first to start inside it. Contributions are the previous range's last-tile slot and the first-tile slots from range c on.
+__global__ void __launch_bounds__(256) attn_bwd_merge_kernel(const FusedParams p, int ctas) {
+  const int c = (int)blockIdx.x + 1;
+  const int lo = f_range_start(p, c, ctas);
+  if (lo >= p.rest_base + p.rest_w) return;
+  const int super = f_super_at(p, lo);
+  const int bk = super / p.n_pairs, pr = super - bk * p.n_pairs;
+  const int n0 = (p.n_qt - pr) * p.group;
+  int j = pr, first = f_pos(p, super) + 1, nu = n0;
+  if (lo >= first + n0 && pr != p.n_qt - 1 - pr) {
+    j = p.n_qt - 1 - pr;
+    first += n0 + 1;
+    nu = (p.n_qt - j) * p.group;
+  }
+  if (lo <= first || lo >= first + nu) return;                           // the range starts between tiles
+  if (f_range_start(p, c - 1, ctas) > first) return;                     // an earlier range starts inside this tile
+  const int b = bk / p.Hkv, kvh = bk - b * p.Hkv, key0 = b * p.S + j * 128;
+  const float4* part = reinterpret_cast<const float4*>(p.part);
+  {
+    const int i = blockIdx.y * 256 + threadIdx.x;                        // (dK | dV, row, 8 columns), 2 x 128 x 8 over grid.y
+    const int oc = i & 7, r = (i >> 3) & 127, which = i >> 10;
+    const size_t off = (size_t)which * 2048 + oc * 256 + r;
+    float4 x0 = part[(size_t)(2 * (c - 1) + 1) * 4096 + off], x1 = part[(size_t)(2 * (c - 1) + 1) * 4096 + off + 128];
+    for (int k = c; k < ctas && f_range_start(p, k, ctas) < first + nu; ++k) {
+      if (f_range_start(p, k, ctas) == f_range_start(p, k + 1, ctas)) continue;      // fewer units than CTAs: an empty range
+      const float4 y0 = part[(size_t)(2 * k) * 4096 + off], y1 = part[(size_t)(2 * k) * 4096 + off + 128];
+      x0.x += y0.x; x0.y += y0.y; x0.z += y0.z; x0.w += y0.w;
+      x1.x += y1.x; x1.y += y1.y; x1.z += y1.z; x1.w += y1.w;
+    }
+    float f[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    __nv_bfloat16* out = (which ? p.dv + (size_t)(key0 + r) * p.lddv : p.dk + (size_t)(key0 + r) * p.lddk) + kvh * F_HD + oc * 8;
+    const float mul = which ? 1.f : p.scale;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] *= mul;
+    if (which && p.accumulate_dv) {
+      const uint4 q = *reinterpret_cast<const uint4*>(out);
+      const float2 a0 = unpack_bf16x2(q.x), a1 = unpack_bf16x2(q.y), a2 = unpack_bf16x2(q.z), a3 = unpack_bf16x2(q.w);
+      f[0] += a0.x; f[1] += a0.y; f[2] += a1.x; f[3] += a1.y; f[4] += a2.x; f[5] += a2.y; f[6] += a3.x; f[7] += a3.y;
+    }
+    *reinterpret_cast<uint4*>(out) = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
   }
 }
 
@@ -593,13 +692,22 @@ CUtensorMap fused_map(const void* ptr, long long ld, int cols, long long rows) {
 
 size_t attn_bwd_fused_scratch_floats(int B, int S, int H) { return (size_t)B * H * S * F_HD; }
 
+static int bwd_sms() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+size_t attn_bwd_fused_part_floats() { return (size_t)bwd_sms() * 2 * 2 * 8192; }
+
 void attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse, float* dsum, float* dq_acc, void* dq,
                     void* dk, void* dv, long long ldq, long long ldk, long long ldv, long long ldo, long long lddo, long long lddq, long long lddk,
-                    long long lddv, int B, int S, int H, int Hkv, int hd, int accumulate_dv, int* status, cudaStream_t st, int dsum_ready) {
+                    long long lddv, int B, int S, int H, int Hkv, int hd, int accumulate_dv, int* status, cudaStream_t st, int dsum_ready, float* part,
+                    const QkNormRopeBwd* qk) {
   if (hd != F_HD) throw std::runtime_error("attention kernel is specialised for head_dim 64");
   if (S % 128) throw std::runtime_error("attention kernel needs seq_len to be a multiple of 128");
   if (H % Hkv) throw std::runtime_error("attention: the number of KV heads must divide the number of query heads");
-  if ((ldo % 8) || (lddo % 8) || (lddq % 8) || (lddk % 8) || (lddv % 8)) throw std::runtime_error("attention: row strides must be multiples of 8 elements");
+  if ((ldo % 8) || (lddo % 8) || (dq && (lddq % 8)) || (lddk % 8) || (lddv % 8)) throw std::runtime_error("attention: row strides must be multiples of 8 elements");
   const long long T = (long long)B * S;
   FusedParams p;
   p.B = B; p.S = S; p.H = H; p.Hkv = Hkv;
@@ -614,9 +722,26 @@ void attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, 
   p.lddk = lddk; p.lddv = lddv;
   p.accumulate_dv = accumulate_dv;
   p.status = status;
-  int dev = 0, sms = 148;
+  const int sms = bwd_sms();
+  const int grid = part ? sms : std::min(p.n_super, sms);
+  p.part = part;
+  p.w_pair = (p.n_qt + 1) * p.group + 2;
+  p.w_bk = p.w_pair * (p.n_pairs - 1) + (p.n_qt % 2 ? p.n_pairs * p.group + 1 : p.w_pair);
+  p.whole = (p.n_super + grid - 1) / grid;
+  p.rest_base = p.rest_w = 0;
+  if (part) {
+    // Split the last, partly filled round when that shortens the longest CTA by more than two units (what the shared tiles' slots and
+    // the merge cost; a round that is nearly full is left as it is).
+    const int full = p.n_super / grid * grid;
+    const long long end = (long long)B * Hkv * p.w_bk, base = (long long)(full / p.n_pairs) * p.w_bk + (long long)(full % p.n_pairs) * p.w_pair;
+    if (full < p.n_super && end < 0x7fffffffll && (end - base) / grid + 2 < p.w_pair) {
+      p.whole = full / grid;
+      p.rest_base = (int)base;
+      p.rest_w = (int)(end - base);
+    }
+  }
+  int dev = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   static bool configured[64] = {};          // the attribute is a per-device property of the kernel
   if (dev < 0 || dev >= 64 || !configured[dev]) {
     cudaFuncSetAttribute(attn_bwd_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM);
@@ -627,8 +752,10 @@ void attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, 
     attn_bwd_prep_kernel<<<(unsigned)((n_chunks + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, ldo, lddo, dsum, T, S, H);
   const CUtensorMap mq = fused_map(q, ldq, H * hd, T), mk = fused_map(k, ldk, Hkv * hd, T), mv = fused_map(v, ldv, Hkv * hd, T),
                     mdo = fused_map(d_o, lddo, H * hd, T);
-  attn_bwd_fused_kernel<<<std::min(p.n_super, sms), F_THREADS, F_SMEM, st>>>(mq, mk, mv, mdo, p);
-  attn_bwd_finish_kernel<<<B * H * p.n_qt, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, lddq, S, H, p.n_qt, p.scale);
+  attn_bwd_fused_kernel<<<std::min(grid, p.rest_w ? grid : p.n_super), F_THREADS, F_SMEM, st>>>(mq, mk, mv, mdo, p);
+  if (p.rest_w) attn_bwd_merge_kernel<<<dim3(grid - 1, 8), 256, 0, st>>>(p, grid);
+  if (qk) qk_norm_rope_bwd64_acc(dq_acc, *qk, (int)T, H, Hkv, S, p.scale, st);
+  else attn_bwd_finish_kernel<<<B * H * p.n_qt, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, lddq, S, H, p.n_qt, p.scale);
 }
 
 }  // namespace pgb

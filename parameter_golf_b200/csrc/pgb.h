@@ -102,6 +102,20 @@ void mix_norm_bwd_v2(const void* d_h, const void* d_res, const void* x_in, const
 bool qk_norm_rope_fast_ok(int H, int hd, int rope_dims);
 void qk_norm_rope_fwd64(const void* src, void* dst, const float* cosT, const float* sinT, const float* gain, int rows, int ld, int H, int Hkv,
                         int rope_dims, int seq_len, float eps, cudaStream_t st);
+// d_post holds the key heads' gradient (columns H*64 on), d_pre receives query and key heads; all three share the row pitch `ld`
+struct QkNormRopeBwd {
+  const void* d_post = nullptr;
+  const void* pre = nullptr;
+  void* d_pre = nullptr;
+  const float* cosT = nullptr;
+  const float* sinT = nullptr;
+  const float* gain = nullptr;
+  float* d_gain = nullptr;
+  int ld = 0, rope_dims = 0;
+  float eps = 0.f;
+};
+// queries' gradient = scale * the attention backward's accumulator (zeroed here)
+void qk_norm_rope_bwd64_acc(float* dq_acc, const QkNormRopeBwd& a, int rows, int H, int Hkv, int seq_len, float scale, cudaStream_t st);
 void qk_norm_rope_bwd64(const void* d_post, const void* pre, void* d_pre, const float* cosT, const float* sinT, const float* gain, float* d_gain,
                         int rows, int ld, int H, int Hkv, int rope_dims, int seq_len, float eps, cudaStream_t st);
 
@@ -174,6 +188,11 @@ void attn_bwd(const void* q, const void* k, const void* v, const void* o, const 
 size_t attn_bwd_fused_scratch_floats(int B, int S, int H);
 void attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse, float* dsum, float* dq_acc, void* dq,
                     void* dk, void* dv, long long ldq, long long ldk, long long ldv, long long ldo, long long lddo, long long lddq, long long lddk,
-                    long long lddv, int B, int S, int H, int Hkv, int hd, int accumulate_dv, int* status, cudaStream_t st, int dsum_ready = 0);
+                    long long lddv, int B, int S, int H, int Hkv, int hd, int accumulate_dv, int* status, cudaStream_t st, int dsum_ready = 0,
+                    float* part = nullptr, const QkNormRopeBwd* qk = nullptr);
+// `part` (attn_bwd_fused_part_floats() floats, no initial value needed) lets the last, partly filled round of work be split evenly over
+// the SMs. With `qk` the accumulator goes through the backward of the per-head norm and rotation (qk_norm_rope_bwd64_acc) instead
+// of into `dq`, which may be null; qk->d_post + H * 64 must be `dk`.
+size_t attn_bwd_fused_part_floats();
 
 }  // namespace pgb

@@ -334,6 +334,108 @@ void qk_norm_rope_bwd64(const void* d_post, const void* pre, void* d_pre, const 
                                                   d_gain, nvec, ld, H, Hkv, rope_dims, seq_len, eps);
 }
 
+// The same backward with the queries' gradient taken from the fp32 accumulator of the single-pass attention backward, which is left
+// zeroed for the next call: the accumulator's own pass (scale, round to bf16, zero) and the bf16 copy it wrote are gone, and the
+// gradient reaches the rotation unrounded. Bound by DRAM: per query head vector 256 B of accumulator read and 256 B zeroed, 128 B of
+// projection read, 128 B written. Accumulator blocks are [16 column chunks][128 rows][4 floats] per (batch, head, 128-row query
+// tile); a CTA takes one block (or 128 rows of a key head), reads it in its own order, 512 contiguous bytes per warp, and turns
+// it into rows through shared memory. (Without that step, eight lanes per row reading their chunks from the block in place, 64
+// contiguous bytes at a time, the kernel took 1398 us at B = 48, S = 2048 instead of @@.)
+constexpr int QKA_PITCH = 68;                              // floats per staged row: 64 + 4, so that rows start in different banks
+__global__ void __launch_bounds__(256) qk_norm_rope_bwd64_acc_kernel(float* __restrict__ dq_acc, const __nv_bfloat16* __restrict__ d_post,
+                                                                     const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __restrict__ d_pre,
+                                                                     const float* __restrict__ cosT, const float* __restrict__ sinT,
+                                                                     const float* __restrict__ gain, float* __restrict__ d_gain, int ld, int H, int Hkv,
+                                                                     int rope_dims, int seq_len, float eps, float scale) {
+  __shared__ __align__(16) float tile[128 * QKA_PITCH];
+  __shared__ float sg[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7;
+  const int nh = H + Hkv, half = rope_dims / 2, hp = half / 8, n_qt = seq_len >> 7;
+  const int rt = (int)((unsigned)blockIdx.x / (unsigned)nh), head = (int)blockIdx.x - rt * nh;       // 128-row tile, head
+  const int b = (int)((unsigned)rt / (unsigned)n_qt), qi = rt - b * n_qt;
+  const bool query = head < H;
+  const size_t off0 = ((size_t)rt * 128 + (threadIdx.x >> 3)) * ld + head * 64 + sub * 8;
+  float4* blk = reinterpret_cast<float4*>(dq_acc) + (((size_t)b * H + head) * n_qt + qi) * 2048 + threadIdx.x;       // queries only
+  uint4 xq[4], dq[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) xq[i] = ldraw(pre + off0 + (size_t)i * 32 * ld);
+  if (query) {
+    float4 a[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = __ldcg(blk + i * 256);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int idx = i * 256 + threadIdx.x;               // chunk idx / 128 (4 columns), row idx % 128
+      *reinterpret_cast<float4*>(tile + (idx & 127) * QKA_PITCH + (idx >> 7) * 4) = a[i];
+    }
+    __syncthreads();
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dq[i] = ldraw(d_post + off0 + (size_t)i * 32 * ld);
+  }
+  const float g = (query && gain) ? gain[head] : 1.f;
+  float dg = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = i * 32 + (threadIdx.x >> 3);
+    V8 dy;
+    if (query) {
+      const float4 a0 = *reinterpret_cast<const float4*>(tile + r * QKA_PITCH + sub * 8), a1 = *reinterpret_cast<const float4*>(tile + r * QKA_PITCH + sub * 8 + 4);
+      dy.v[0] = a0.x * scale; dy.v[1] = a0.y * scale; dy.v[2] = a0.z * scale; dy.v[3] = a0.w * scale;
+      dy.v[4] = a1.x * scale; dy.v[5] = a1.y * scale; dy.v[6] = a1.z * scale; dy.v[7] = a1.w * scale;
+    } else {
+      dy = cvt8(dq[i]);
+    }
+    const V8 x = cvt8(xq[i]);
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss += x.v[e] * x.v[e];
+    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 4);
+    const float ms = ss / 64.f + eps;
+    const float inv = rsqrtf(ms);
+    if (hp > 0) rope8(dy, sub, hp, qi * 128 + r, half, cosT, sinT, true);
+    float dot = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) dot += x.v[e] * dy.v[e];
+    dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+    dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+    dot += __shfl_xor_sync(0xffffffffu, dot, 4);
+    dg += dot * inv;                                       // the same in all eight lanes of a row
+    const float k2 = g * dot / (ms * 64.f), gi = g * inv;
+    V8 o;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o.v[e] = gi * dy.v[e] - inv * x.v[e] * k2;
+    stv(d_pre + off0 + (size_t)i * 32 * ld, o);
+  }
+  if (query) {                                             // every load of the block was consumed before the barrier above
+#pragma unroll
+    for (int i = 0; i < 8; ++i) blk[i * 256] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (d_gain != nullptr && query) {                        // uniform over the CTA
+    dg += __shfl_xor_sync(0xffffffffu, dg, 8);
+    dg += __shfl_xor_sync(0xffffffffu, dg, 16);
+    if (lane == 0) sg[warp] = dg;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float t = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) t += sg[i];
+      atomicAdd(d_gain + head, t);
+    }
+  }
+}
+
+void qk_norm_rope_bwd64_acc(float* dq_acc, const QkNormRopeBwd& a, int rows, int H, int Hkv, int seq_len, float scale, cudaStream_t st) {
+  if (!qk_norm_rope_fast_ok(H, 64, a.rope_dims)) throw std::runtime_error("qk_norm_rope: shape outside the head_dim 64 kernel");
+  if (seq_len <= 0 || seq_len % 128 || rows % seq_len) throw std::runtime_error("qk_norm_rope: whole sequences of a multiple of 128 tokens only");
+  if ((long long)rows * (H + Hkv) > 0x7fffff00ll) throw std::runtime_error("qk_norm_rope: too many head vectors for 32-bit indexing");
+  qk_norm_rope_bwd64_acc_kernel<<<rows / 128 * (H + Hkv), 256, 0, st>>>(dq_acc, (const __nv_bfloat16*)a.d_post, (const __nv_bfloat16*)a.pre,
+                                                                        (__nv_bfloat16*)a.d_pre, a.cosT, a.sinT, a.gain, a.d_gain, a.ld, H, Hkv, a.rope_dims,
+                                                                        seq_len, a.eps, scale);
+}
+
 // ---- XSA forward / backward, head_dim 64, 8 lanes per (token, KV head) ------------------------------------------------------
 // z_h = y_h - (<y_h, v> / (|v|^2 + eps)) v for the `group` query heads h that share one value head. A lane holds 8 of the 64
 // features (one 16-byte load, 128 contiguous bytes per head vector), the three inner products are 8-lane shuffles, and no

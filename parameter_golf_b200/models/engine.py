@@ -319,6 +319,7 @@ class CudaEngine:
             self.dsum = torch.empty(self.B, self.H, self.S, dtype=torch.float32, device=dev)
             # fp32 dQ accumulator of the single-pass attention backward: zero between calls (the kernels restore that)
             self.dq_acc = None if self.t.reproducible_backward else torch.zeros(self.B * self.H * self.S * self.hd, dtype=torch.float32, device=dev)
+            self.bwd_part = None if self.t.reproducible_backward else N.attn_bwd_part(dev)
             self.d_skip = [buf(T, d) for _ in range(max(self.enc - 1, 0))] if self.unet else []
             self.d_xe = buf(T, d)
             if m.bigram.enabled:
@@ -459,7 +460,16 @@ class CudaEngine:
         self.lse[li] = N.attn_fwd(q, k, v, self.y[li], B, S, H, Hkv, hd, self.lse[li], z, 1e-8)
 
     def _attn_bwd(self, l, j):
+        """Attention backward and the backward of the per-head norm, rotation and query gain: ``d_qkv_pre`` is complete afterwards."""
         d, kv, B, S, H, Hkv, hd = self.d, self.kv, self.B, self.S, self.H, self.Hkv, self.hd
+        m = self.m
+        gain, d_gain = self.p["q_gain"][l], self.g["q_gain"][l]
+        if self.dq_acc is not None and hd == 64 and H <= 64 and m.rope_dims % 16 == 0 and m.rope_dims <= 64:
+            # the attention kernel's fp32 query accumulator feeds the norm / rotation backward directly
+            xsa = l in m.xsa_layers()
+            self.C.attn_bwd_qk(self.qk_post[j], self.qkv_pre[j], self.y[j], self.d_y, self.lse[j], self.dsum, self.dq_acc, self.d_qk_post, self.d_qkv_pre,
+                               self.cos, self.sin, gain, d_gain, B, S, H, Hkv, m.rope_dims, self.eps, xsa, N.status_word(self.dev), xsa, self.bwd_part)
+            return
         q = self.qk_post[j][:, :d]
         k = self.qk_post[j][:, d:d + kv]
         v = self.qkv_pre[j][:, d + kv:]
@@ -469,6 +479,7 @@ class CudaEngine:
         # in XSA layers `xsa_bwd` has just produced d_y and, in the same pass, the -rowsum(d_y * y) term of the single-pass form
         N.attn_bwd(q, k, v, self.y[j], self.d_y, self.lse[j], dq, dk, dv, B, S, H, Hkv, hd, accumulate_dv=xsa, dsum=self.dsum,
                    dq_acc=self.dq_acc, reproducible=self.t.reproducible_backward, dsum_ready=xsa and not self.t.reproducible_backward)
+        self.C.qk_norm_rope_bwd(self.d_qk_post, self.qkv_pre[j], self.d_qkv_pre, self.cos, self.sin, gain, d_gain, H, Hkv, hd, m.rope_dims, S, self.eps)
 
     def _block_fwd(self, j: int, x, skip, sw, recompute: bool = False):
         """Block of activation slot ``j`` on input ``x`` (with the U-Net skip it consumes, if any); returns the block output.
@@ -659,8 +670,6 @@ class CudaEngine:
                 else:
                     C.xsa_bwd(self.d_z, self.y[aj], vview, self.d_y, dv, False, self.Hkv, self.H // self.Hkv, self.hd, 1e-8, self.dsum, S)
             self._attn_bwd(l, aj)
-            C.qk_norm_rope_bwd(self.d_qk_post, self.qkv_pre[aj], self.d_qkv_pre, self.cos, self.sin, p["q_gain"][l], g["q_gain"][l], self.H, self.Hkv,
-                               self.hd, m.rope_dims, S, self.eps)
             if m.value_embedding.enabled and l in m.value_embedding.layers:
                 vi = m.value_embedding.layers.index(l)
                 self.Gvp.zero_()

@@ -46,7 +46,8 @@ def load():
 class _Counting:
     """Forwards to the extension and counts kernel launches issued through it (`launch_count`)."""
 
-    _PER_CALL = {"attn_bwd": 2, "attn_bwd_fused": 3}
+    _PER_CALL = {"attn_bwd": 2, "attn_bwd_fused": 4, "attn_bwd_qk": 4}
+    _DSUM_READY = {"attn_bwd_fused": 18, "attn_bwd_qk": 21}       # position of that argument
 
     def __init__(self, mod):
         self._mod = mod
@@ -55,11 +56,11 @@ class _Counting:
 
     def __getattr__(self, name):
         fn = getattr(self._mod, name)
-        n = self._PER_CALL.get(name, 1)
+        n, skip = self._PER_CALL.get(name, 1), self._DSUM_READY.get(name)
 
         def call(*a, **k):
             # the single-pass attention backward skips its first kernel when the caller supplies the per-query term
-            self.launches += n - 1 if (name == "attn_bwd_fused" and len(a) >= 19 and a[18]) else n
+            self.launches += n - 1 if (skip is not None and len(a) > skip and a[skip]) else n
             if self.timing is None:
                 return fn(*a, **k)
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -208,8 +209,14 @@ def attn_bwd(q, k, v, o, d_o, lse, dq, dk, dv, B, S, H, Hkv, hd, accumulate_dv=F
         return dsum
     if dq_acc is None:
         dq_acc = attn_dq_scratch(q.device, B, S, H, hd)
-    load().attn_bwd_fused(q, k, v, o, d_o, lse, dsum, dq_acc, dq, dk, dv, B, S, H, Hkv, hd, accumulate_dv, status_word(q.device), dsum_ready)
+    load().attn_bwd_fused(q, k, v, o, d_o, lse, dsum, dq_acc, dq, dk, dv, B, S, H, Hkv, hd, accumulate_dv, status_word(q.device), dsum_ready,
+                          attn_bwd_part(q.device))
     return dsum
+
+
+def attn_bwd_part(device):
+    """Slots for the key tiles that two CTAs of the single-pass attention backward share (no initial value needed)."""
+    return torch.empty(load()._mod.attn_bwd_part_floats(), dtype=torch.float32, device=device)
 
 
 def gptq_rows(Wp, U, scales, bits, block=128):

@@ -217,6 +217,7 @@ def estimate_engine_memory(spec: RunSpec, micro_batch_tokens: int, train: bool =
         scratch += 2 * T * d                                                            # d_xe
         if not t.reproducible_backward:
             scratch += 4 * T * d                                                        # fp32 dQ accumulator of the single-pass attention backward
+            scratch += 148 * 2 * 2 * 4 * 128 * 64                                       # its per-SM slots for shared key tiles (fp32 dK and dV)
         if m.bigram.enabled:
             scratch += 2 * T * m.bigram.dim
         if gates and not m.parallel:

@@ -128,3 +128,49 @@ def test_attention_backward_single_pass_many_tiles_and_clean_scratch():
         for g, r in zip(got, ref):
             err = (g.float() - r.float()).abs().max().item()
             assert err <= 0.01 * r.float().abs().max().item() + 1e-3, err
+
+
+@pytest.mark.parametrize("B,S,H,Hkv,rope", [(1, 128, 2, 1, 16), (2, 2048, 8, 4, 16), (3, 1920, 8, 4, 0), (1, 640, 4, 1, 64), (9, 1024, 8, 4, 32), (5, 384, 3, 3, 16)])
+def test_attention_backward_through_norm_and_rope_in_one_call(B, S, H, Hkv, rope):
+    """The combined backward (fp32 query accumulator straight into the norm / rotation backward, last round of key tiles split over the
+    SMs) against the two-kernel attention backward followed by the row kernel. The split's dK/dV sums are fp32 in CTA order, so two
+    calls agree bit for bit in the value columns; bf16 intermediates of the reference path bound the difference (2^-8 of the largest)."""
+    from parameter_golf_b200.ops import native as n, reference as R
+    C = n.load()
+    hd, T, eps = 64, B * S, 1e-6
+    d, kv = H * hd, Hkv * hd
+    torch.manual_seed(S + H + rope)
+    pre = torch.randn(T, d + 2 * kv, device="cuda").bfloat16()
+    post = torch.zeros_like(pre)
+    gain = torch.rand(H, device="cuda") + 0.75
+    cos = sin = None
+    if rope:
+        cos, sin = (t.contiguous() for t in R.rope_tables(S, rope, 10000.0, device="cuda"))
+    C.qk_norm_rope_fwd(pre, post, cos, sin, gain, H, Hkv, hd, rope, S, eps)
+    q, k, v = post[:, :d], post[:, d:d + kv], pre[:, d + kv:]
+    y, dy = torch.empty(T, d, device="cuda", dtype=torch.bfloat16), (torch.randn(T, d, device="cuda") * 0.5).bfloat16()
+    lse = n.attn_fwd(q, k, v, y, B, S, H, Hkv, hd)
+    base = (torch.randn(T, kv, device="cuda") * 0.1).bfloat16()
+    dsum = torch.empty(B, H, S, device="cuda")
+
+    ref, ref_gain, tmp = torch.empty_like(pre), torch.zeros(H, device="cuda"), torch.zeros_like(pre)
+    ref[:, d + kv:] = base
+    n.attn_bwd(q, k, v, y, dy, lse, tmp[:, :d], tmp[:, d:d + kv], ref[:, d + kv:], B, S, H, Hkv, hd, accumulate_dv=True, reproducible=True)
+    C.qk_norm_rope_bwd(tmp, pre, ref, cos, sin, gain, ref_gain, H, Hkv, hd, rope, S, eps)
+
+    acc = torch.zeros(B * H * S * hd, device="cuda")
+    outs = []
+    for _ in range(2):
+        got, d_gain, d_post = torch.full_like(pre, 7.0), torch.zeros(H, device="cuda"), torch.full_like(pre, 7.0)
+        got[:, d + kv:] = base
+        C.attn_bwd_qk(post, pre, y, dy, lse, dsum, acc, d_post, got, cos, sin, gain, d_gain, B, S, H, Hkv, rope, eps, True, n.status_word(pre.device),
+                      False, n.attn_bwd_part(pre.device))
+        torch.cuda.synchronize()
+        n.check_status()
+        assert float(acc.abs().max()) == 0.0
+        outs.append(got)
+        for lo, hi in ((0, d), (d, d + kv), (d + kv, d + 2 * kv)):
+            r = ref[:, lo:hi].float()
+            assert (got[:, lo:hi].float() - r).abs().max() <= 0.012 * r.abs().max() + 1e-3, (lo, hi)
+        assert (d_gain - ref_gain).abs().max() <= 0.01 * ref_gain.abs().max() + 0.05
+    assert torch.equal(outs[0][:, d:], outs[1][:, d:])
