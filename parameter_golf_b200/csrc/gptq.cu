@@ -1,8 +1,8 @@
-// GPTQ row kernel: column-by-column quantisation with Hessian error feedback, GQ_ROWS weight rows per CTA.
+// GPTQ row kernel: column-by-column quantisation with Hessian error feedback, several weight rows per CTA.
 //
 // Inputs are what the host prepared once per matrix: the column-permuted weights Wp [rows, cols] (activation order),
-// the upper Cholesky factor U [cols, cols] of the inverse permuted Hessian, and one fixed scale per row (one clip
-// candidate; the caller loops over candidates and keeps the best per row).  Rows are independent, so the only serial
+// the upper Cholesky factor U [cols, cols] of the inverse permuted Hessian, and one fixed scale per row and clip candidate (the
+// caller keeps the best candidate per row).  A (row, candidate) pair is a row of its own here.  Rows are independent, so the only serial
 // dimension is the column index, and what bounds the kernel is the chain of dependent operations along it.
 //   * One warp per row walks a 128-column block (4 values per lane in registers, the current one broadcast with a shuffle,
 //     the rank-1 feedback reads U from a shared 128x128 tile). The two divisions of a column sit on the chain: each is a
@@ -14,6 +14,9 @@
 // Four rows per CTA spread 512 rows over 128 SMs. The form with eight rows per CTA, in which every warp also did the far
 // updates of its row by itself, took 2.42 ms at 512 x 1536 (6-bit); four rows with near and far update in one phase between two
 // blocks 0.53 ms; this one 0.35 ms.
+// The chain leaves most issue slots free, so when there are more than four rows per SM (five clip candidates of one matrix) a
+// larger CTA walks up to 20 rows at once, five per scheduler (`gptq_rows`); it holds one diagonal tile instead of two, which is
+// fetched during the near update. Five candidates of 512 x 1536: 1.74 ms as five launches, 0.88 ms as one.
 // The arithmetic inside a block is written with explicitly rounded operations (no fused multiply-add) so that the
 // codes match the float32 reference except where the two summation orders of the trailing update differ.
 //
@@ -27,9 +30,10 @@
 namespace pgb {
 
 namespace {
-constexpr int GQ_ROWS = 4;
-constexpr int GQ_THREADS = 512;
-constexpr int GQ_FAR_THREADS = GQ_THREADS - 32 * GQ_ROWS;
+constexpr int GQ_ROWS = 4;                   // rows of the small form
+constexpr int GQ_MAX_ROWS = 20;              // rows of the large one
+constexpr int GQ_FAR_THREADS = 384;
+constexpr int GQ_GROUP_SMALL = 4, GQ_GROUP_LARGE = 8;      // rows that share one pass over U in the far update
 constexpr int GQ_BLOCK = 128;
 constexpr int GQ_TILE = GQ_BLOCK * GQ_BLOCK;
 
@@ -96,32 +100,36 @@ __device__ __forceinline__ void gq_copy(float* smem_dst, const float* gmem_src, 
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(gmem_src), "n"(BYTES), "r"(valid ? BYTES : 0) : "memory");
 }
 
-__global__ void __launch_bounds__(GQ_THREADS)
+// `rows` counts (candidate, row) pairs, candidate-major; R of them per CTA (one warp each), then 12 warps for the far updates.
+template <int GROUP, int MAX_THREADS, bool TWO_TILES>
+__global__ void __launch_bounds__(MAX_THREADS)
 gptq_rows_kernel(const float* __restrict__ Wp, const float* __restrict__ U, const float* __restrict__ scales, int8_t* __restrict__ Q, int rows,
-                 int cols, float qmin, float qmax) {
+                 int weight_rows, int cols, int R, float qmin, float qmax) {
   extern __shared__ __align__(16) float sm[];
-  float* sU = sm;                                   // 2 diagonal tiles of U, [128][128] each
-  float* sR = sU + 2 * GQ_TILE;                     // [128] reciprocals of the current tile's diagonal
-  float* sE = sR + GQ_BLOCK;                        // 2 x [rows][128] scaled errors of a block
-  float* sW = sE + 2 * GQ_ROWS * GQ_BLOCK;          // [rows][cols] working rows
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row0 = blockIdx.x * GQ_ROWS;
-  const int live = min(GQ_ROWS, rows - row0);
-  const float* src = Wp + (size_t)row0 * cols;
-  for (int i = threadIdx.x; i < GQ_ROWS * cols; i += GQ_THREADS) sW[i] = i < live * cols ? src[i] : 0.f;
-  for (int i = threadIdx.x; i < 2 * GQ_ROWS * GQ_BLOCK; i += GQ_THREADS) sE[i] = 0.f;
+  float* sU = sm;                                   // diagonal tiles of U, [128][128] each: this block's and, with two, the next one's
+  float* sR = sU + (TWO_TILES ? 2 : 1) * GQ_TILE;   // [128] reciprocals of the current tile's diagonal
+  float* sE = sR + GQ_BLOCK;                        // 2 x [R][128] scaled errors of a block
+  float* sW = sE + 2 * R * GQ_BLOCK;                // [R][cols] working rows
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, threads = blockDim.x;
+  const int row0 = blockIdx.x * R;
+  const int live = min(R, rows - row0);
+  for (int r = warp; r < R; r += threads / 32) {
+    const float* src = Wp + (size_t)((row0 + min(r, live - 1)) % weight_rows) * cols;
+    for (int c = lane; c < cols; c += 32) sW[r * cols + c] = r < live ? src[c] : 0.f;
+  }
+  for (int i = threadIdx.x; i < 2 * R * GQ_BLOCK; i += threads) sE[i] = 0.f;
   const bool wide = (cols & 3) == 0 && (reinterpret_cast<uintptr_t>(U) & 15) == 0;      // rows of U start on 16-byte boundaries
-  auto load_tile = [&](int i1, int t, int threads) {     // elements outside the matrix read as zero
+  auto load_tile = [&](int i1, int t, int nthreads) {    // elements outside the matrix read as zero
     const int nb = min(GQ_BLOCK, cols - i1);
-    float* dst = sU + ((i1 / GQ_BLOCK) & 1) * GQ_TILE;
+    float* dst = sU + (TWO_TILES ? ((i1 / GQ_BLOCK) & 1) * GQ_TILE : 0);
     if (wide) {
-      for (int idx = t * 4; idx < GQ_TILE; idx += threads * 4) {
+      for (int idx = t * 4; idx < GQ_TILE; idx += nthreads * 4) {
         const int j = idx >> 7, c = idx & 127;
         const bool in = j < nb && c < nb;
         gq_copy<16>(dst + idx, in ? U + (size_t)(i1 + j) * cols + i1 + c : U, in);
       }
     } else {
-      for (int idx = t; idx < GQ_TILE; idx += threads) {
+      for (int idx = t; idx < GQ_TILE; idx += nthreads) {
         const int j = idx >> 7, c = idx & 127;
         const bool in = j < nb && c < nb;
         gq_copy<4>(dst + idx, in ? U + (size_t)(i1 + j) * cols + i1 + c : U, in);
@@ -129,61 +137,71 @@ gptq_rows_kernel(const float* __restrict__ Wp, const float* __restrict__ U, cons
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  load_tile(0, threadIdx.x, GQ_THREADS);
+  auto reciprocals = [&](int i1) {
+    const float* tile = sU + (TWO_TILES ? ((i1 / GQ_BLOCK) & 1) * GQ_TILE : 0);
+    if (threadIdx.x < min(GQ_BLOCK, cols - i1)) sR[threadIdx.x] = __frcp_rn(tile[threadIdx.x * (GQ_BLOCK + 1)]);
+  };
+  load_tile(0, threadIdx.x, threads);
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  if (threadIdx.x < min(GQ_BLOCK, cols)) sR[threadIdx.x] = __frcp_rn(sU[threadIdx.x * (GQ_BLOCK + 1)]);
+  reciprocals(0);
   __syncthreads();
   const float s = warp < live ? scales[row0 + warp] : 1.f;
   const float rs = __frcp_rn(s);
   for (int i1 = 0; i1 < cols; i1 += GQ_BLOCK) {
     const int nb = min(GQ_BLOCK, cols - i1);
     const int buf = (i1 / GQ_BLOCK) & 1;
-    if (warp < GQ_ROWS) {
+    if (warp < R) {
       if (warp < live) {
-        const float* tile = sU + buf * GQ_TILE;
-        float* e_row = sE + (buf * GQ_ROWS + warp) * GQ_BLOCK;
+        const float* tile = sU + (TWO_TILES ? buf * GQ_TILE : 0);
+        float* e_row = sE + (buf * R + warp) * GQ_BLOCK;
         const float* w_row = sW + warp * cols + i1;
         int8_t* q_row = Q + (size_t)(row0 + warp) * cols + i1;
         if (nb == GQ_BLOCK) walk_block<true>(tile, sR, w_row, q_row, e_row, lane, nb, s, rs, qmin, qmax);
         else walk_block<false>(tile, sR, w_row, q_row, e_row, lane, nb, s, rs, qmin, qmax);
       }
     } else {
-      const int t = threadIdx.x - 32 * GQ_ROWS;
-      if (i1 + GQ_BLOCK < cols) load_tile(i1 + GQ_BLOCK, t, GQ_FAR_THREADS);
+      const int t = threadIdx.x - 32 * R;
+      if (TWO_TILES && i1 + GQ_BLOCK < cols) load_tile(i1 + GQ_BLOCK, t, GQ_FAR_THREADS);
       if (i1 > 0) {
         // far: the previous block's errors into the columns beyond this block, w[r][c] -= sum_j err[r][j] * U[j][c]
-        const float* e_prev = sE + (buf ^ 1) * GQ_ROWS * GQ_BLOCK;
         for (int c = i1 + GQ_BLOCK + t; c < cols; c += GQ_FAR_THREADS) {
-          float a[GQ_ROWS][4] = {};
           const float* u = U + (size_t)(i1 - GQ_BLOCK) * cols + c;
+          for (int r0 = 0; r0 < live; r0 += GROUP) {
+            const float* e_prev = sE + ((buf ^ 1) * R + r0) * GQ_BLOCK;
+            const int rn = min(GROUP, R - r0);              // R is a multiple of 4: a group may be half full
+            float a[GROUP][4] = {};
 #pragma unroll 4
-          for (int j = 0; j < GQ_BLOCK; j += 4) {
-            const float u0 = __ldg(u + (size_t)j * cols), u1 = __ldg(u + (size_t)(j + 1) * cols), u2 = __ldg(u + (size_t)(j + 2) * cols),
-                        u3 = __ldg(u + (size_t)(j + 3) * cols);
+            for (int j = 0; j < GQ_BLOCK; j += 4) {
+              const float u0 = __ldg(u + (size_t)j * cols), u1 = __ldg(u + (size_t)(j + 1) * cols), u2 = __ldg(u + (size_t)(j + 2) * cols),
+                          u3 = __ldg(u + (size_t)(j + 3) * cols);
 #pragma unroll
-            for (int r = 0; r < GQ_ROWS; ++r) {
-              const float4 e = *reinterpret_cast<const float4*>(e_prev + r * GQ_BLOCK + j);
-              a[r][0] = fmaf(e.x, u0, a[r][0]);
-              a[r][1] = fmaf(e.y, u1, a[r][1]);
-              a[r][2] = fmaf(e.z, u2, a[r][2]);
-              a[r][3] = fmaf(e.w, u3, a[r][3]);
+              for (int r = 0; r < GROUP; ++r) {
+                if (r >= 4 && r >= rn) break;
+                const float4 e = *reinterpret_cast<const float4*>(e_prev + r * GQ_BLOCK + j);
+                a[r][0] = fmaf(e.x, u0, a[r][0]);
+                a[r][1] = fmaf(e.y, u1, a[r][1]);
+                a[r][2] = fmaf(e.z, u2, a[r][2]);
+                a[r][3] = fmaf(e.w, u3, a[r][3]);
+              }
             }
-          }
 #pragma unroll
-          for (int r = 0; r < GQ_ROWS; ++r) sW[r * cols + c] -= (a[r][0] + a[r][1]) + (a[r][2] + a[r][3]);
+            for (int r = 0; r < GROUP; ++r)
+              if (r < 4 || r < rn) sW[(r0 + r) * cols + c] -= (a[r][0] + a[r][1]) + (a[r][2] + a[r][3]);
+          }
         }
       }
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      if (TWO_TILES) asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
-    __syncthreads();                                // this block's errors, the far updates and the next tile are visible
+    __syncthreads();                                // this block's errors and the far updates (and the next of two tiles) are visible
     if (i1 + GQ_BLOCK >= cols) break;
-    {
-      // near: this (whole) block's errors into the next block's columns
-      const int r = threadIdx.x >> 7, cc = threadIdx.x & 127, c = i1 + GQ_BLOCK + cc;
-      if (r == 0 && c < cols) sR[cc] = __frcp_rn(sU[(buf ^ 1) * GQ_TILE + cc * (GQ_BLOCK + 1)]);
+    if (!TWO_TILES) load_tile(i1 + GQ_BLOCK, threadIdx.x, threads);
+    if (TWO_TILES) reciprocals(i1 + GQ_BLOCK);
+    // near: this (whole) block's errors into the next block's columns
+    for (int i = threadIdx.x; i < R * GQ_BLOCK; i += threads) {
+      const int r = i >> 7, c = i1 + GQ_BLOCK + (i & 127);
       if (c < cols) {
-        const float* e_row = sE + (buf * GQ_ROWS + r) * GQ_BLOCK;
+        const float* e_row = sE + (buf * R + r) * GQ_BLOCK;
         const float* u = U + (size_t)i1 * cols + c;
         float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
 #pragma unroll 8
@@ -197,26 +215,53 @@ gptq_rows_kernel(const float* __restrict__ Wp, const float* __restrict__ U, cons
         sW[r * cols + c] -= (a0 + a1) + (a2 + a3);
       }
     }
+    if (!TWO_TILES) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      reciprocals(i1 + GQ_BLOCK);
+    }
     __syncthreads();
   }
 }
+
+size_t gq_smem(int R, int cols, bool two_tiles) {
+  return ((two_tiles ? 2 : 1) * (size_t)GQ_TILE + GQ_BLOCK + 2 * (size_t)R * GQ_BLOCK + (size_t)R * cols) * sizeof(float);
+}
+
+template <int GROUP, int MAX_THREADS, bool TWO_TILES>
+void gq_launch(const float* Wp, const float* U, const float* scales, int8_t* Q, int rows, int weight_rows, int cols, int R, float qmin, float qmax,
+               cudaStream_t st) {
+  auto kern = gptq_rows_kernel<GROUP, MAX_THREADS, TWO_TILES>;
+  const size_t smem = gq_smem(R, cols, TWO_TILES);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  kern<<<(rows + R - 1) / R, 32 * R + GQ_FAR_THREADS, smem, st>>>(Wp, U, scales, Q, rows, weight_rows, cols, R, qmin, qmax);
+}
 }  // namespace
 
-void gptq_rows(const float* Wp, const float* U, const float* scales, int8_t* Q, int rows, int cols, int bits, cudaStream_t st) {
-  if (rows <= 0 || cols <= 0) return;
+void gptq_rows(const float* Wp, const float* U, const float* scales, int8_t* Q, int candidates, int rows, int cols, int bits, cudaStream_t st) {
+  if (rows <= 0 || cols <= 0 || candidates <= 0) return;
   if (bits < 2 || bits > 8) throw std::runtime_error("gptq_rows: bits must be in 2..8");
-  constexpr size_t fixed = 2 * (size_t)GQ_TILE + GQ_BLOCK + 2 * GQ_ROWS * GQ_BLOCK;
-  const size_t smem = (fixed + (size_t)GQ_ROWS * cols) * sizeof(float);
-  if (smem > 227 * 1024) throw std::runtime_error("gptq_rows: rows of more than " + std::to_string((227 * 1024 / 4 - fixed) / GQ_ROWS) + " columns do not fit in shared memory");
-  static size_t configured[64] = {};        // largest size set so far, per device (the attribute is a per-device property)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || smem > configured[dev]) {
-    cudaFuncSetAttribute(gptq_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (dev >= 0 && dev < 64) configured[dev] = smem;
-  }
+  if ((long long)rows * candidates > 0x7fffffffll) throw std::runtime_error("gptq_rows: too many rows");
+  const size_t limit = 227 * 1024;
+  if (gq_smem(GQ_ROWS, cols, true) > limit)
+    throw std::runtime_error("gptq_rows: rows of more than " + std::to_string((limit - gq_smem(GQ_ROWS, 0, true)) / sizeof(float) / GQ_ROWS) +
+                             " columns do not fit in shared memory");
   const float qmax = (float)((1 << (bits - 1)) - 1), qmin = -(float)(1 << (bits - 1));
-  gptq_rows_kernel<<<(rows + GQ_ROWS - 1) / GQ_ROWS, GQ_THREADS, smem, st>>>(Wp, U, scales, Q, rows, cols, qmin, qmax);
+  const int total = rows * candidates;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // A CTA fills an SM in both forms and takes about as long for 20 rows as for 4 (the chain along the columns), so the count of rounds
+  // decides: four rows per CTA while those fit in one round, else as many as shared memory allows, evened out over the rounds.
+  int R = GQ_ROWS;
+  if ((total + GQ_ROWS - 1) / GQ_ROWS > sms) {
+    int most = GQ_MAX_ROWS;
+    while (most > GQ_ROWS && gq_smem(most, cols, false) > limit) most -= 4;
+    const int rounds = (total + sms * most - 1) / (sms * most);
+    R = std::min(most, ((total + sms * rounds - 1) / (sms * rounds) + 3) / 4 * 4);
+  }
+  if (R == GQ_ROWS) gq_launch<GQ_GROUP_SMALL, 32 * GQ_ROWS + GQ_FAR_THREADS, true>(Wp, U, scales, Q, total, rows, cols, R, qmin, qmax, st);
+  else gq_launch<GQ_GROUP_LARGE, 32 * GQ_MAX_ROWS + GQ_FAR_THREADS, false>(Wp, U, scales, Q, total, rows, cols, R, qmin, qmax, st);
 }
 
 }  // namespace pgb

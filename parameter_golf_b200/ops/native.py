@@ -220,9 +220,11 @@ def attn_bwd_part(device):
 
 
 def gptq_rows(Wp, U, scales, bits, block=128):
-    """GPTQ row kernel (one clip candidate): int8 codes for the permuted rows ``Wp`` given the Cholesky factor ``U``."""
+    """GPTQ row kernel: int8 codes for the permuted rows ``Wp`` given the Cholesky factor ``U``; ``scales`` is [rows] (one clip
+    candidate) or [candidates, rows], which gives codes [candidates, rows, cols] from one launch."""
     if block != 128:
         raise ValueError("the GPTQ kernel works on 128-column blocks")
-    Q = torch.empty(Wp.shape, dtype=torch.int8, device=Wp.device)
+    shape = tuple(Wp.shape) if scales.numel() == Wp.shape[0] else (scales.shape[0], *Wp.shape)
+    Q = torch.empty(shape, dtype=torch.int8, device=Wp.device)
     load().gptq_rows(Wp.contiguous().float(), U.contiguous().float(), scales.contiguous().float(), Q, bits)
     return Q

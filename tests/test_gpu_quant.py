@@ -79,3 +79,19 @@ def test_gptq_prepare_gives_the_upper_factor_of_the_inverse():
     want = torch.linalg.cholesky(torch.cholesky_inverse(torch.linalg.cholesky(Hp)), upper=True)
     assert torch.equal(perm[inv_perm], torch.arange(192, device=perm.device)) and float(U.tril(-1).abs().max()) == 0.0
     assert float((U.double() - want).norm() / want.norm()) < 1e-6          # one rounding to fp32: 2^-24 per element
+
+
+@pytest.mark.parametrize("rows,cols", [(7, 129), (150, 256), (700, 384), (1100, 200), (130, 2600)])
+def test_gptq_rows_of_several_candidates_are_those_of_one_at_a_time(rows, cols):
+    """One launch over (candidate, row) pairs, in the small form and in the large one (row counts around a CTA's 4 to 20 rows, one and
+    two rounds, columns off 16 bytes), gives the codes of one launch per candidate: the arithmetic of a row is the same."""
+    from parameter_golf_b200.ops import native as n
+    from parameter_golf_b200.quant.gptq import gptq_prepare
+    W, H = _problem(rows, cols, rows + cols)
+    perm, _, U = gptq_prepare(H)
+    Wp = W[:, perm].contiguous()
+    scales = torch.stack([(Wp.abs().amax(1) * f / 31).clamp_min(1e-8) for f in (1.0, 0.9, 0.8, 0.7, 0.6)])
+    got = n.gptq_rows(Wp, U, scales, 6)
+    for k in range(5):
+        want = torch.cat([n.gptq_rows(Wp[i:i + 500], U, scales[k, i:i + 500], 6) for i in range(0, rows, 500)])
+        assert torch.equal(got[k], want), k
