@@ -87,6 +87,8 @@ void head_gate_bwd(void* d_out, const void* y, const void* x, const float* W, co
 // of rows the sum covers when this call sees only a chunk of them (0: the same `rows`)
 void softcap_ce(const void* logits, const int* targets, float* nll, void* dlogits, float* loss_sum, int rows, int V, float cap, float gscale,
                 cudaStream_t st, const float* tok_w = nullptr, const float* w_total = nullptr, int norm_rows = 0);
+// out[i] = cap * tanh(z[i] / cap), z bf16, n a multiple of 8, both 16-byte aligned
+void softcap_logits(const void* z, float* out, long long n, float cap, cudaStream_t st);
 // w[i] = table[prev[i] * V + curr[i]], *w_total = sum_i w[i] (zeroed here first)
 void pair_weights(const int* prev, const int* curr, const float* table, float* w, float* w_total, int rows, int V, cudaStream_t st);
 // ids outside [0, table_rows) give a zero row and ST_BAD_INDEX in the status word instead of an address

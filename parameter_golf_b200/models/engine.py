@@ -907,8 +907,8 @@ class EngineRunner:
         e = self._engine(ids.shape[0], ids.shape[1])
         e.set_lora(self.lora)
         e.forward(ids.to(self.device, torch.int32), None)
-        z = (e.logits if e.logit_rows >= e.T else e._logits_full).view(*ids.shape, -1).float()
-        return self.model.logit_softcap * torch.tanh(z / self.model.logit_softcap)
+        z = e.logits if e.logit_rows >= e.T else e._logits_full
+        return N.softcap_logits(z, self.model.logit_softcap).view(*ids.shape, -1)
 
     @torch.no_grad()
     def loss_and_grads(self, ids, targets, qat: bool = False, names=None):

@@ -219,6 +219,13 @@ def attn_bwd_part(device):
     return torch.empty(load()._mod.attn_bwd_part_floats(), dtype=torch.float32, device=device)
 
 
+def softcap_logits(z, cap):
+    """fp32 ``cap * tanh(z / cap)`` of bf16 logits."""
+    out = torch.empty(z.shape, dtype=torch.float32, device=z.device)
+    load().softcap_logits(z, out, cap)
+    return out
+
+
 def gptq_rows(Wp, U, scales, bits, block=128):
     """GPTQ row kernel: int8 codes for the permuted rows ``Wp`` given the Cholesky factor ``U``; ``scales`` is [rows] (one clip
     candidate) or [candidates, rows], which gives codes [candidates, rows, cols] from one launch."""

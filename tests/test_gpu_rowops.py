@@ -218,3 +218,16 @@ def test_embedding_gather_and_scatter_with_bigram_hash(B, S):
     ref = torch.zeros(V, d, device="cuda").index_add_(0, ids.long(), g.float())
     bref = torch.zeros(buckets, bd, device="cuda").index_add_(0, hashed, bg.float())
     assert rel(dt, ref) < 1e-5 and rel(dbt, bref) < 1e-5
+
+
+@pytest.mark.parametrize("shape", [(1, 64), (3, 1024), (257, 8192)])
+def test_softcap_logits(shape):
+    """cap * tanh(z / cap) in fp32: four roundings of a value below the cap (4 * 2^-24 * cap), infinities to the cap, NaN to NaN."""
+    from parameter_golf_b200.ops import native as n
+    torch.manual_seed(shape[0])
+    z = (torch.randn(shape, device="cuda") * 40).bfloat16()
+    z[0, :4] = torch.tensor([float("inf"), float("-inf"), float("nan"), 0.0])
+    got, want = n.softcap_logits(z, 30.0), 30.0 * torch.tanh(z.double() / 30.0)
+    assert got.shape == z.shape and got.dtype == torch.float32
+    assert bool(got[0, 2].isnan()) and int(got.isnan().sum()) == 1
+    assert float((got.double() - want).nan_to_num(0.0).abs().max()) <= 30.0 * 4 * 2.0 ** -24
