@@ -60,12 +60,12 @@ __device__ __forceinline__ float4 load_w4<__nv_bfloat16>(const __nv_bfloat16* p)
 }
 
 template <typename WT>
-__global__ void __launch_bounds__(256) fold_scaled_grad_kernel(const float* __restrict__ G, const WT* __restrict__ W, const float* __restrict__ rowscale,
+__global__ void __launch_bounds__(256) fold_scaled_grad_kernel(float* __restrict__ G, const WT* __restrict__ W, const float* __restrict__ rowscale,
                                                                int scale_stride, int scale_mod, float* __restrict__ dW, float* __restrict__ dscale,
                                                                int rows, int cols, int qat) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int row = blockIdx.x * 8 + warp; row < rows; row += gridDim.x * 8) {
-    const float* g = G + (size_t)row * cols;
+    float* g = G + (size_t)row * cols;
     const WT* w = W + (size_t)row * cols;
     float* o = dW + (size_t)row * cols;
     float qs = 0.f;
@@ -97,6 +97,8 @@ __global__ void __launch_bounds__(256) fold_scaled_grad_kernel(const float* __re
     }
     dot = warp_sum(dot);
     if (lane == 0) atomicAdd(dscale + sidx, dot);
+    // the product that fills G accumulates into it: leave it zero (after the row's last load; a store behind each load is slow)
+    for (int c = lane * 4; c < cols; c += 128) *reinterpret_cast<float4*>(g + c) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
@@ -260,14 +262,14 @@ void cast_rows(const float* src, void* dst, const float* rowscale, int scale_str
                                                                      cols, ld_dst, qat);
 }
 
-void fold_scaled_grad(const float* G, const float* W, const float* rowscale, int scale_stride, int scale_mod, float* dW, float* dscale, int rows,
+void fold_scaled_grad(float* G, const float* W, const float* rowscale, int scale_stride, int scale_mod, float* dW, float* dscale, int rows,
                       int cols, int qat, cudaStream_t st) {
   if (cols % 4) throw std::runtime_error("fold_scaled_grad: cols must be a multiple of 4");
   fold_scaled_grad_kernel<float><<<std::min((rows + 7) / 8, 148 * 8), 256, 0, st>>>(G, W, rowscale, scale_stride, std::max(scale_mod, 1), dW, dscale,
                                                                                    rows, cols, qat);
 }
 
-void fold_scaled_grad_bf16(const float* G, const void* W, const float* rowscale, int scale_stride, int scale_mod, float* dW, float* dscale, int rows,
+void fold_scaled_grad_bf16(float* G, const void* W, const float* rowscale, int scale_stride, int scale_mod, float* dW, float* dscale, int rows,
                            int cols, cudaStream_t st) {
   if (cols % 4) throw std::runtime_error("fold_scaled_grad: cols must be a multiple of 4");
   fold_scaled_grad_kernel<__nv_bfloat16><<<std::min((rows + 7) / 8, 148 * 8), 256, 0, st>>>(G, (const __nv_bfloat16*)W, rowscale, scale_stride,

@@ -129,9 +129,10 @@ void xsa_bwd64(const void* dz, const void* y, const void* v, void* dy, void* dv,
 // hp: device fp32[8] = {lr_scale, muon_momentum, adam_bias_corr1, adam_bias_corr2, grad_scale, ...}
 void cast_rows(const float* src, void* dst, const float* rowscale, int scale_stride, int scale_mod, int rows, int cols, long long ld_dst, int qat,
                cudaStream_t st);
-void fold_scaled_grad(const float* G, const float* W, const float* rowscale, int scale_stride, int scale_mod, float* dW, float* dscale, int rows,
+// G is left zeroed, ready for the next product that accumulates into it
+void fold_scaled_grad(float* G, const float* W, const float* rowscale, int scale_stride, int scale_mod, float* dW, float* dscale, int rows,
                       int cols, int qat, cudaStream_t st);
-void fold_scaled_grad_bf16(const float* G, const void* W, const float* rowscale, int scale_stride, int scale_mod, float* dW, float* dscale, int rows,
+void fold_scaled_grad_bf16(float* G, const void* W, const float* rowscale, int scale_stride, int scale_mod, float* dW, float* dscale, int rows,
                            int cols, cudaStream_t st);
 void sumsq(const float* x, long long n, float scale, float* out, cudaStream_t st);
 void sum_splits_add(const float* part, int splits, long long split_stride, float* dst, long long n, cudaStream_t st);

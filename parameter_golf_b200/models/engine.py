@@ -112,7 +112,7 @@ class CudaEngine:
         if share is not None:
             assert share.dev == self.dev and share.train == train and share.m == self.m
             for name in ("p", "g", "groups", "Wqkv", "Wo", "Wup", "Wd", "Wo_u", "Wd_u", "E", "LM", "BE", "BP", "VE", "VP", "ve_eff", "ema", "mom",
-                         "ns", "Gd", "Go", "Gbp", "Gvp"):
+                         "ns", "Gd", "Go", "Gbp", "Gvp", "fold_open"):
                 if hasattr(share, name):
                     setattr(self, name, getattr(share, name))
         else:
@@ -136,6 +136,7 @@ class CudaEngine:
         # for per-layer gradient reduction overlapped with the rest of the backward (role of `GpuBackwardLayerObserver`,
         # pg-model/src/gpu.rs:517-525).
         self.backward_observer = None
+        self.want = None                 # names whose gradients the backward has to produce (None: every parameter)
         self.adam_t = 0
         self.layer_flags = None          # set by the sharded optimizer: per-layer weight-ready counters
         self.layer_flag_value = 0
@@ -234,6 +235,9 @@ class CudaEngine:
                 self.ns[k] = {"U": torch.empty(Bk, Mk, Nk, dtype=BF, device=dev), "X0": torch.empty(Bk, Mk, Nk, dtype=BF, device=dev),
                               "X1": torch.empty(Bk, Mk, Nk, dtype=BF, device=dev), "A": torch.empty(Bk, r, r, dtype=BF, device=dev),
                               "Bm": torch.empty(Bk, r, r, dtype=BF, device=dev), "sq": torch.zeros(Bk, dtype=torch.float32, device=dev)}
+            # staging of the scaled weights' gradients: zero between uses (the fold kernel leaves it so); the flag is set while one holds
+            # a product that has not been folded yet
+            self.fold_open = [False]
             self.Gd = torch.zeros(d, mlp, dtype=torch.float32, device=dev)
             self.Go = torch.zeros(d, d, dtype=torch.float32, device=dev)
             if m.bigram.enabled:
@@ -398,6 +402,20 @@ class CudaEngine:
         bounds = [(G, 0)] + [(t_, r_) for r_, t_ in segs if t_ is not None]
         for i, (dst, start) in enumerate(bounds):            # row range [start, end) of every partial goes to `dst`
             self.C.sum_splits_add(self._dw_ws, start * Nn, splits, M * Nn, dst)
+
+    def _wants(self, *names) -> bool:
+        """Whether any of these parameters' gradients was asked for (`want` is None: all of them)."""
+        return self.want is None or any(k in self.want for k in names)
+
+    def _dw_folded(self, dY, X, G, fold, *fold_args):
+        """``G = dY^T X`` handed to a fold kernel, which leaves ``G`` zero for the next layer."""
+        if self.fold_open[0]:                    # a call that raised in between left its product behind
+            for t in (self.Gd, self.Go) + ((self.Gbp,) if self.m.bigram.enabled else ()):
+                t.zero_()
+        self.fold_open[0] = True
+        self._dw(dY, X, G)
+        fold(G, *fold_args)
+        self.fold_open[0] = False
 
     # ---- Q-LoRA (test-time training) ---------------------------------------------------------------------------------------
     def set_lora(self, lora: Optional[dict]):
@@ -599,7 +617,8 @@ class CudaEngine:
                          self.tok_w[r0:r1] if weighted else None, self.w_total if weighted else None, T)
             if want_grad:
                 N.gemm(lg, self.LM, self.d_h[r0:r1], True, False)          # d_hf rows
-                self._dw(lg, self.hf[r0:r1], gW)
+                if self._wants("tok_emb" if m.tie_embeddings else "lm_head"):
+                    self._dw(lg, self.hf[r0:r1], gW)
         self._head_grads_done = want_grad
 
     def set_token_weight_table(self, table) -> None:
@@ -622,9 +641,11 @@ class CudaEngine:
         C, m, p, g = self.C, self.m, self.p, self.g
         n, d, kv, S = self.n, self.d, self.kv, self.S
         A = N.EPI_F32_ATOMIC
+        wants_ve = self._wants("ve_embed", "ve_proj", "ve_layer_scales", "ve_scale")
         if not self._head_grads_done:              # the chunked head has already produced d_hf and the output-embedding gradient
             N.gemm(self.logits, self.LM, self.d_h, True, False)                              # d_hf
-            self._dw(self.logits, self.hf, g["tok_emb"] if m.tie_embeddings else g["lm_head"])
+            if self._wants("tok_emb" if m.tie_embeddings else "lm_head"):
+                self._dw(self.logits, self.hf, g["tok_emb"] if m.tie_embeddings else g["lm_head"])
         C.mix_norm_bwd(self.d_h, None, self.x_last, None, None, None, None, None, None, self.dx, None, None, None, None, False, 1.0, self.eps)
         self.d_x0.zero_()
         xsa_layers = m.xsa_layers()
@@ -635,11 +656,12 @@ class CudaEngine:
             if not self.saved[j]:
                 self._block_fwd(j, *self.block_in[j], recompute=True)
             # ---- MLP
-            self.Gd.zero_()
-            self._dw(self.dx, self.a[aj], self.Gd)
-            C.fold_scaled_grad_bf16(self.Gd, self.Wd_u[l], p["mlp_scale"][l], 1, d, g["mlp_down_bank"][l], g["mlp_scale"][l])
+            if self._wants("mlp_down_bank", "mlp_scale"):
+                self._dw_folded(self.dx, self.a[aj], self.Gd, C.fold_scaled_grad_bf16, self.Wd_u[l], p["mlp_scale"][l], 1, d, g["mlp_down_bank"][l],
+                                g["mlp_scale"][l])
             N.gemm(self.dx, self.Wd[l], self.d_hu, True, False, N.EPI_MUL_ACTGRAD, slope=self.slope, aux=self.hu[aj])
-            self._dw(self.d_hu, self.mm[aj], g["mlp_up_bank"][l])
+            if self._wants("mlp_up_bank"):
+                self._dw(self.d_hu, self.mm[aj], g["mlp_up_bank"][l])
             N.gemm(self.d_hu, self.Wup[l], self.d_m, True, False)
             if self.parallel:
                 dx_mid, dx_next = self.dx, self.dx_mid      # no norm between x_mid and the MLP: the residual gradient passes through
@@ -650,9 +672,8 @@ class CudaEngine:
                 d_hx = self.d_hx if self.gates else None
             # ---- attention output projection
             zz = self.zz[aj]
-            self.Go.zero_()
-            self._dw(dx_mid, zz, self.Go)
-            C.fold_scaled_grad_bf16(self.Go, self.Wo_u[l], p["attn_scale"][l], 1, d, g["qo_bank"][n + l], g["attn_scale"][l])
+            if self._wants("qo_bank", "attn_scale"):
+                self._dw_folded(dx_mid, zz, self.Go, C.fold_scaled_grad_bf16, self.Wo_u[l], p["attn_scale"][l], 1, d, g["qo_bank"][n + l], g["attn_scale"][l])
             vview = self.qkv_pre[aj][:, d + kv:]
             dv = self.d_qkv_pre[:, d + kv:]
             xsa = l in xsa_layers
@@ -670,7 +691,7 @@ class CudaEngine:
                 else:
                     C.xsa_bwd(self.d_z, self.y[aj], vview, self.d_y, dv, False, self.Hkv, self.H // self.Hkv, self.hd, 1e-8, self.dsum, S)
             self._attn_bwd(l, aj)
-            if m.value_embedding.enabled and l in m.value_embedding.layers:
+            if m.value_embedding.enabled and l in m.value_embedding.layers and wants_ve:
                 vi = m.value_embedding.layers.index(l)
                 self.Gvp.zero_()
                 N.gemm(dv, self.ve_e, self.Gvp, False, False, A)                         # d(ve_eff * ve_proj)
@@ -684,7 +705,8 @@ class CudaEngine:
                 N.gemm(dv, self.VP[vi], self.d_ve_e, True, False)
                 self.d_ve_acc.add_(self.d_ve_e)
             # one weight-gradient product for the packed QKV rows, written to the Q, K and V slots of the gradient banks
-            self._dw(self.d_qkv_pre, self.h[aj], g["qo_bank"][l], segs=((d, g["kv_bank"][l]), (d + kv, g["kv_bank"][n + l])))
+            if self._wants("qo_bank", "kv_bank"):
+                self._dw(self.d_qkv_pre, self.h[aj], g["qo_bank"][l], segs=((d, g["kv_bank"][l]), (d + kv, g["kv_bank"][n + l])))
             if d_hx is not None:
                 N.gemm(self.d_qkv_pre, self.Wqkv[l], self.d_h, True, False, N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=d_hx)
             else:
@@ -712,21 +734,22 @@ class CudaEngine:
                 self.dx, self.dx_mid = self.dx_mid, self.dx
             if self.backward_observer is not None:
                 self.backward_observer(l, j)
+        if m.value_embedding.enabled and hasattr(self, "d_ve_acc") and wants_ve:
+            self.d_ve_e.copy_(self.d_ve_acc)
+            self.d_ve_acc.zero_()
+            C.embed_scatter_add(self.ids, self.d_ve_e, g["ve_embed"], 0, S)
+        if not self._wants("smear_gate", "tok_emb", "bigram_embed", "bigram_proj", "bigram_scale"):
+            return
         self.dx.add_(self.d_x0)
         bid = m.smear_gate_boundary_token_id
         C.norm_smear_bwd(self.dx, self.xe, p["smear_gate"] if m.smear_gate else None, self.ids if (m.smear_gate and bid is not None) else None,
                          self.d_xe, g["smear_gate"] if m.smear_gate else None, S, -1 if bid is None else bid, self.eps)
         C.embed_scatter_add(self.ids, self.d_xe, g["tok_emb"], 0, S)
         if m.bigram.enabled:
-            self.Gbp.zero_()
-            self._dw(self.d_xe, self.bg, self.Gbp)
-            C.fold_scaled_grad(self.Gbp, p["bigram_proj"], p["bigram_scale"], 0, 1, g["bigram_proj"], g["bigram_scale"], False)
+            self._dw_folded(self.d_xe, self.bg, self.Gbp, C.fold_scaled_grad, p["bigram_proj"], p["bigram_scale"], 0, 1, g["bigram_proj"],
+                            g["bigram_scale"], False)
             N.gemm(self.d_xe, self.BP, self.d_bg, True, False)
             C.embed_scatter_add(self.ids, self.d_bg, g["bigram_embed"], m.bigram.vocab_size, S)
-        if m.value_embedding.enabled and hasattr(self, "d_ve_acc"):
-            self.d_ve_e.copy_(self.d_ve_acc)
-            self.d_ve_acc.zero_()
-            C.embed_scatter_add(self.ids, self.d_ve_e, g["ve_embed"], 0, S)
 
     # ---- public pieces -----------------------------------------------------------------------------------------------------------
     def zero_grads(self):
@@ -918,9 +941,13 @@ class EngineRunner:
             e.cast_weights()
         e.set_lora(self.lora)
         e.zero_grads()
-        e.micro_step(ids.to(self.device, torch.int32), targets.to(self.device, torch.int32), 1)
-        loss = e.loss_sum[0] / e.T
         names = list(e.g) if names is None else list(names)
+        e.want = frozenset(names)                # products that only feed other gradients are left out
+        try:
+            e.micro_step(ids.to(self.device, torch.int32), targets.to(self.device, torch.int32), 1)
+        finally:
+            e.want = None
+        loss = e.loss_sum[0] / e.T
         grads = {k: e.g[k] for k in names}
         if self.lora is not None and self.lora.get("trainable", False):
             grads["lora.a"], grads["lora.b"] = e.g_lora_a, e.g_lora_b

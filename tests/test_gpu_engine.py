@@ -652,3 +652,27 @@ def test_chunked_output_head_matches_the_full_logits_path(weighted):
     r = EngineRunner(spec, gpt.fill_deterministic(spec.model), "cuda", batch=4, train=False)
     full = EngineRunner(small_spec(), gpt.fill_deterministic(spec.model), "cuda", batch=4, train=False)
     assert torch.allclose(r.logits(ids), full.logits(ids), atol=1e-3) and torch.allclose(r.nll(ids, tgt), full.nll(ids, tgt), atol=1e-5)
+
+
+@pytest.mark.parametrize("names", [["mlp_up_bank", "q_gain"], ["bigram_proj", "attn_scale"], ["tok_emb"], ["kv_bank", "mlp_scale", "smear_gate"]])
+def test_gradients_of_some_parameters_are_those_of_all(names):
+    """`loss_and_grads(names=...)` leaves out the products that feed other gradients only; what it returns is what the full call
+    returns, up to the order of the fp32 adds (relative 2-norm 1e-4: about sqrt(terms) 2^-24), also on the next full call."""
+    from parameter_golf_b200.models import gpt
+    from parameter_golf_b200.models.engine import EngineRunner
+    from parameter_golf_b200.ops import native
+    spec = small_spec()
+    params = gpt.fill_deterministic(spec.model)
+    torch.manual_seed(5)
+    ids, tgt = torch.randint(0, 256, (4, 128)), torch.randint(0, 256, (4, 128))
+    eng = EngineRunner(spec, params, "cuda", batch=4)
+    names = [k for k in names if k in params]
+    full = {k: v.clone() for k, v in eng.loss_and_grads(ids, tgt)[1].items()}
+    some = {k: v.clone() for k, v in eng.loss_and_grads(ids, tgt, names=names)[1].items()}
+    again = eng.loss_and_grads(ids, tgt)[1]
+    native.check_status()
+    assert sorted(some) == sorted(names)
+    for k in names:
+        assert float((some[k] - full[k]).norm()) <= 1e-4 * float(full[k].norm()) + 1e-12, k
+    for k in full:
+        assert float((again[k] - full[k]).norm()) <= 1e-4 * float(full[k].norm()) + 1e-12, k
