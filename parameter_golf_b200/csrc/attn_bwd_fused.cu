@@ -43,6 +43,7 @@
 // (parameter-golf-rs/crates/pg-kernels/cpp/cudnn_sdpa.cu:364-435).
 #include "common.cuh"
 #include "pgb.h"
+#include "launch.h"
 #include "tma_host.h"
 
 namespace pgb {
@@ -259,6 +260,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_next();
+  chain_wait();
   // TMEM columns: S^T [0,128)  dP^T [128,256)  P^T bf16 [256,320)  dK [320,384)  dV [384,448)  dQ [448,512)
 
   if (warp < 4) {
@@ -584,6 +587,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 // dK/dV of the key tiles whose units two or more CTAs shared: CTA c handles the tile in which range c starts, if range c is the
 // first to start inside it. Contributions are the previous range's last-tile slot and the first-tile slots from range c on.
 __global__ void __launch_bounds__(256) attn_bwd_merge_kernel(const FusedParams p, int ctas) {
+  chain_next();
+  chain_wait();
   const int c = (int)blockIdx.x + 1;
   const int lo = f_range_start(p, c, ctas);
   if (lo >= p.rest_base + p.rest_w) return;
@@ -628,6 +633,8 @@ __global__ void __launch_bounds__(256) attn_bwd_merge_kernel(const FusedParams p
 // D = rowsum(dO * O) per (token, head), stored negated in [B, H, S] order. Eight lanes share one head's 64 columns.
 __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO, long long ldo,
                                                             long long lddo, float* __restrict__ dsum, long long T, int S, int H) {
+  chain_next();
+  chain_wait();
   const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
   const int chunk = (int)(idx & 7);
   const long long rh = idx >> 3;
@@ -655,6 +662,8 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
 // tile, and written out one 128-byte head row per 8 lanes.
 __global__ void __launch_bounds__(256) attn_bwd_finish_kernel(float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long lddq, int S, int H,
                                                               int n_qt, float scale) {
+  chain_next();
+  chain_wait();
   constexpr int PITCH = 136;                        // bytes per staged row: 128 + 8, so that rows start in different banks
   __shared__ __align__(16) uint8_t tile[128 * PITCH];
   const int blk = blockIdx.x;                       // (b * H + head) * n_qt + qi
@@ -749,13 +758,13 @@ void attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, 
   }
   const long long n_chunks = T * H * 8;
   if (!dsum_ready)          // otherwise the producer of d_o has already written -rowsum(d_o * o) (`xsa_bwd` does)
-    attn_bwd_prep_kernel<<<(unsigned)((n_chunks + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, ldo, lddo, dsum, T, S, H);
+    launch_chained(T, attn_bwd_prep_kernel, (unsigned)((n_chunks + 255) / 256), 256, 0, st, (const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, ldo, lddo, dsum, T, S, H);
   const CUtensorMap mq = fused_map(q, ldq, H * hd, T), mk = fused_map(k, ldk, Hkv * hd, T), mv = fused_map(v, ldv, Hkv * hd, T),
                     mdo = fused_map(d_o, lddo, H * hd, T);
-  attn_bwd_fused_kernel<<<std::min(grid, p.rest_w ? grid : p.n_super), F_THREADS, F_SMEM, st>>>(mq, mk, mv, mdo, p);
-  if (p.rest_w) attn_bwd_merge_kernel<<<dim3(grid - 1, 8), 256, 0, st>>>(p, grid);
+  launch_chained(T, attn_bwd_fused_kernel, std::min(grid, p.rest_w ? grid : p.n_super), F_THREADS, F_SMEM, st, mq, mk, mv, mdo, p);
+  if (p.rest_w) launch_chained(T, attn_bwd_merge_kernel, dim3(grid - 1, 8), 256, 0, st, p, grid);
   if (qk) qk_norm_rope_bwd64_acc(dq_acc, *qk, (int)T, H, Hkv, S, p.scale, st);
-  else attn_bwd_finish_kernel<<<B * H * p.n_qt, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, lddq, S, H, p.n_qt, p.scale);
+  else launch_chained(T, attn_bwd_finish_kernel, B * H * p.n_qt, 256, 0, st, dq_acc, (__nv_bfloat16*)dq, lddq, S, H, p.n_qt, p.scale);
 }
 
 }  // namespace pgb

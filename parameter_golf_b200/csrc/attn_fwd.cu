@@ -20,6 +20,7 @@
 #include <atomic>
 #include <cstdlib>
 
+#include "launch.h"
 #include "tma_host.h"
 
 namespace pgb {
@@ -159,6 +160,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_next();
+  chain_wait();
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(A1_REG_ROLE));
@@ -508,7 +511,7 @@ void attn_fwd(const void* q, const void* k, const void* v, void* y, float* lse, 
   }
   p.sched = base + 2 * (sched_next.fetch_add(1, std::memory_order_relaxed) % A1_SCHED_SLOTS);
   const int grid = std::min(p.n_qt * B * H, 2 * sms);
-  attn_fwd_kernel<<<grid, A1_THREADS, A1_SMEM, st>>>(mq, mk, mv, p);
+  launch_chained(T, attn_fwd_kernel, grid, A1_THREADS, A1_SMEM, st, mq, mk, mv, p);
 }
 
 }  // namespace pgb

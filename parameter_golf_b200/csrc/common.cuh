@@ -67,6 +67,15 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// ---- programmatic dependent launch (host side and its range: launch_chained in launch.h) ----------------------------------------------------
+// A kernel launched that way may start while the kernel before it in the stream still runs: its launch latency and its set-up
+// (barriers, tensor-memory allocation, descriptor fetch) are then off the chain of small kernels. `chain_wait` returns once the
+// kernel before has completed and its writes are visible; no thread touches global memory before it, and every thread that does so
+// passes it. `chain_next` lets the kernel after this one start as soon as every CTA has come here. A kernel that allocates tensor
+// memory calls it after the allocation: a CTA of the next kernel, which waits for this one, must not take the columns first.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- mbarrier ----------------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -18,6 +18,7 @@
 // Tile 128 x BN x 64, BN in {64, 128, 256} (`pick_tile`); grid = min(#tiles, #SMs); tile index = n fastest so CTAs
 // working at the same time share the rows of the large operand in L2. The 64-column form has four epilogue warps (6 warps in all).
 #include "common.cuh"
+#include "launch.h"
 #include "pgb.h"
 #include "tma_host.h"
 
@@ -382,6 +383,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_next();
+  chain_wait();
 
   const int tiles_per_batch = p.tiles_m * p.tiles_n * p.splits;
   const int total_tiles = tiles_per_batch * p.batch;
@@ -667,7 +670,7 @@ static void launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const C
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  kern<<<grid, gemm_threads(BN), GemmSmem<BN>::TOTAL, stream>>>(ma, mb, mx, p);
+  launch_chained(std::max(p.M, p.K), kern, grid, gemm_threads(BN), GemmSmem<BN>::TOTAL, stream, ma, mb, mx, p);
 }
 
 template <int BN, int EPI>

@@ -5,6 +5,7 @@
 // module (parameter-golf-rs/crates/pg-kernels/src/gpu_kernels.rs:549-2377, 2429-3610, 5635-5894), each
 // of which was a separate fp32 pass there.
 #include "common.cuh"
+#include "launch.h"
 #include "pgb.h"
 
 namespace pgb {
@@ -60,6 +61,8 @@ __global__ void __launch_bounds__(ROW_THREADS) mix_norm_fwd_kernel(const __nv_bf
                                                                    const __nv_bfloat16* __restrict__ skip, const float* __restrict__ sw,
                                                                    const float* __restrict__ mix, __nv_bfloat16* __restrict__ x_in,
                                                                    __nv_bfloat16* __restrict__ h, int rows, int d, float s, float eps) {
+  chain_next();
+  chain_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int row = blockIdx.x * ROW_WARPS + warp; row < rows; row += gridDim.x * ROW_WARPS) {
     const size_t base = (size_t)row * d;
@@ -876,7 +879,7 @@ static int row_grid(int rows) {
 
 void mix_norm_fwd(const void* x, const void* x0, const void* skip, const float* sw, const float* mix, void* x_in, void* h, int rows, int d, float s,
                   float eps, cudaStream_t st) {
-  PGB_NV_DISPATCH(d, (mix_norm_fwd_kernel<NV><<<row_grid(rows), ROW_THREADS, 0, st>>>(
+  PGB_NV_DISPATCH(d, (launch_chained(rows, mix_norm_fwd_kernel<NV>, row_grid(rows), ROW_THREADS, 0, st, 
                          (const __nv_bfloat16*)x, (const __nv_bfloat16*)x0, (const __nv_bfloat16*)skip, sw, mix, (__nv_bfloat16*)x_in,
                          (__nv_bfloat16*)h, rows, d, s, eps)));
 }

@@ -4,6 +4,7 @@
 //   * per-head RMSNorm + partial RoPE (+ q gain) forward/backward for head_dim 64 with 8 lanes per head
 //     vector (one 16-byte load per lane, fully coalesced) instead of one thread per vector.
 #include "common.cuh"
+#include "launch.h"
 #include "pgb.h"
 
 namespace pgb {
@@ -65,6 +66,8 @@ mix_norm_bwd2_kernel(const __nv_bfloat16* __restrict__ d_h, const __nv_bfloat16*
                      const float* __restrict__ sw, const float* __restrict__ mix, const __nv_bfloat16* __restrict__ add_grad,
                      __nv_bfloat16* __restrict__ d_x, __nv_bfloat16* __restrict__ d_x0, __nv_bfloat16* __restrict__ d_skip, float* __restrict__ d_mix,
                      float* __restrict__ d_sw, int skip_to_dx, int rows, int d, float s, float eps) {
+  chain_next();
+  chain_wait();
   extern __shared__ float sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float am0[MIX ? NV : 1][8], am1[MIX ? NV : 1][8], asw[SKIP ? NV : 1][8];
@@ -183,7 +186,7 @@ static void launch_mnb(const void* d_h, const void* d_res, const void* x_in, con
   {                                                                                                                                       \
     auto kern = mix_norm_bwd2_kernel<NV, MIXF, SKIPF>;                                                                                    \
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                             \
-    kern<<<grid, RT, (MIXF) ? smem : 0, st>>>((const __nv_bfloat16*)d_h, (const __nv_bfloat16*)d_res, (const __nv_bfloat16*)x_in,          \
+    launch_chained(rows, kern, grid, RT, (MIXF) ? smem : 0, st, (const __nv_bfloat16*)d_h, (const __nv_bfloat16*)d_res, (const __nv_bfloat16*)x_in,          \
                                               (const __nv_bfloat16*)x, (const __nv_bfloat16*)x0, (const __nv_bfloat16*)skip, sw, mix,      \
                                               (const __nv_bfloat16*)add_grad, (__nv_bfloat16*)d_x, (__nv_bfloat16*)d_x0,                  \
                                               (__nv_bfloat16*)d_skip, d_mix, d_sw, skip_to_dx, rows, d, s, eps);                          \
@@ -347,6 +350,8 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd64_acc_kernel(float* __re
                                                                      const float* __restrict__ cosT, const float* __restrict__ sinT,
                                                                      const float* __restrict__ gain, float* __restrict__ d_gain, int ld, int H, int Hkv,
                                                                      int rope_dims, int seq_len, float eps, float scale) {
+  chain_next();
+  chain_wait();
   __shared__ __align__(16) float tile[128 * QKA_PITCH];
   __shared__ float sg[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7;
@@ -431,7 +436,7 @@ void qk_norm_rope_bwd64_acc(float* dq_acc, const QkNormRopeBwd& a, int rows, int
   if (!qk_norm_rope_fast_ok(H, 64, a.rope_dims)) throw std::runtime_error("qk_norm_rope: shape outside the head_dim 64 kernel");
   if (seq_len <= 0 || seq_len % 128 || rows % seq_len) throw std::runtime_error("qk_norm_rope: whole sequences of a multiple of 128 tokens only");
   if ((long long)rows * (H + Hkv) > 0x7fffff00ll) throw std::runtime_error("qk_norm_rope: too many head vectors for 32-bit indexing");
-  qk_norm_rope_bwd64_acc_kernel<<<rows / 128 * (H + Hkv), 256, 0, st>>>(dq_acc, (const __nv_bfloat16*)a.d_post, (const __nv_bfloat16*)a.pre,
+  launch_chained(rows, qk_norm_rope_bwd64_acc_kernel, rows / 128 * (H + Hkv), 256, 0, st, dq_acc, (const __nv_bfloat16*)a.d_post, (const __nv_bfloat16*)a.pre,
                                                                         (__nv_bfloat16*)a.d_pre, a.cosT, a.sinT, a.gain, a.d_gain, a.ld, H, Hkv, a.rope_dims,
                                                                         seq_len, a.eps, scale);
 }
@@ -480,6 +485,8 @@ __global__ void __launch_bounds__(256) xsa_bwd64_kernel(const __nv_bfloat16* __r
                                                         const __nv_bfloat16* __restrict__ v, __nv_bfloat16* __restrict__ dy,
                                                         __nv_bfloat16* __restrict__ dv, int accumulate_dv, int nvec, int Hkv, int group, int ld_y,
                                                         int ld_v, int ld_dv, float eps, float* __restrict__ dsum, int seq_len) {
+  chain_next();
+  chain_wait();
   const int sub = threadIdx.x & 7;
   const int vstride = (int)gridDim.x * (blockDim.x / 8);
   const int nvec_pad = (nvec + 3) / 4 * 4;
@@ -545,7 +552,7 @@ void xsa_bwd64(const void* dz, const void* y, const void* v, void* dy, void* dv,
   if ((long long)rows * Hkv > 0x7fffff00ll) throw std::runtime_error("xsa: too many head vectors for 32-bit indexing");
   const int nvec = rows * Hkv;
   const int grid = std::max(1, std::min((nvec + 31) / 32, 148 * 16));
-  xsa_bwd64_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)dz, (const __nv_bfloat16*)y, (const __nv_bfloat16*)v, (__nv_bfloat16*)dy,
+  launch_chained(rows, xsa_bwd64_kernel, grid, 256, 0, st, (const __nv_bfloat16*)dz, (const __nv_bfloat16*)y, (const __nv_bfloat16*)v, (__nv_bfloat16*)dy,
                                          (__nv_bfloat16*)dv, accumulate_dv, nvec, Hkv, group, ld_y, ld_v, ld_dv, eps, dsum, seq_len);
 }
 
