@@ -112,11 +112,13 @@ class CudaEngine:
         if share is not None:
             assert share.dev == self.dev and share.train == train and share.m == self.m
             for name in ("p", "g", "groups", "Wqkv", "Wo", "Wup", "Wd", "Wo_u", "Wd_u", "E", "LM", "BE", "BP", "VE", "VP", "ve_eff", "ema", "mom",
-                         "ns", "Gd", "Go", "Gbp", "Gvp", "fold_open"):
+                         "ns", "Gd", "Go", "Gbp", "Gvp", "fold_open", "fwd_views", "bwd_views"):
                 if hasattr(share, name):
                     setattr(self, name, getattr(share, name))
         else:
             self._alloc_params(params)
+            self.make_layer_views()
+        self.xsa_set = frozenset(self.m.xsa_layers())
         self._alloc_acts()
         # Pinned staging for the per-step hyper-parameters: a ring of buffers, each guarded by the event recorded after its
         # asynchronous upload, so that a host that runs ahead of the stream (no per-step synchronisation, graph replay)
@@ -245,6 +247,19 @@ class CudaEngine:
             if m.value_embedding.enabled:
                 self.Gvp = torch.zeros(kv, m.value_embedding.dim, dtype=torch.float32, device=dev)
 
+    def make_layer_views(self):
+        """Per-layer slices of the weights, controls and gradients, made once: indexing a tensor costs the host about as much as
+        launching a small kernel (~1.3 us), and a block uses a dozen of them. Call again after replacing any of that storage."""
+        p, n, d = self.p, self.n, self.d
+        self.fwd_views = [(p["resid_mix"][l], p["q_gain"][l], self.Wqkv[l], self.Wo[l], self.Wup[l], self.Wd[l]) for l in range(n)]
+        self.bwd_views = []
+        if self.train:
+            g = self.g
+            self.bwd_views = [{"down": (self.Wd_u[l], p["mlp_scale"][l], 1, d, g["mlp_down_bank"][l], g["mlp_scale"][l]), "up": g["mlp_up_bank"][l],
+                               "o": (self.Wo_u[l], p["attn_scale"][l], 1, d, g["qo_bank"][n + l], g["attn_scale"][l]), "q": g["qo_bank"][l],
+                               "kv": ((d, g["kv_bank"][l]), (d + self.kv, g["kv_bank"][n + l])), "gain": g["q_gain"][l], "mix": g["resid_mix"][l]}
+                              for l in range(n)]
+
     def _alloc_acts(self):
         dev, T, d, n = self.dev, self.T, self.d, self.n
 
@@ -290,6 +305,10 @@ class CudaEngine:
 
         self.x_in, self.h = per_layer(T, d), per_layer(T, d)
         self.qkv_pre, self.qk_post = per_layer(T, self.qkvw), per_layer(T, self.qkvw)
+        # query, key and value columns of each set, sliced once (see `make_layer_views`)
+        self.q_cols = [t[:, :d] for t in self.qk_post]
+        self.k_cols = [t[:, d:d + self.kv] for t in self.qk_post]
+        self.v_cols = [t[:, d + self.kv:] for t in self.qkv_pre]
         self.y, self.x_mid = per_layer(T, d), per_layer(T, d)
         self.mm = self.h if self.parallel else per_layer(T, d)      # parallel residual: the MLP reads the attention branch's normed input
         xsa_sets = {self.act_slot[j] for j, (l, _) in enumerate(self.sched) if l in m.xsa_layers()} if self.train else ({0} if m.xsa_last_n > 0 else set())
@@ -469,31 +488,27 @@ class CudaEngine:
     # ---- attention -----------------------------------------------------------------------------------------------------
     def _attn_fwd(self, l, li):
         d, kv, B, S, H, Hkv, hd = self.d, self.kv, self.B, self.S, self.H, self.Hkv, self.hd
-        q = self.qk_post[li][:, :d]
-        k = self.qk_post[li][:, d:d + kv]
-        v = self.qkv_pre[li][:, d + kv:]
+        q, k, v = self.q_cols[li], self.k_cols[li], self.v_cols[li]
         # exclusive self attention: the projection off the token's own value vector is applied to the accumulator in the
         # attention kernel's output stage, which writes both y (the backward needs it) and z
-        z = self.z[li] if l in self.m.xsa_layers() else None
+        z = self.z[li] if l in self.xsa_set else None
         self.lse[li] = N.attn_fwd(q, k, v, self.y[li], B, S, H, Hkv, hd, self.lse[li], z, 1e-8)
 
     def _attn_bwd(self, l, j):
         """Attention backward and the backward of the per-head norm, rotation and query gain: ``d_qkv_pre`` is complete afterwards."""
         d, kv, B, S, H, Hkv, hd = self.d, self.kv, self.B, self.S, self.H, self.Hkv, self.hd
         m = self.m
-        gain, d_gain = self.p["q_gain"][l], self.g["q_gain"][l]
+        gain, d_gain = self.fwd_views[l][1], self.bwd_views[l]["gain"]
         if self.dq_acc is not None and hd == 64 and H <= 64 and m.rope_dims % 16 == 0 and m.rope_dims <= 64:
             # the attention kernel's fp32 query accumulator feeds the norm / rotation backward directly
-            xsa = l in m.xsa_layers()
+            xsa = l in self.xsa_set
             self.C.attn_bwd_qk(self.qk_post[j], self.qkv_pre[j], self.y[j], self.d_y, self.lse[j], self.dsum, self.dq_acc, self.d_qk_post, self.d_qkv_pre,
                                self.cos, self.sin, gain, d_gain, B, S, H, Hkv, m.rope_dims, self.eps, xsa, N.status_word(self.dev), xsa, self.bwd_part)
             return
-        q = self.qk_post[j][:, :d]
-        k = self.qk_post[j][:, d:d + kv]
-        v = self.qkv_pre[j][:, d + kv:]
+        q, k, v = self.q_cols[j], self.k_cols[j], self.v_cols[j]
         dq, dk = self.d_qk_post[:, :d], self.d_qk_post[:, d:d + kv]
         dv = self.d_qkv_pre[:, d + kv:]
-        xsa = l in self.m.xsa_layers()
+        xsa = l in self.xsa_set
         # in XSA layers `xsa_bwd` has just produced d_y and, in the same pass, the -rowsum(d_y * y) term of the single-pass form
         N.attn_bwd(q, k, v, self.y[j], self.d_y, self.lse[j], dq, dk, dv, B, S, H, Hkv, hd, accumulate_dv=xsa, dsum=self.dsum,
                    dq_acc=self.dq_acc, reproducible=self.t.reproducible_backward, dsum_ready=xsa and not self.t.reproducible_backward)
@@ -508,7 +523,8 @@ class CudaEngine:
         l, rep = self.sched[j]
         li = self.act_slot[j] if self.train else 0
         s_l = gpt.layer_ln_scale(m, l)
-        C.mix_norm_fwd(x, self.x0, skip, sw, p["resid_mix"][l], self.x_in[li], self.h[li], s_l, self.eps)
+        mix, gain, Wqkv, Wo, Wup, Wd = self.fwd_views[l]
+        C.mix_norm_fwd(x, self.x0, skip, sw, mix, self.x_in[li], self.h[li], s_l, self.eps)
         # Per-head RMSNorm, partial RoPE and the query gain run in the output stage of the QKV product unless something has to
         # touch the raw queries first (a Q-LoRA adapter) or the shape is outside what that stage handles.
         fused_qk = self.lora is None and N.qkv_epilogue_supported(self.hd, m.rope_dims)
@@ -523,10 +539,10 @@ class CudaEngine:
                     self.layer_wait_needed = False
             wait = dict(wait_flag=self.layer_flags[l:l + 1], wait_value=self.layer_flag_value)
         if fused_qk:
-            N.gemm_qkv_norm_rope(self.h[li], self.Wqkv[l], self.qkv_pre[li], self.qk_post[li], self.cos, self.sin, p["q_gain"][l], self.H, self.Hkv,
+            N.gemm_qkv_norm_rope(self.h[li], Wqkv, self.qkv_pre[li], self.qk_post[li], self.cos, self.sin, gain, self.H, self.Hkv,
                                  m.rope_dims, S, self.eps, **wait)
         else:
-            N.gemm(self.h[li], self.Wqkv[l], self.qkv_pre[li], **wait)
+            N.gemm(self.h[li], Wqkv, self.qkv_pre[li], **wait)
         if m.value_embedding.enabled and l in m.value_embedding.layers:
             vi = m.value_embedding.layers.index(l)
             vview = self.qkv_pre[li][:, d + kv:]
@@ -534,21 +550,21 @@ class CudaEngine:
         if self.lora is not None:
             self._lora_fwd(l, li)
         if not fused_qk:
-            C.qk_norm_rope_fwd(self.qkv_pre[li], self.qk_post[li], self.cos, self.sin, p["q_gain"][l], self.H, self.Hkv, self.hd, m.rope_dims, S, self.eps)
+            C.qk_norm_rope_fwd(self.qkv_pre[li], self.qk_post[li], self.cos, self.sin, gain, self.H, self.Hkv, self.hd, m.rope_dims, S, self.eps)
         self._attn_fwd(l, li)
-        zz = self.z[li] if l in m.xsa_layers() else self.y[li]
+        zz = self.z[li] if l in self.xsa_set else self.y[li]
         for gi, (wname, bname, gscale_, gmult) in enumerate(self.gates):
             out = self.yg[gi][li]
             C.head_gate_fwd(zz, self.h[li], p[wname][l], p[bname][l] if bname else None, out, self.gv[gi][li], self.H, self.hd, gscale_, gmult)
             zz = out
         self.zz[li] = zz
-        N.gemm(zz, self.Wo[l], self.x_mid[li], epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_in[li])
+        N.gemm(zz, Wo, self.x_mid[li], epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_in[li])
         if not self.parallel:
             C.mix_norm_fwd(self.x_mid[li], None, None, None, None, None, self.mm[li], s_l, self.eps)
-        N.gemm(self.mm[li], self.Wup[l], self.hu[li], epi=N.EPI_ACT_SQ, slope=self.slope, D2=self.a[li])
+        N.gemm(self.mm[li], Wup, self.hu[li], epi=N.EPI_ACT_SQ, slope=self.slope, D2=self.a[li])
         xo = self.x_out[j]
         if not recompute:
-            N.gemm(self.a[li], self.Wd[l], xo, epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_mid[li])
+            N.gemm(self.a[li], Wd, xo, epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_mid[li])
         return xo
 
     # ---- forward -------------------------------------------------------------------------------------------------------------
@@ -577,7 +593,6 @@ class CudaEngine:
                          S, -1 if bid is None else bid, self.eps)
         x = self.x0
         skips: List[torch.Tensor] = []
-        xsa_layers = m.xsa_layers()
         for j, (l, rep) in enumerate(self.sched):
             skip = sw = None
             if self.unet and l >= self.enc and rep == 0 and skips:
@@ -648,21 +663,23 @@ class CudaEngine:
                 self._dw(self.logits, self.hf, g["tok_emb"] if m.tie_embeddings else g["lm_head"])
         C.mix_norm_bwd(self.d_h, None, self.x_last, None, None, None, None, None, None, self.dx, None, None, None, None, False, 1.0, self.eps)
         self.d_x0.zero_()
-        xsa_layers = m.xsa_layers()
+        xsa_layers = self.xsa_set
+        dv = self.d_qkv_pre[:, d + kv:]
         for j in range(self.nslots - 1, -1, -1):
             l, rep = self.sched[j]
             s_l = gpt.layer_ln_scale(m, l)
             aj = self.act_slot[j]
             if not self.saved[j]:
                 self._block_fwd(j, *self.block_in[j], recompute=True)
+            mix, _, Wqkv, Wo, Wup, Wd = self.fwd_views[l]
+            view = self.bwd_views[l]
             # ---- MLP
             if self._wants("mlp_down_bank", "mlp_scale"):
-                self._dw_folded(self.dx, self.a[aj], self.Gd, C.fold_scaled_grad_bf16, self.Wd_u[l], p["mlp_scale"][l], 1, d, g["mlp_down_bank"][l],
-                                g["mlp_scale"][l])
-            N.gemm(self.dx, self.Wd[l], self.d_hu, True, False, N.EPI_MUL_ACTGRAD, slope=self.slope, aux=self.hu[aj])
+                self._dw_folded(self.dx, self.a[aj], self.Gd, C.fold_scaled_grad_bf16, *view["down"])
+            N.gemm(self.dx, Wd, self.d_hu, True, False, N.EPI_MUL_ACTGRAD, slope=self.slope, aux=self.hu[aj])
             if self._wants("mlp_up_bank"):
-                self._dw(self.d_hu, self.mm[aj], g["mlp_up_bank"][l])
-            N.gemm(self.d_hu, self.Wup[l], self.d_m, True, False)
+                self._dw(self.d_hu, self.mm[aj], view["up"])
+            N.gemm(self.d_hu, Wup, self.d_m, True, False)
             if self.parallel:
                 dx_mid, dx_next = self.dx, self.dx_mid      # no norm between x_mid and the MLP: the residual gradient passes through
                 d_hx = self.d_m                             # and the MLP-input gradient joins the QKV-input gradient below
@@ -673,12 +690,11 @@ class CudaEngine:
             # ---- attention output projection
             zz = self.zz[aj]
             if self._wants("qo_bank", "attn_scale"):
-                self._dw_folded(dx_mid, zz, self.Go, C.fold_scaled_grad_bf16, self.Wo_u[l], p["attn_scale"][l], 1, d, g["qo_bank"][n + l], g["attn_scale"][l])
-            vview = self.qkv_pre[aj][:, d + kv:]
-            dv = self.d_qkv_pre[:, d + kv:]
+                self._dw_folded(dx_mid, zz, self.Go, C.fold_scaled_grad_bf16, *view["o"])
+            vview = self.v_cols[aj]
             xsa = l in xsa_layers
             d_att = self.d_z if xsa else self.d_y            # gradient of what the gates / the output projection consumed
-            N.gemm(dx_mid, self.Wo[l], d_att, True, False)
+            N.gemm(dx_mid, Wo, d_att, True, False)
             for gi in range(len(self.gates) - 1, -1, -1):
                 wname, bname, gscale_, gmult = self.gates[gi]
                 gate_in = self.yg[gi - 1][aj] if gi > 0 else (self.z[aj] if xsa else self.y[aj])
@@ -706,11 +722,11 @@ class CudaEngine:
                 self.d_ve_acc.add_(self.d_ve_e)
             # one weight-gradient product for the packed QKV rows, written to the Q, K and V slots of the gradient banks
             if self._wants("qo_bank", "kv_bank"):
-                self._dw(self.d_qkv_pre, self.h[aj], g["qo_bank"][l], segs=((d, g["kv_bank"][l]), (d + kv, g["kv_bank"][n + l])))
+                self._dw(self.d_qkv_pre, self.h[aj], view["q"], segs=view["kv"])
             if d_hx is not None:
-                N.gemm(self.d_qkv_pre, self.Wqkv[l], self.d_h, True, False, N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=d_hx)
+                N.gemm(self.d_qkv_pre, Wqkv, self.d_h, True, False, N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=d_hx)
             else:
-                N.gemm(self.d_qkv_pre, self.Wqkv[l], self.d_h, True, False)
+                N.gemm(self.d_qkv_pre, Wqkv, self.d_h, True, False)
             if self.lora is not None:
                 self._lora_bwd(l, aj)
             # ---- block input: RMSNorm backward, residual mix, U-Net skip
@@ -728,8 +744,8 @@ class CudaEngine:
                 lp = self.sched[j - 1][0]                        # x_prev is the (last-pass) output of an encoder layer whose skip
                 if lp != l and lp < self.enc and self.first_slot.get(2 * self.enc - 1 - lp, -1) not in (-1, j):   # consumer is further up
                     add_grad = self.d_skip[lp]
-            C.mix_norm_bwd(self.d_h, dx_mid, self.x_in[aj], x_prev, self.x0, skip, sw, p["resid_mix"][l], add_grad, dx_next, self.d_x0, d_skip,
-                           g["resid_mix"][l], d_sw, self_pair, s_l, self.eps)
+            C.mix_norm_bwd(self.d_h, dx_mid, self.x_in[aj], x_prev, self.x0, skip, sw, mix, add_grad, dx_next, self.d_x0, d_skip,
+                           view["mix"], d_sw, self_pair, s_l, self.eps)
             if self.parallel:
                 self.dx, self.dx_mid = self.dx_mid, self.dx
             if self.backward_observer is not None:

@@ -124,6 +124,9 @@ _status = {}
 
 def status_word(device=None) -> torch.Tensor:
     """Per-device int32[4] status word that bounded waits write to: [code, block, detail, count]."""
+    st = _status.get(device)                              # a device that names its index, as a tensor's does
+    if st is not None:
+        return st
     dev = torch.device(device if device is not None else f"cuda:{torch.cuda.current_device()}")
     if dev.type == "cuda" and dev.index is None:          # "cuda" and "cuda:N" must name the same word
         dev = torch.device("cuda", torch.cuda.current_device())

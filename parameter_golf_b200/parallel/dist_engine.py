@@ -118,6 +118,7 @@ class DistributedStep:
             new = self.wbuf.view(self.w_off[name] * 2, old.shape, BF)
             new.copy_(old)
             setattr(e, name, new)
+        e.make_layer_views()               # weights and gradients have new storage
         self.sig = SymmetricBuffer(1024 * 4, group)
         self.val = SymmetricBuffer(256 * 4, group)
         self.sig_local = self.sig.view(0, (1024,), torch.int32)
