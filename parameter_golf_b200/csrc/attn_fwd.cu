@@ -535,13 +535,13 @@ __global__ void __launch_bounds__(256) attn_fwd_merge_kernel(const AttnFwdParams
 
 // Key tiles per chunk, or 0 where query tiles stay whole. A tile's key range is a serial chain of ~1.7 us per key tile, and the longest
 // chain is the kernel's time when there are few items: B = 1, S = 2048, H = 8 has 128 items for 296 CTAs, the longest of 16
-// key tiles, against 3.7 per CTA on average. Chunks of about the average (at least 4: a chunk costs its slot's traffic and a share of
-// the merge) are used where the longest chain is at least 1.5 times that.
+// key tiles, against 3.7 per CTA on average. Chunks of about the average, at least 4, are used where they shorten the longest chain by
+// at least six key tiles: slots and merge cost about 8 us, as much as five (5 x 896 tokens, 7 key tiles cut at 4, lost 3 us per call).
 static int fwd_chunk(int B, int S, int H, int sms) {
   const int n_qt = S / AT_BM;
   const long long units = (long long)B * H * n_qt * (n_qt + 1) / 2;
   const long long even = std::max(4ll, (units + 2 * sms - 1) / (2 * sms));
-  return 2 * n_qt >= 3 * even ? (int)even : 0;
+  return n_qt - even >= 6 ? (int)even : 0;
 }
 static int fwd_items(int B, int S, int H, int chunk) {
   const int n_qt = S / AT_BM;
