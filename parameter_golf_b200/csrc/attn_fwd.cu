@@ -45,12 +45,7 @@ struct AttnFwdParams {
   const __nv_bfloat16* V;
   long long ldv;
   float xsa_eps;
-  // Query tiles of more than `chunk` key tiles are cut into chunks (0: none): each chunk is a work item that leaves its unnormalised
-  // output and {maximum, sum} of every row in its slot of `part`, and attn_fwd_merge_kernel combines them.
-  int chunk, n_items;
-  float* part;
 };
-constexpr int AT_PART = AT_BM * AT_HD + 2 * AT_BM;       // floats per slot: 16 column chunks x 128 rows x 4, then maxima, then sums
 
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
@@ -91,30 +86,17 @@ static_assert(128 * A1_REG_ROLE + 128 * A1_REG_SOFTMAX == A1_THREADS * A1_REG_LA
 static_assert(2 * (A1_SMEM + 1024) <= 227 * 1024, "two CTAs must fit the shared memory of one SM");
 
 struct FwdItem {
-  int qt, b, head, kvh, n_kv, row0, j0, slot;      // key tiles j0 .. j0 + n_kv - 1; slot of a partial result or -1
+  int qt, b, head, kvh, n_kv, row0;
 };
 __device__ __forceinline__ FwdItem fwd_item(const AttnFwdParams& p, int item) {
   FwdItem w;
   const int per_qt = p.B * p.H;
-  int pos = item / per_qt;
-  w.j0 = 0;
-  if (p.chunk > 0) {                         // first chunks of all query tiles, then the second ones of those that have one, ...
-    for (int count = p.n_qt; pos >= count; count -= p.chunk) {
-      pos -= count;
-      w.j0 += p.chunk;
-    }
-  }
-  w.qt = p.n_qt - 1 - pos;                   // heavy (long KV range) query tiles first
+  w.qt = p.n_qt - 1 - item / per_qt;         // heavy (long KV range) query tiles first
   const int rem = item % per_qt;
   w.b = rem / p.H;
   w.head = rem % p.H;                        // the heads of a KV group are neighbours, so their K/V fetches share L2 lines
   w.kvh = w.head / (p.H / p.Hkv);
-  w.n_kv = w.qt + 1 - w.j0;
-  w.slot = -1;
-  if (p.chunk > 0 && w.qt >= p.chunk) {
-    w.n_kv = min(w.n_kv, p.chunk);
-    w.slot = item;
-  }
+  w.n_kv = w.qt + 1;
   w.row0 = w.b * p.S + w.qt * AT_BM;
   return w;
 }
@@ -151,7 +133,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   volatile int* sched_item = abort_flag + 1;   // 2 slots; -1 ends the list
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_items = p.n_items;
+  const int n_items = p.n_qt * p.B * p.H;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
@@ -206,11 +188,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         for (int j = 0; j < w.n_kv; ++j) {
           if (!mbar_wait(&k_empty[ks], kph ^ 1, abort_flag, p.status, ST_WAIT_EMPTY, j)) { ok = false; break; }
           mbar_expect_tx(&k_full[ks], AT_TILE_BYTES);
-          tma_load_2d(sK + ks * AT_TILE_BYTES, &map_k, &k_full[ks], w.kvh * AT_HD, w.b * p.S + (w.j0 + j) * AT_BN);
+          tma_load_2d(sK + ks * AT_TILE_BYTES, &map_k, &k_full[ks], w.kvh * AT_HD, w.b * p.S + j * AT_BN);
           if (++ks == A1_KST) { ks = 0; kph ^= 1; }
           if (!mbar_wait(&v_empty[vs], vph ^ 1, abort_flag, p.status, ST_WAIT_EMPTY, j)) { ok = false; break; }
           mbar_expect_tx(&v_full[vs], AT_TILE_BYTES);
-          tma_load_2d(sV + vs * AT_TILE_BYTES, &map_v, &v_full[vs], w.kvh * AT_HD, w.b * p.S + (w.j0 + j) * AT_BN);
+          tma_load_2d(sV + vs * AT_TILE_BYTES, &map_v, &v_full[vs], w.kvh * AT_HD, w.b * p.S + j * AT_BN);
           if (++vs == A1_VST) { vs = 0; vph ^= 1; }
         }
       }
@@ -298,15 +280,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     FwdItem wp = {};
     float m_p = 0.f, l_p = 1.f;
     auto store_out = [&](const uint32_t* o, const FwdItem& w, float m, float lsum) {
-      if (w.slot >= 0) {
-        float* part = p.part + (size_t)w.slot * AT_PART;
-#pragma unroll
-        for (int c = 0; c < 16; ++c)
-          reinterpret_cast<uint4*>(part)[c * AT_BM + r] = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
-        part[AT_BM * AT_HD + r] = m;
-        part[AT_BM * AT_HD + AT_BM + r] = lsum;
-        return;
-      }
       const float inv = 1.f / lsum;
       __nv_bfloat16* yrow = p.Y + (size_t)(w.row0 + r) * p.ldy + w.head * AT_HD;
 #pragma unroll
@@ -368,7 +341,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(s_free);          // the scores are in registers: the next tile's may overwrite them
-        if (w.j0 + j == w.qt) {
+        if (j == w.qt) {
 #pragma unroll
           for (int c = 0; c < 128; ++c)
             if (c > r) s[c] = 0xff800000u;            // -inf
@@ -482,88 +455,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   }
 }
 
-// Rows of a query tile whose key range was cut: O = sum_i 2^(m_i - M) O_i, l = sum_i 2^(m_i - M) l_i with M = max m_i, then the same output
-// as the uncut form. Eight lanes per row, 32 rows per CTA.
-__global__ void __launch_bounds__(256) attn_fwd_merge_kernel(const AttnFwdParams p) {
-  chain_next();
-  chain_wait();
-  const int sub = threadIdx.x & 7, r = (blockIdx.x & 3) * 32 + (threadIdx.x >> 3);
-  const int per_qt = p.B * p.H;
-  const int t = blockIdx.x >> 2, qt = p.n_qt - 1 - t / per_qt, rem = t % per_qt, b = rem / p.H, head = rem % p.H, kvh = head / (p.H / p.Hkv);
-  float M = -INFINITY;
-  int item = t;                                      // the tile's chunks: each round of chunks is `chunk` query tiles shorter than the last
-  for (int j0 = 0, count = p.n_qt; j0 <= qt; j0 += p.chunk, item += count * per_qt, count -= p.chunk)
-    M = fmaxf(M, p.part[(size_t)item * AT_PART + AT_BM * AT_HD + r]);
-  float o[8] = {}, l = 0.f;
-  item = t;
-  for (int j0 = 0, count = p.n_qt; j0 <= qt; j0 += p.chunk, item += count * per_qt, count -= p.chunk) {
-    const float* part = p.part + (size_t)item * AT_PART;
-    const float f = ex2(part[AT_BM * AT_HD + r] - M);
-    l += f * part[AT_BM * AT_HD + AT_BM + r];
-    const float4 a = reinterpret_cast<const float4*>(part)[2 * sub * AT_BM + r], c = reinterpret_cast<const float4*>(part)[(2 * sub + 1) * AT_BM + r];
-    o[0] += f * a.x; o[1] += f * a.y; o[2] += f * a.z; o[3] += f * a.w;
-    o[4] += f * c.x; o[5] += f * c.y; o[6] += f * c.z; o[7] += f * c.w;
-  }
-  const float inv = 1.f / l;
-  const size_t row = (size_t)b * p.S + qt * AT_BM + r;
-  *reinterpret_cast<uint4*>(p.Y + row * p.ldy + head * AT_HD + sub * 8) =
-      make_uint4(pack_bf16x2(o[0] * inv, o[1] * inv), pack_bf16x2(o[2] * inv, o[3] * inv), pack_bf16x2(o[4] * inv, o[5] * inv), pack_bf16x2(o[6] * inv, o[7] * inv));
-  if (sub == 0) p.lse[((size_t)b * p.H + head) * p.S + qt * AT_BM + r] = -(M + log2f(l));
-  if (p.Z != nullptr) {
-    const uint4 q = *reinterpret_cast<const uint4*>(p.V + row * p.ldv + kvh * AT_HD + sub * 8);
-    const float2 v0 = unpack_bf16x2(q.x), v1 = unpack_bf16x2(q.y), v2 = unpack_bf16x2(q.z), v3 = unpack_bf16x2(q.w);
-    const float v[8] = {v0.x, v0.y, v1.x, v1.y, v2.x, v2.y, v3.x, v3.y};
-    float n = 0.f, dot = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      n += v[e] * v[e];
-      dot += o[e] * v[e];
-    }
-#pragma unroll
-    for (int s = 1; s < 8; s *= 2) {
-      n += __shfl_xor_sync(0xffffffffu, n, s);
-      dot += __shfl_xor_sync(0xffffffffu, dot, s);
-    }
-    const float coef = dot * inv / (n + p.xsa_eps);
-    float z[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) z[e] = o[e] * inv - coef * v[e];
-    *reinterpret_cast<uint4*>(p.Z + row * p.ldz + head * AT_HD + sub * 8) =
-        make_uint4(pack_bf16x2(z[0], z[1]), pack_bf16x2(z[2], z[3]), pack_bf16x2(z[4], z[5]), pack_bf16x2(z[6], z[7]));
-  }
-}
-
-// Key tiles per chunk, or 0 where query tiles stay whole. A tile's key range is a serial chain of ~1.7 us per key tile, and the longest
-// chain is the kernel's time when there are few items: B = 1, S = 2048, H = 8 has 128 items for 296 CTAs, the longest of 16
-// key tiles, against 3.7 per CTA on average. Chunks of about the average, at least 4, are used where they shorten the longest chain by
-// at least six key tiles: slots and merge cost about 8 us, as much as five (5 x 896 tokens, 7 key tiles cut at 4, lost 3 us per call).
-static int fwd_chunk(int B, int S, int H, int sms) {
-  const int n_qt = S / AT_BM;
-  const long long units = (long long)B * H * n_qt * (n_qt + 1) / 2;
-  const long long even = std::max(4ll, (units + 2 * sms - 1) / (2 * sms));
-  return n_qt - even >= 6 ? (int)even : 0;
-}
-static int fwd_items(int B, int S, int H, int chunk) {
-  const int n_qt = S / AT_BM;
-  int tiles = 0;
-  for (int count = n_qt; count > 0; count -= chunk) {
-    tiles += count;
-    if (chunk == 0) break;
-  }
-  return tiles * B * H;
-}
-static int fwd_sms() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-size_t attn_fwd_part_floats(int B, int S, int H) {
-  if (B <= 0 || H <= 0 || S < AT_BM) return 0;
-  const int chunk = fwd_chunk(B, S, H, fwd_sms());
-  return chunk ? (size_t)fwd_items(B, S, H, chunk) * AT_PART : 0;
-}
-
 static CUtensorMap attn_map(const void* ptr, long long ld, int cols, long long rows) {
   uint64_t dims[2] = {(uint64_t)cols, (uint64_t)rows};
   uint64_t strides[1] = {(uint64_t)ld * 2};
@@ -572,7 +463,7 @@ static CUtensorMap attn_map(const void* ptr, long long ld, int cols, long long r
 }
 
 void attn_fwd(const void* q, const void* k, const void* v, void* y, float* lse, long long ldq, long long ldk, long long ldv, long long ldy, int B,
-              int S, int H, int Hkv, int hd, int* status, cudaStream_t st, void* z, long long ldz, float xsa_eps, float* part) {
+              int S, int H, int Hkv, int hd, int* status, cudaStream_t st, void* z, long long ldz, float xsa_eps) {
   if (hd != AT_HD) throw std::runtime_error("attention kernel is specialised for head_dim 64");
   if (S % 128) throw std::runtime_error("attention kernel needs seq_len to be a multiple of 128");
   if (H % Hkv) throw std::runtime_error("num_heads must be divisible by num_kv_heads");
@@ -619,13 +510,8 @@ void attn_fwd(const void* q, const void* k, const void* v, void* y, float* lse, 
     }
   }
   p.sched = base + 2 * (sched_next.fetch_add(1, std::memory_order_relaxed) % A1_SCHED_SLOTS);
-  // the merge reads and writes whole 16-byte pieces of the output rows, which the kernel itself does too
-  p.chunk = part ? fwd_chunk(B, S, H, sms) : 0;
-  p.part = part;
-  p.n_items = fwd_items(B, S, H, p.chunk);
-  const int grid = std::min(p.n_items, 2 * sms);
+  const int grid = std::min(p.n_qt * B * H, 2 * sms);
   launch_chained(T, attn_fwd_kernel, grid, A1_THREADS, A1_SMEM, st, mq, mk, mv, p);
-  if (p.chunk) launch_chained(T, attn_fwd_merge_kernel, (p.n_qt - p.chunk) * B * H * 4, 256, 0, st, p);
 }
 
 }  // namespace pgb

@@ -180,9 +180,7 @@ void gptq_rows(const float* Wp, const float* U, const float* scales, int8_t* Q, 
 // base-2 log-sum-exp of the scaled scores (the form the backward kernels feed straight into their FMAs).
 // z (optional): second output with the exclusive-self-attention projection applied, z_h = y_h - (<y_h, v> / (|v|^2 + eps)) v
 void attn_fwd(const void* q, const void* k, const void* v, void* y, float* lse, long long ldq, long long ldk, long long ldv, long long ldy, int B,
-              int S, int H, int Hkv, int hd, int* status, cudaStream_t st, void* z = nullptr, long long ldz = 0, float xsa_eps = 0.f, float* part = nullptr);
-// floats of `part` (no initial value needed) that let a small batch cut long key ranges; 0 where it would not
-size_t attn_fwd_part_floats(int B, int S, int H);
+              int S, int H, int Hkv, int hd, int* status, cudaStream_t st, void* z = nullptr, long long ldz = 0, float xsa_eps = 0.f);
 // dsum: fp32 [B, H, S] scratch-free side output (rowsum(dO * O)), written by the dQ kernel and read by the dK/dV kernel.
 void attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse, float* dsum, void* dq, void* dk, void* dv,
               long long ldq, long long ldk, long long ldv, long long ldo, long long lddo, long long lddq, long long lddk, long long lddv, int B, int S,

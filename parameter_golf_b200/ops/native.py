@@ -177,13 +177,7 @@ def attn_fwd(q, k, v, y, B, S, H, Hkv, hd, lse=None, z=None, xsa_eps=1e-8):
     accumulator it already holds (`xsa_fwd` as a separate pass is then not needed)."""
     if lse is None:
         lse = torch.empty(B, H, S, dtype=torch.float32, device=q.device)
-    C = load()
-    need = C._mod.attn_fwd_part_floats(B, S, H)
-    if need:                                              # a small batch: long key ranges are cut and merged by a second kernel
-        C.launches += 1
-        C.attn_fwd(q, k, v, y, lse, B, S, H, Hkv, hd, status_word(q.device), z, xsa_eps, torch.empty(need, dtype=torch.float32, device=q.device))
-    else:
-        C.attn_fwd(q, k, v, y, lse, B, S, H, Hkv, hd, status_word(q.device), z, xsa_eps)
+    load().attn_fwd(q, k, v, y, lse, B, S, H, Hkv, hd, status_word(q.device), z, xsa_eps)
     return lse
 
 

@@ -676,3 +676,18 @@ def test_gradients_of_some_parameters_are_those_of_all(names):
         assert float((some[k] - full[k]).norm()) <= 1e-4 * float(full[k].norm()) + 1e-12, k
     for k in full:
         assert float((again[k] - full[k]).norm()) <= 1e-4 * float(full[k].norm()) + 1e-12, k
+
+
+@pytest.mark.parametrize("S", [128, 1280])
+def test_a_window_scores_the_same_alone_and_in_a_batch(S):
+    """Scoring one window by itself, in a ragged last batch or among many gives the same bits: no sum over features, keys or
+    vocabulary is cut by the number of sequences."""
+    from parameter_golf_b200.models import gpt
+    from parameter_golf_b200.models.engine import EngineRunner
+    spec = small_spec(**{"model.train_seq_len": S, "model.eval_seq_len": S, "train.seq_len": S, "train.batch_tokens": 4 * S})
+    r = EngineRunner(spec, gpt.fill_deterministic(spec.model), "cuda", batch=12, train=False)
+    torch.manual_seed(S)
+    ids, tgt = torch.randint(0, 256, (12, S)), torch.randint(0, 256, (12, S))
+    whole = r.nll(ids, tgt)
+    for lo, hi in ((0, 1), (11, 12), (4, 7)):
+        assert torch.equal(r.nll(ids[lo:hi], tgt[lo:hi]), whole[lo:hi]), (lo, hi)
