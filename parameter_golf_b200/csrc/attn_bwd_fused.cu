@@ -399,7 +399,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         for (int u = 0; u < it.nu; ++u, up.next()) {
           const int stage = up.stage;
           const size_t vidx = ((size_t)it.b * p.H + head) * p.S + qi * 128 + lane * 4;
-          const float4 l4 = *reinterpret_cast<const float4*>(p.lse + vidx), d4 = *reinterpret_cast<const float4*>(p.Dsum + vidx);
+          const float4 l4 = __ldcg(reinterpret_cast<const float4*>(p.lse + vidx)), d4 = __ldcg(reinterpret_cast<const float4*>(p.Dsum + vidx));
           if (!mbar_wait(&st_empty[stage], up.phase ^ 1, abort_flag, p.status, ST_WAIT_EMPTY, u, F_BACKOFF_NS)) { ok = false; break; }
           uint8_t* tl = sBX + stage * 2 * F_BIAS_TILE;
           const float lv[4] = {l4.x * inv_c, l4.y * inv_c, l4.z * inv_c, l4.w * inv_c}, dv4[4] = {d4.x, d4.y, d4.z, d4.w};
@@ -609,10 +609,10 @@ __global__ void __launch_bounds__(256) attn_bwd_merge_kernel(const FusedParams p
     const int i = blockIdx.y * 256 + threadIdx.x;                        // (dK | dV, row, 8 columns), 2 x 128 x 8 over grid.y
     const int oc = i & 7, r = (i >> 3) & 127, which = i >> 10;
     const size_t off = (size_t)which * 2048 + oc * 256 + r;
-    float4 x0 = part[(size_t)(2 * (c - 1) + 1) * 4096 + off], x1 = part[(size_t)(2 * (c - 1) + 1) * 4096 + off + 128];
+    float4 x0 = __ldcg(part + (size_t)(2 * (c - 1) + 1) * 4096 + off), x1 = __ldcg(part + (size_t)(2 * (c - 1) + 1) * 4096 + off + 128);
     for (int k = c; k < ctas && f_range_start(p, k, ctas) < first + nu; ++k) {
       if (f_range_start(p, k, ctas) == f_range_start(p, k + 1, ctas)) continue;      // fewer units than CTAs: an empty range
-      const float4 y0 = part[(size_t)(2 * k) * 4096 + off], y1 = part[(size_t)(2 * k) * 4096 + off + 128];
+      const float4 y0 = __ldcg(part + (size_t)(2 * k) * 4096 + off), y1 = __ldcg(part + (size_t)(2 * k) * 4096 + off + 128);
       x0.x += y0.x; x0.y += y0.y; x0.z += y0.z; x0.w += y0.w;
       x1.x += y1.x; x1.y += y1.y; x1.z += y1.z; x1.w += y1.w;
     }
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(256) attn_bwd_merge_kernel(const FusedParams p
 }
 
 // D = rowsum(dO * O) per (token, head), stored negated in [B, H, S] order. Eight lanes share one head's 64 columns.
-__global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO, long long ldo,
+__global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* O, const __nv_bfloat16* dO, long long ldo,
                                                             long long lddo, float* __restrict__ dsum, long long T, int S, int H) {
   chain_next();
   chain_wait();
@@ -642,8 +642,8 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
   const long long row = rh / H;
   float dot = 0.f;
   if (row < T) {
-    const uint4 a = *reinterpret_cast<const uint4*>(O + row * ldo + head * F_HD + chunk * 8);
-    const uint4 g = *reinterpret_cast<const uint4*>(dO + row * lddo + head * F_HD + chunk * 8);
+    const uint4 a = __ldcg(reinterpret_cast<const uint4*>(O + row * ldo + head * F_HD + chunk * 8));
+    const uint4 g = __ldcg(reinterpret_cast<const uint4*>(dO + row * lddo + head * F_HD + chunk * 8));
     const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), a2 = unpack_bf16x2(a.z), a3 = unpack_bf16x2(a.w);
     const float2 g0 = unpack_bf16x2(g.x), g1 = unpack_bf16x2(g.y), g2 = unpack_bf16x2(g.z), g3 = unpack_bf16x2(g.w);
     dot = a0.x * g0.x + a0.y * g0.y + a1.x * g1.x + a1.y * g1.y + a2.x * g2.x + a2.y * g2.y + a3.x * g3.x + a3.y * g3.y;

@@ -296,7 +296,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         uint32_t vv[32];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          const uint4 t = __ldg(vp + c);
+          const uint4 t = __ldcg(vp + c);
           vv[4 * c] = t.x; vv[4 * c + 1] = t.y; vv[4 * c + 2] = t.z; vv[4 * c + 3] = t.w;
         }
         float n = p.xsa_eps, dot = 0.f;

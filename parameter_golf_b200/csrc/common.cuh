@@ -73,6 +73,9 @@ __device__ __forceinline__ bool elect_one() {
 // kernel before has completed and its writes are visible; no thread touches global memory before it, and every thread that does so
 // passes it. `chain_next` lets the kernel after this one start as soon as every CTA has come here. A kernel that allocates tensor
 // memory calls it after the allocation: a CTA of the next kernel, which waits for this one, must not take the columns first.
+// Such a kernel is resident while the ones before it still write, so nothing they may have written is constant over its lifetime:
+// its inputs are not `const __restrict__` and not read with `__ldg` (both permit the non-coherent path, which asks for exactly
+// that); activations come through `__ldcg`, TMA or plain loads. Only the rotary tables, written once at set-up, are read as constants.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

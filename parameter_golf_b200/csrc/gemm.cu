@@ -193,7 +193,7 @@ __device__ __forceinline__ void epilogue_chunk_staged(const GemmKernelParams& p,
     if ((reinterpret_cast<uintptr_t>(p.colscale + n0) & 15) == 0) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float4 t = __ldg(reinterpret_cast<const float4*>(p.colscale + n0) + i);
+        const float4 t = __ldcg(reinterpret_cast<const float4*>(p.colscale + n0) + i);
         cs[4 * i] = t.x; cs[4 * i + 1] = t.y; cs[4 * i + 2] = t.z; cs[4 * i + 3] = t.w;
       }
     } else {

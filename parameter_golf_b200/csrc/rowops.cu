@@ -24,6 +24,14 @@ __device__ __forceinline__ F8 ld8(const __nv_bfloat16* p) {
   r.v[0] = a.x; r.v[1] = a.y; r.v[2] = b.x; r.v[3] = b.y; r.v[4] = c.x; r.v[5] = c.y; r.v[6] = d.x; r.v[7] = d.y;
   return r;
 }
+// the same from memory that the kernel before may still be writing when this one starts (see chain_wait)
+__device__ __forceinline__ F8 ld8cg(const __nv_bfloat16* p) {
+  const uint4 q = __ldcg(reinterpret_cast<const uint4*>(p));
+  F8 r;
+  float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
+  r.v[0] = a.x; r.v[1] = a.y; r.v[2] = b.x; r.v[3] = b.y; r.v[4] = c.x; r.v[5] = c.y; r.v[6] = d.x; r.v[7] = d.y;
+  return r;
+}
 __device__ __forceinline__ void st8(__nv_bfloat16* p, const F8& r) {
   *reinterpret_cast<uint4*>(p) =
       make_uint4(pack_bf16x2(r.v[0], r.v[1]), pack_bf16x2(r.v[2], r.v[3]), pack_bf16x2(r.v[4], r.v[5]), pack_bf16x2(r.v[6], r.v[7]));
@@ -57,9 +65,8 @@ __device__ __forceinline__ void flush_cols(float (&acc)[NV][8], float* dst, int 
 // -------------------------------------------------------------------------------------------------------------
 // mix + RMSNorm forward:  xe = x (+ sw*skip);  x_in = bf16(mix0*xe + mix1*x0);  h = bf16(rmsnorm(x_in) * s)
 template <int NV>
-__global__ void __launch_bounds__(ROW_THREADS) mix_norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ x0,
-                                                                   const __nv_bfloat16* __restrict__ skip, const float* __restrict__ sw,
-                                                                   const float* __restrict__ mix, __nv_bfloat16* __restrict__ x_in,
+__global__ void __launch_bounds__(ROW_THREADS) mix_norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* x0, const __nv_bfloat16* skip,
+                                                                   const float* sw, const float* mix, __nv_bfloat16* __restrict__ x_in,
                                                                    __nv_bfloat16* __restrict__ h, int rows, int d, float s, float eps) {
   chain_next();
   chain_wait();
@@ -72,14 +79,14 @@ __global__ void __launch_bounds__(ROW_THREADS) mix_norm_fwd_kernel(const __nv_bf
     for (int j = 0; j < NV; ++j) {
       const int c = (j * 32 + lane) * 8;
       if (c < d) {
-        F8 a = ld8(x + base + c);
+        F8 a = ld8cg(x + base + c);
         if (skip) {
-          F8 k = ld8(skip + base + c), w = ld8f(sw + c);
+          F8 k = ld8cg(skip + base + c), w = ld8f(sw + c);
 #pragma unroll
           for (int e = 0; e < 8; ++e) a.v[e] = bfround(a.v[e] + w.v[e] * k.v[e]);
         }
         if (mix) {
-          F8 b = ld8(x0 + base + c), m0 = ld8f(mix + c), m1 = ld8f(mix + d + c);
+          F8 b = ld8cg(x0 + base + c), m0 = ld8f(mix + c), m1 = ld8f(mix + d + c);
 #pragma unroll
           for (int e = 0; e < 8; ++e) a.v[e] = bfround(m0.v[e] * a.v[e] + m1.v[e] * b.v[e]);
         }

@@ -31,7 +31,8 @@ __device__ __forceinline__ V8 ldf(const float* p) {
   return r;
 }
 __device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16(x)); }
-__device__ __forceinline__ uint4 ldraw(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
+// for memory that the kernel before may still be writing when this one starts (see chain_wait)
+__device__ __forceinline__ uint4 ldraw(const __nv_bfloat16* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ V8 cvt8(const uint4& q) {
   V8 r;
   float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
@@ -61,9 +62,8 @@ __device__ __forceinline__ void flush_cols2(float (&acc)[NV][8], float* dst, int
 
 template <int NV, bool MIX, bool SKIP>
 __global__ void __launch_bounds__(RT, (NV <= 2) ? 2 : 1)
-mix_norm_bwd2_kernel(const __nv_bfloat16* __restrict__ d_h, const __nv_bfloat16* __restrict__ d_res, const __nv_bfloat16* __restrict__ x_in,
-                     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ x0, const __nv_bfloat16* __restrict__ skip,
-                     const float* __restrict__ sw, const float* __restrict__ mix, const __nv_bfloat16* __restrict__ add_grad,
+mix_norm_bwd2_kernel(const __nv_bfloat16* d_h, const __nv_bfloat16* d_res, const __nv_bfloat16* x_in, const __nv_bfloat16* x,
+                     const __nv_bfloat16* x0, const __nv_bfloat16* skip, const float* sw, const float* mix, const __nv_bfloat16* add_grad,
                      __nv_bfloat16* __restrict__ d_x, __nv_bfloat16* __restrict__ d_x0, __nv_bfloat16* __restrict__ d_skip, float* __restrict__ d_mix,
                      float* __restrict__ d_sw, int skip_to_dx, int rows, int d, float s, float eps) {
   chain_next();
@@ -347,10 +347,10 @@ void qk_norm_rope_bwd64(const void* d_post, const void* pre, void* d_pre, const 
 // with the zeroing right after the loads, and 1398 us with eight lanes per row loading and zeroing their chunks in place, 64
 // contiguous bytes at a time; the two kernels it replaces took 238 us.
 constexpr int QKA_PITCH = 68;                              // floats per staged row: 64 + 4, so that rows start in different banks
-__global__ void __launch_bounds__(256) qk_norm_rope_bwd64_acc_kernel(float* __restrict__ dq_acc, const __nv_bfloat16* __restrict__ d_post,
-                                                                     const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __restrict__ d_pre,
+__global__ void __launch_bounds__(256) qk_norm_rope_bwd64_acc_kernel(float* __restrict__ dq_acc, const __nv_bfloat16* d_post,
+                                                                     const __nv_bfloat16* pre, __nv_bfloat16* __restrict__ d_pre,
                                                                      const float* __restrict__ cosT, const float* __restrict__ sinT,
-                                                                     const float* __restrict__ gain, float* __restrict__ d_gain, int ld, int H, int Hkv,
+                                                                     const float* gain, float* __restrict__ d_gain, int ld, int H, int Hkv,
                                                                      int rope_dims, int seq_len, float eps, float scale) {
   chain_next();
   chain_wait();
@@ -483,8 +483,7 @@ __global__ void __launch_bounds__(256) xsa_fwd64_kernel(const __nv_bfloat16* __r
 }
 
 // dy_h = dz_h - (<dz_h,v>/n) v ;  dv (+)= sum_h [ -c_h dz_h - (<dz_h,v>/n) y_h + 2 c_h (<dz_h,v>/n) v ],  c_h = <y_h,v>/n
-__global__ void __launch_bounds__(256) xsa_bwd64_kernel(const __nv_bfloat16* __restrict__ dz, const __nv_bfloat16* __restrict__ y,
-                                                        const __nv_bfloat16* __restrict__ v, __nv_bfloat16* __restrict__ dy,
+__global__ void __launch_bounds__(256) xsa_bwd64_kernel(const __nv_bfloat16* dz, const __nv_bfloat16* y, const __nv_bfloat16* v, __nv_bfloat16* __restrict__ dy,
                                                         __nv_bfloat16* __restrict__ dv, int accumulate_dv, int nvec, int Hkv, int group, int ld_y,
                                                         int ld_v, int ld_dv, float eps, float* __restrict__ dsum, int seq_len) {
   chain_next();
@@ -496,11 +495,11 @@ __global__ void __launch_bounds__(256) xsa_bwd64_kernel(const __nv_bfloat16* __r
     const bool live = i < nvec;
     const int ii = live ? i : nvec - 1;
     const int row = (int)((unsigned)ii / (unsigned)Hkv), kh = ii - row * Hkv;
-    const V8 vv = ldv(v + (size_t)row * ld_v + kh * 64 + sub * 8);
+    const V8 vv = cvt8(ldraw(v + (size_t)row * ld_v + kh * 64 + sub * 8));
     __nv_bfloat16* dvp = dv + (size_t)row * ld_dv + kh * 64 + sub * 8;
     V8 acc;
     if (accumulate_dv) {
-      acc = ldv(dvp);
+      acc = cvt8(ldraw(dvp));
     } else {
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc.v[e] = 0.f;
@@ -511,7 +510,7 @@ __global__ void __launch_bounds__(256) xsa_bwd64_kernel(const __nv_bfloat16* __r
     n = sum8(n) + eps;
     for (int g = 0; g < group; ++g) {
       const size_t off = (size_t)row * ld_y + (kh * group + g) * 64 + sub * 8;
-      const V8 a = ldv(y + off), b = ldv(dz + off);
+      const V8 a = cvt8(ldraw(y + off)), b = cvt8(ldraw(dz + off));
       float yv = 0.f, gv = 0.f;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
