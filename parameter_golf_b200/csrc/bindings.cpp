@@ -29,7 +29,7 @@ void gemm(torch::Tensor A, torch::Tensor B, torch::Tensor D, bool a_kmajor, bool
           double slope, c10::optional<torch::Tensor> aux, c10::optional<torch::Tensor> colscale, c10::optional<torch::Tensor> D2,
           int64_t splits, c10::optional<torch::Tensor> status, c10::optional<torch::Tensor> wait_flag, int64_t wait_value,
           int64_t seg_row0, c10::optional<torch::Tensor> seg_D0, int64_t seg_row1, c10::optional<torch::Tensor> seg_D1,
-          c10::optional<torch::Tensor> batch_sumsq, int64_t sumsq_pow, int64_t tile_n) {
+          c10::optional<torch::Tensor> batch_sumsq, int64_t sumsq_pow, int64_t tile_n, int64_t chain_rows) {
   check_bf16(A, "A");
   check_bf16(B, "B");
   TORCH_CHECK(A.dim() == B.dim() && A.dim() == D.dim() && (A.dim() == 2 || A.dim() == 3), "gemm: operands must all be 2-D or all 3-D");
@@ -102,6 +102,7 @@ void gemm(torch::Tensor A, torch::Tensor B, torch::Tensor D, bool a_kmajor, bool
   g.slope = (float)slope;
   g.splits = (int)splits;
   g.tile_n = (int)tile_n;
+  g.chain_rows = chain_rows;
   g.status = status_ptr(status);
   if (wait_flag.has_value()) {
     TORCH_CHECK(wait_flag->is_cuda() && wait_flag->scalar_type() == torch::kInt32, "wait_flag must be a CUDA int32 tensor");

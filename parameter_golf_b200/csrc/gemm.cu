@@ -661,7 +661,8 @@ static CUtensorMap operand_map(const void* ptr, bool kmajor, int rows, int K, lo
 }
 
 template <int BN, bool AK, bool BKM, int EPI>
-static void launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mx, const GemmKernelParams& p, int grid, cudaStream_t stream) {
+static void launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mx, const GemmKernelParams& p, int grid,
+                           long long chain_rows, cudaStream_t stream) {
   auto kern = gemm_tcgen05_kernel<BN, AK, BKM, EPI>;
   static bool configured[64] = {};          // the attribute is a per-device property of the kernel
   int dev = 0;
@@ -670,17 +671,17 @@ static void launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const C
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  launch_chained(std::max(p.M, p.K), kern, grid, gemm_threads(BN), GemmSmem<BN>::TOTAL, stream, ma, mb, mx, p);
+  launch_chained(chain_rows, kern, grid, gemm_threads(BN), GemmSmem<BN>::TOTAL, stream, ma, mb, mx, p);
 }
 
 template <int BN, int EPI>
 static void launch_major(const GemmArgs& a, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mx, const GemmKernelParams& p, int grid,
                          cudaStream_t stream) {
-  if (a.a_kmajor && a.b_kmajor) launch_variant<BN, true, true, EPI>(ma, mb, mx, p, grid, stream);
-  else if (a.a_kmajor && !a.b_kmajor) launch_variant<BN, true, false, EPI>(ma, mb, mx, p, grid, stream);
+  if (a.a_kmajor && a.b_kmajor) launch_variant<BN, true, true, EPI>(ma, mb, mx, p, grid, a.chain_rows, stream);
+  else if (a.a_kmajor && !a.b_kmajor) launch_variant<BN, true, false, EPI>(ma, mb, mx, p, grid, a.chain_rows, stream);
   else if constexpr (BN == 64) throw std::runtime_error("gemm: 64-column tiles take row-major activations");
-  else if (!a.a_kmajor && a.b_kmajor) launch_variant<BN, false, true, EPI>(ma, mb, mx, p, grid, stream);
-  else launch_variant<BN, false, false, EPI>(ma, mb, mx, p, grid, stream);
+  else if (!a.a_kmajor && a.b_kmajor) launch_variant<BN, false, true, EPI>(ma, mb, mx, p, grid, a.chain_rows, stream);
+  else launch_variant<BN, false, false, EPI>(ma, mb, mx, p, grid, a.chain_rows, stream);
 }
 
 template <int BN>
@@ -701,7 +702,7 @@ static void launch_epi(const GemmArgs& a, const CUtensorMap& ma, const CUtensorM
     case EPI_MUL_ACTGRAD: launch_major<BN, EPI_MUL_ACTGRAD>(a, ma, mb, mx, p, grid, stream); break;
     case EPI_QKV_NORM_ROPE:
       if (!(a.a_kmajor && a.b_kmajor)) throw std::runtime_error("gemm: the QKV epilogue takes row-major activations and [N][K] weights");
-      launch_variant<BN, true, true, EPI_QKV_NORM_ROPE>(ma, mb, mx, p, grid, stream);
+      launch_variant<BN, true, true, EPI_QKV_NORM_ROPE>(ma, mb, mx, p, grid, a.chain_rows, stream);
       break;
     default: throw std::runtime_error("gemm: unknown epilogue");
   }

@@ -1,7 +1,10 @@
 // Kernel launch with programmatic dependency on the kernel before it in the stream (`chain_wait` / `chain_next` in common.cuh). Only
 // for kernels in which every CTA calls chain_wait, and only up to CHAIN_ROWS token rows: where a launch gap is a visible share of a
 // kernel. With every launch chained a step of 4,096 tokens took 4349 us instead of 4783, but one of 98,304 tokens got 3 % slower (CTAs
-// of the next kernel settle on the SMs that finish first); at 16,384 it gains 2 %, at 24,576 nothing.
+// of the next kernel settle on the SMs that finish first); at 16,384 it gains 2 %, at 24,576 nothing. The rows are those of the whole
+// pass, which a product cannot see from its own sizes (a chunk of the output head has fewer, an optimizer product none): its
+// caller hands them over. 0 rows: not a link of a chain. The sharded optimizer's products pass 0: they run beside the next
+// forward, and a CTA that waits for its predecessor would hold shared and tensor memory that the forward could use.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -20,7 +23,7 @@ inline void launch_chained(long long rows, void (*kern)(P...), dim3 grid, dim3 b
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = rows <= CHAIN_ROWS ? 1 : 0;
+  cfg.numAttrs = rows > 0 && rows <= CHAIN_ROWS ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 

@@ -37,6 +37,7 @@ struct GemmArgs {
   int epi = EPI_BF16;
   int splits = 0;            // 0 = automatic
   int tile_n = 0;            // output tile columns (64, 128 or 256); 0 = automatic
+  long long chain_rows = 0;  // token rows of the pass this product is a link of (see launch.h); 0: it starts when its predecessor has finished
   float alpha = 1.f, beta = 0.f, slope = 0.f;
   int* status = nullptr;     // device status word (4 ints) or null
   const int* wait_flag = nullptr;   // optional readiness counter for B (see comm.cu); polled with a bounded wait

@@ -27,6 +27,7 @@ from __future__ import annotations
 
 import math
 import os
+from functools import partial
 from typing import Dict, List, Optional, Tuple
 
 import torch
@@ -77,6 +78,7 @@ class CudaEngine:
         self.dev = torch.device(device)
         self.B, self.S = micro_batch, seq_len
         self.T = micro_batch * seq_len
+        self.gemm = partial(N.gemm, chain_rows=self.T)       # every product of a pass over this engine's tokens
         self.train = train
         self.qat = False
         m = self.m
@@ -405,7 +407,7 @@ class CudaEngine:
         kernel, so two runs give the same bits (the fixed-order fp32 reduction the reference's parity mode relies on,
         ``parameter-golf-rs/crates/pg-bench/src/bin/parity_step.rs:9-14``)."""
         if not self.t.reproducible_backward:
-            N.gemm(dY, X, G, False, False, N.EPI_F32_ATOMIC, segs=segs)
+            self.gemm(dY, X, G, False, False, N.EPI_F32_ATOMIC, segs=segs)
             return
         T, M, Nn = dY.shape[0], dY.shape[1], X.shape[1]
         splits = 1
@@ -417,7 +419,7 @@ class CudaEngine:
         if getattr(self, "_dw_ws", None) is None or self._dw_ws.numel() < need:
             self._dw_ws = torch.empty(need, dtype=torch.float32, device=self.dev)
         ws = self._dw_ws[:need].view(splits, M, Nn)
-        N.gemm(dY.unflatten(0, (splits, T // splits)), X.unflatten(0, (splits, T // splits)), ws, False, False, N.EPI_F32)
+        self.gemm(dY.unflatten(0, (splits, T // splits)), X.unflatten(0, (splits, T // splits)), ws, False, False, N.EPI_F32)
         bounds = [(G, 0)] + [(t_, r_) for r_, t_ in segs if t_ is not None]
         for i, (dst, start) in enumerate(bounds):            # row range [start, end) of every partial goes to `dst`
             self.C.sum_splits_add(self._dw_ws, start * Nn, splits, M * Nn, dst)
@@ -469,8 +471,8 @@ class CudaEngine:
         d = self.d
         s = float(self.lora["alpha"]) / self._lora_rank
         qv = self.qkv_pre[li][:, :d]
-        N.gemm(self.h[li], self.lora_a_bf[l], self.lora_t[li])                                                   # t = h A^T      [T, r]
-        N.gemm(self.lora_t[li], self.lora_b_bf[l], qv, epi=N.EPI_AXPBY_BF16, alpha=s, beta=1.0, aux=qv)          # q += s t B^T
+        self.gemm(self.h[li], self.lora_a_bf[l], self.lora_t[li])                                                   # t = h A^T      [T, r]
+        self.gemm(self.lora_t[li], self.lora_b_bf[l], qv, epi=N.EPI_AXPBY_BF16, alpha=s, beta=1.0, aux=qv)          # q += s t B^T
 
     def _lora_bwd(self, l, aj):
         """Adapter gradients of layer l and the adapter's share of d_h (added in place). ``d_qkv_pre[:, :d]`` holds dL/dq_pre."""
@@ -479,11 +481,11 @@ class CudaEngine:
         dq = self.d_qkv_pre[:, :d]
         A = N.EPI_F32_ATOMIC
         if self.lora.get("trainable", False):
-            N.gemm(dq, self.lora_t[aj], self.g_lora_b[l], False, False, A, alpha=s)                             # dB += s dq^T t  [d, r]
-        N.gemm(dq, self.lora_b_bf[l], self.lora_dt, True, False, alpha=s)                                        # d_t = s dq B    [T, r]
+            self.gemm(dq, self.lora_t[aj], self.g_lora_b[l], False, False, A, alpha=s)                             # dB += s dq^T t  [d, r]
+        self.gemm(dq, self.lora_b_bf[l], self.lora_dt, True, False, alpha=s)                                        # d_t = s dq B    [T, r]
         if self.lora.get("trainable", False):
-            N.gemm(self.lora_dt, self.h[aj], self.g_lora_a[l], False, False, A)                                  # dA += d_t^T h   [r, d]
-        N.gemm(self.lora_dt, self.lora_a_bf[l], self.d_h, True, False, N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.d_h)   # d_h += d_t A
+            self.gemm(self.lora_dt, self.h[aj], self.g_lora_a[l], False, False, A)                                  # dA += d_t^T h   [r, d]
+        self.gemm(self.lora_dt, self.lora_a_bf[l], self.d_h, True, False, N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.d_h)   # d_h += d_t A
 
     # ---- attention -----------------------------------------------------------------------------------------------------
     def _attn_fwd(self, l, li):
@@ -542,11 +544,11 @@ class CudaEngine:
             N.gemm_qkv_norm_rope(self.h[li], Wqkv, self.qkv_pre[li], self.qk_post[li], self.cos, self.sin, gain, self.H, self.Hkv,
                                  m.rope_dims, S, self.eps, **wait)
         else:
-            N.gemm(self.h[li], Wqkv, self.qkv_pre[li], **wait)
+            self.gemm(self.h[li], Wqkv, self.qkv_pre[li], **wait)
         if m.value_embedding.enabled and l in m.value_embedding.layers:
             vi = m.value_embedding.layers.index(l)
             vview = self.qkv_pre[li][:, d + kv:]
-            N.gemm(self.ve_e, self.VP[vi], vview, epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=vview)
+            self.gemm(self.ve_e, self.VP[vi], vview, epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=vview)
         if self.lora is not None:
             self._lora_fwd(l, li)
         if not fused_qk:
@@ -558,13 +560,13 @@ class CudaEngine:
             C.head_gate_fwd(zz, self.h[li], p[wname][l], p[bname][l] if bname else None, out, self.gv[gi][li], self.H, self.hd, gscale_, gmult)
             zz = out
         self.zz[li] = zz
-        N.gemm(zz, Wo, self.x_mid[li], epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_in[li])
+        self.gemm(zz, Wo, self.x_mid[li], epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_in[li])
         if not self.parallel:
             C.mix_norm_fwd(self.x_mid[li], None, None, None, None, None, self.mm[li], s_l, self.eps)
-        N.gemm(self.mm[li], Wup, self.hu[li], epi=N.EPI_ACT_SQ, slope=self.slope, D2=self.a[li])
+        self.gemm(self.mm[li], Wup, self.hu[li], epi=N.EPI_ACT_SQ, slope=self.slope, D2=self.a[li])
         xo = self.x_out[j]
         if not recompute:
-            N.gemm(self.a[li], Wd, xo, epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_mid[li])
+            self.gemm(self.a[li], Wd, xo, epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_mid[li])
         return xo
 
     # ---- forward -------------------------------------------------------------------------------------------------------------
@@ -585,7 +587,7 @@ class CudaEngine:
         C.embed_gather(self.ids, self.E, self.e, 0, S, N.status_word(self.dev))
         if m.bigram.enabled:
             C.embed_gather(self.ids, self.BE, self.bg, m.bigram.vocab_size, S, N.status_word(self.dev))
-            N.gemm(self.bg, self.BP, self.xe, epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.e)
+            self.gemm(self.bg, self.BP, self.xe, epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.e)
         if m.value_embedding.enabled:
             C.embed_gather(self.ids, self.VE, self.ve_e, 0, S, N.status_word(self.dev))
         bid = m.smear_gate_boundary_token_id
@@ -616,7 +618,7 @@ class CudaEngine:
                 if self._logits_full is None:
                     self._logits_full = torch.empty(T, m.vocab_size, dtype=BF, device=self.dev)
                 logits = self._logits_full
-            N.gemm(self.hf, self.LM, logits)
+            self.gemm(self.hf, self.LM, logits)
             if targets is not None:
                 C.softcap_ce(logits, self.tgt, self.nll, logits if want_grad else None, self.loss_sum, m.logit_softcap, gscale,
                              self.tok_w if weighted else None, self.w_total if weighted else None)
@@ -627,11 +629,11 @@ class CudaEngine:
         for r0 in range(0, T, R):
             r1 = min(r0 + R, T)
             lg = self.logits[:r1 - r0]
-            N.gemm(self.hf[r0:r1], self.LM, lg)
+            self.gemm(self.hf[r0:r1], self.LM, lg)
             C.softcap_ce(lg, self.tgt[r0:r1], self.nll[r0:r1], lg if want_grad else None, self.loss_sum, m.logit_softcap, gscale,
                          self.tok_w[r0:r1] if weighted else None, self.w_total if weighted else None, T)
             if want_grad:
-                N.gemm(lg, self.LM, self.d_h[r0:r1], True, False)          # d_hf rows
+                self.gemm(lg, self.LM, self.d_h[r0:r1], True, False)          # d_hf rows
                 if self._wants("tok_emb" if m.tie_embeddings else "lm_head"):
                     self._dw(lg, self.hf[r0:r1], gW)
         self._head_grads_done = want_grad
@@ -658,7 +660,7 @@ class CudaEngine:
         A = N.EPI_F32_ATOMIC
         wants_ve = self._wants("ve_embed", "ve_proj", "ve_layer_scales", "ve_scale")
         if not self._head_grads_done:              # the chunked head has already produced d_hf and the output-embedding gradient
-            N.gemm(self.logits, self.LM, self.d_h, True, False)                              # d_hf
+            self.gemm(self.logits, self.LM, self.d_h, True, False)                              # d_hf
             if self._wants("tok_emb" if m.tie_embeddings else "lm_head"):
                 self._dw(self.logits, self.hf, g["tok_emb"] if m.tie_embeddings else g["lm_head"])
         C.mix_norm_bwd(self.d_h, None, self.x_last, None, None, None, None, None, None, self.dx, None, None, None, None, False, 1.0, self.eps)
@@ -676,10 +678,10 @@ class CudaEngine:
             # ---- MLP
             if self._wants("mlp_down_bank", "mlp_scale"):
                 self._dw_folded(self.dx, self.a[aj], self.Gd, C.fold_scaled_grad_bf16, *view["down"])
-            N.gemm(self.dx, Wd, self.d_hu, True, False, N.EPI_MUL_ACTGRAD, slope=self.slope, aux=self.hu[aj])
+            self.gemm(self.dx, Wd, self.d_hu, True, False, N.EPI_MUL_ACTGRAD, slope=self.slope, aux=self.hu[aj])
             if self._wants("mlp_up_bank"):
                 self._dw(self.d_hu, self.mm[aj], view["up"])
-            N.gemm(self.d_hu, Wup, self.d_m, True, False)
+            self.gemm(self.d_hu, Wup, self.d_m, True, False)
             if self.parallel:
                 dx_mid, dx_next = self.dx, self.dx_mid      # no norm between x_mid and the MLP: the residual gradient passes through
                 d_hx = self.d_m                             # and the MLP-input gradient joins the QKV-input gradient below
@@ -694,7 +696,7 @@ class CudaEngine:
             vview = self.v_cols[aj]
             xsa = l in xsa_layers
             d_att = self.d_z if xsa else self.d_y            # gradient of what the gates / the output projection consumed
-            N.gemm(dx_mid, Wo, d_att, True, False)
+            self.gemm(dx_mid, Wo, d_att, True, False)
             for gi in range(len(self.gates) - 1, -1, -1):
                 wname, bname, gscale_, gmult = self.gates[gi]
                 gate_in = self.yg[gi - 1][aj] if gi > 0 else (self.z[aj] if xsa else self.y[aj])
@@ -710,7 +712,7 @@ class CudaEngine:
             if m.value_embedding.enabled and l in m.value_embedding.layers and wants_ve:
                 vi = m.value_embedding.layers.index(l)
                 self.Gvp.zero_()
-                N.gemm(dv, self.ve_e, self.Gvp, False, False, A)                         # d(ve_eff * ve_proj)
+                self.gemm(dv, self.ve_e, self.Gvp, False, False, A)                         # d(ve_eff * ve_proj)
                 ds = (self.Gvp * p["ve_proj"]).sum()
                 g["ve_proj"].add_(self.Gvp * self.ve_eff[vi])
                 g["ve_layer_scales"][vi] += ds * p["ve_scale"][0]
@@ -718,15 +720,15 @@ class CudaEngine:
                 if not hasattr(self, "d_ve_e"):
                     self.d_ve_e = torch.empty_like(self.ve_e)
                     self.d_ve_acc = torch.zeros_like(self.ve_e, dtype=torch.float32)
-                N.gemm(dv, self.VP[vi], self.d_ve_e, True, False)
+                self.gemm(dv, self.VP[vi], self.d_ve_e, True, False)
                 self.d_ve_acc.add_(self.d_ve_e)
             # one weight-gradient product for the packed QKV rows, written to the Q, K and V slots of the gradient banks
             if self._wants("qo_bank", "kv_bank"):
                 self._dw(self.d_qkv_pre, self.h[aj], view["q"], segs=view["kv"])
             if d_hx is not None:
-                N.gemm(self.d_qkv_pre, Wqkv, self.d_h, True, False, N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=d_hx)
+                self.gemm(self.d_qkv_pre, Wqkv, self.d_h, True, False, N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=d_hx)
             else:
-                N.gemm(self.d_qkv_pre, Wqkv, self.d_h, True, False)
+                self.gemm(self.d_qkv_pre, Wqkv, self.d_h, True, False)
             if self.lora is not None:
                 self._lora_bwd(l, aj)
             # ---- block input: RMSNorm backward, residual mix, U-Net skip
@@ -764,7 +766,7 @@ class CudaEngine:
         if m.bigram.enabled:
             self._dw_folded(self.d_xe, self.bg, self.Gbp, C.fold_scaled_grad, p["bigram_proj"], p["bigram_scale"], 0, 1, g["bigram_proj"],
                             g["bigram_scale"], False)
-            N.gemm(self.d_xe, self.BP, self.d_bg, True, False)
+            self.gemm(self.d_xe, self.BP, self.d_bg, True, False)
             C.embed_scatter_add(self.ids, self.d_bg, g["bigram_embed"], m.bigram.vocab_size, S)
 
     # ---- public pieces -----------------------------------------------------------------------------------------------------------
@@ -827,29 +829,30 @@ class CudaEngine:
         for gi, grp in enumerate(self.groups):
             grp["ema"] = grp["p"].clone()
 
-    def newton_schulz(self, key: str, Bcount: Optional[int] = None) -> torch.Tensor:
+    def newton_schulz(self, key: str, Bcount: Optional[int] = None, chain_rows: int = 0) -> torch.Tensor:
         """Orthogonalise the momentum update ns[key]["U"] (bf16, NOT normalised; ns[key]["sq"] holds each matrix's sum of
         squares) and return the result buffer. The first iteration folds the normalisation X0 = U / (|U| + 1e-7) into its
         GEMM epilogues as a per-matrix factor (A = X0 X0^T = UU^T / |U|^2, X1 = a X0 + B X0 = (a U + B U) / |U|), so no
         pass over the shard is spent on dividing by the norm (the reference normalises in a kernel of its own,
-        ``pg-kernels/src/gpu_kernels.rs:4520``)."""
+        ``pg-kernels/src/gpu_kernels.rs:4520``). ``chain_rows``: see `native.gemm`."""
         st = self.ns[key]
         X, Xn, Am, Bm, Xalt, sq = st["U"], st["X1"], st["A"], st["Bm"], st["X0"], st["sq"]
         if Bcount is not None:
             X, Xn, Am, Bm, Xalt, sq = X[:Bcount], Xn[:Bcount], Am[:Bcount], Bm[:Bcount], Xalt[:Bcount], sq[:Bcount]
         tall = X.shape[1] > X.shape[2]
+        gemm = partial(N.gemm, chain_rows=chain_rows)
         for s in range(self.t.muon_ns_steps):
             a, b, c = ns_coeff(self.t.muon_ns_profile, s)
             first = s == 0
             if tall:
-                N.gemm(X, X, Am, False, False, batch_sumsq=sq if first else None, sumsq_pow=2)                 # A = X^T X
+                gemm(X, X, Am, False, False, batch_sumsq=sq if first else None, sumsq_pow=2)                 # A = X^T X
             else:
-                N.gemm(X, X, Am, True, True, batch_sumsq=sq if first else None, sumsq_pow=2)                   # A = X X^T
-            N.gemm(Am, Am, Bm, True, True, N.EPI_AXPBY_BF16, alpha=c, beta=b, aux=Am)    # B = b A + c A A   (A symmetric)
+                gemm(X, X, Am, True, True, batch_sumsq=sq if first else None, sumsq_pow=2)                   # A = X X^T
+            gemm(Am, Am, Bm, True, True, N.EPI_AXPBY_BF16, alpha=c, beta=b, aux=Am)    # B = b A + c A A   (A symmetric)
             if tall:
-                N.gemm(X, Bm, Xn, True, True, N.EPI_AXPBY_BF16, alpha=1.0, beta=a, aux=X, batch_sumsq=sq if first else None)    # X = a X + X B
+                gemm(X, Bm, Xn, True, True, N.EPI_AXPBY_BF16, alpha=1.0, beta=a, aux=X, batch_sumsq=sq if first else None)    # X = a X + X B
             else:
-                N.gemm(Bm, X, Xn, True, False, N.EPI_AXPBY_BF16, alpha=1.0, beta=a, aux=X, batch_sumsq=sq if first else None)   # X = a X + B X
+                gemm(Bm, X, Xn, True, False, N.EPI_AXPBY_BF16, alpha=1.0, beta=a, aux=X, batch_sumsq=sq if first else None)   # X = a X + B X
             X, Xn = Xn, (Xalt if first else X)           # U itself is never overwritten: later iterations ping-pong between X1 and X0
         return X
 
@@ -864,7 +867,7 @@ class CudaEngine:
             st = self.ns[k]
             st["sq"].zero_()
             C.muon_momentum(self.g[k], self.mom[k], st["U"], st["sq"], self.hp, True)
-            X = self.newton_schulz(k)
+            X = self.newton_schulz(k, chain_rows=self.T)
             scale = max(1.0, self.p[k].shape[-2] / self.p[k].shape[-1]) ** 0.5
             C.muon_apply(self.p[k].view(-1), X.view(-1), self.ema[k].view(-1) if self.ema else None, self.hp, t.matrix_lr, t.muon_wd, scale, decay)
         self.param_generation += 1

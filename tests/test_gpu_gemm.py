@@ -211,3 +211,42 @@ def test_every_tile_width_gives_the_same_product(tile_n, M, N, K):
     if tile_n == 64:
         with pytest.raises(RuntimeError, match="no tile of this width"):
             n.gemm(A, W, torch.empty(M, N, device="cuda"), epi=n.EPI_F32, tile_n=64)
+
+
+def _early_starts(fn):
+    """Kernels of ``fn`` that may start before the one ahead of them has finished: programmatic edges of its captured graph."""
+    from cuda.bindings import runtime as rt
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    err, _, _, edges, count = rt.cudaGraphGetEdges_v2(rt.cudaGraph_t(graph.raw_cuda_graph()), 4096)
+    assert err == rt.cudaError_t.cudaSuccess
+    return sum(e.type == rt.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic for e in edges[:count])
+
+
+def test_a_product_starts_early_only_as_a_link_of_a_small_pass():
+    """Whether a product may start before its predecessor has finished is decided by the rows of the pass its caller names (up to
+    16,384) and not by its own sizes: not without a pass, and not for a chunk or an optimizer product of a large one."""
+    n = _n()
+    A, W, D = _rand(512, 256), _rand(512, 256), torch.empty(512, 512, device="cuda", dtype=torch.bfloat16)
+
+    def pair(**kw):
+        n.gemm(A, W, D, **kw)
+        n.gemm(A, W, D, **kw)
+
+    assert [_early_starts(lambda: pair(chain_rows=r)) for r in (0, 512, 16384, 16385, 98304)] == [0, 1, 1, 0, 0]
+    assert _early_starts(pair) == 0
+
+
+@pytest.mark.parametrize("seqs,early", [(16, True), (256, False)])
+def test_optimizer_products_start_early_only_behind_a_small_pass(seqs, early):
+    from parameter_golf_b200.models import gpt
+    from parameter_golf_b200.models.engine import CudaEngine
+    from test_gpu_engine import small_spec
+    spec = small_spec()
+    e = CudaEngine(spec, gpt.fill_deterministic(spec.model), "cuda:0", seqs, 128, train=True)
+    e.set_hp(1.0, 0.95)
+    assert (_early_starts(e.optimizer_step) > 0) == early
+    assert _early_starts(lambda: e.newton_schulz("mlp_up_bank")) == 0          # as the sharded step runs it, beside the next forward
