@@ -709,7 +709,7 @@ static int bwd_sms() {
 }
 size_t attn_bwd_fused_part_floats() { return (size_t)bwd_sms() * 2 * 2 * 8192; }
 
-void attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse, float* dsum, float* dq_acc, void* dq,
+int attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse, float* dsum, float* dq_acc, void* dq,
                     void* dk, void* dv, long long ldq, long long ldk, long long ldv, long long ldo, long long lddo, long long lddq, long long lddk,
                     long long lddv, int B, int S, int H, int Hkv, int hd, int accumulate_dv, int* status, cudaStream_t st, int dsum_ready, float* part,
                     const QkNormRopeBwd* qk) {
@@ -765,6 +765,7 @@ void attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, 
   if (p.rest_w) launch_chained(T, attn_bwd_merge_kernel, dim3(grid - 1, 8), 256, 0, st, p, grid);
   if (qk) qk_norm_rope_bwd64_acc(dq_acc, *qk, (int)T, H, Hkv, S, p.scale, st);
   else launch_chained(T, attn_bwd_finish_kernel, B * H * p.n_qt, 256, 0, st, dq_acc, (__nv_bfloat16*)dq, lddq, S, H, p.n_qt, p.scale);
+  return (dsum_ready ? 2 : 3) + (p.rest_w ? 1 : 0);
 }
 
 }  // namespace pgb

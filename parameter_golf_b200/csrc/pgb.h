@@ -190,13 +190,13 @@ void attn_bwd(const void* q, const void* k, const void* v, const void* o, const 
 // (attn_bwd_fused_scratch_floats(B, S, H) floats, ZERO on entry, left zero on return), then scaled and cast into `dq`.
 // dsum is written by a small pre-kernel. dQ is reproducible to fp32 rounding only; attn_bwd is bit-reproducible.
 size_t attn_bwd_fused_scratch_floats(int B, int S, int H);
-void attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse, float* dsum, float* dq_acc, void* dq,
+int attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse, float* dsum, float* dq_acc, void* dq,
                     void* dk, void* dv, long long ldq, long long ldk, long long ldv, long long ldo, long long lddo, long long lddq, long long lddk,
                     long long lddv, int B, int S, int H, int Hkv, int hd, int accumulate_dv, int* status, cudaStream_t st, int dsum_ready = 0,
                     float* part = nullptr, const QkNormRopeBwd* qk = nullptr);
 // `part` (attn_bwd_fused_part_floats() floats, no initial value needed) lets the last, partly filled round of work be split evenly over
 // the SMs. With `qk` the accumulator goes through the backward of the per-head norm and rotation (qk_norm_rope_bwd64_acc) instead
-// of into `dq`, which may be null; qk->d_post + H * 64 must be `dk`.
+// of into `dq`, which may be null; qk->d_post + H * 64 must be `dk`. Returns the number of kernels launched.
 size_t attn_bwd_fused_part_floats();
 
 }  // namespace pgb

@@ -46,8 +46,7 @@ def load():
 class _Counting:
     """Forwards to the extension and counts kernel launches issued through it (`launch_count`)."""
 
-    _PER_CALL = {"attn_bwd": 2, "attn_bwd_fused": 4, "attn_bwd_qk": 4}
-    _DSUM_READY = {"attn_bwd_fused": 18, "attn_bwd_qk": 21}       # position of that argument
+    _PER_CALL = {"attn_bwd": 2, "attn_bwd_fused": None, "attn_bwd_qk": None}      # None: the call returns its number
 
     def __init__(self, mod):
         self._mod = mod
@@ -56,18 +55,18 @@ class _Counting:
 
     def __getattr__(self, name):
         fn = getattr(self._mod, name)
-        n, skip = self._PER_CALL.get(name, 1), self._DSUM_READY.get(name)
+        n = self._PER_CALL.get(name, 1)
 
         def call(*a, **k):
-            # the single-pass attention backward skips its first kernel when the caller supplies the per-query term
-            self.launches += n - 1 if (skip is not None and len(a) > skip and a[skip]) else n
-            if self.timing is None:
-                return fn(*a, **k)
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
+            timing = self.timing
+            if timing is not None:
+                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                e0.record()
             out = fn(*a, **k)
-            e1.record()
-            self.timing.append((_timing_key(name, a, k), e0, e1))
+            if timing is not None:
+                e1.record()
+                timing.append((_timing_key(name, a, k), e0, e1))
+            self.launches += out if n is None else n
             return out
 
         self.__dict__[name] = call

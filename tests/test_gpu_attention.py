@@ -193,3 +193,27 @@ def test_a_sequence_has_the_same_attention_alone_and_in_a_batch(B, S, H, Hkv):
         torch.cuda.synchronize()
         n.check_status()
         assert torch.equal(y1, y[r]) and torch.equal(z1, z[r]) and torch.equal(lse1[0], lse[b]), b
+
+
+@pytest.mark.parametrize("B,S,H,Hkv,merged", [(37, 128, 4, 4, False), (1, 512, 2, 1, True), (3, 1920, 8, 4, True)])
+def test_launch_count_of_the_backward_is_the_number_of_its_kernels(B, S, H, Hkv, merged):
+    """The single-pass backward launches its merge kernel only where a round of key tiles is split (148 items of one tile are a whole
+    round): the count follows what ran, with and without the first kernel."""
+    from torch.profiler import ProfilerActivity, profile
+    from parameter_golf_b200.ops import native as n
+    hd = 64
+    torch.manual_seed(S)
+    q, dy = (torch.randn(B * S, H * hd, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(B * S, Hkv * hd, device="cuda").bfloat16() for _ in range(2))
+    y, dq, dk, dv = torch.empty_like(q), torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    lse = n.attn_fwd(q, k, v, y, B, S, H, Hkv, hd)
+    dsum = n.attn_bwd(q, k, v, y, dy, lse, dq, dk, dv, B, S, H, Hkv, hd)
+    for ready in (False, True):
+        torch.cuda.synchronize()
+        before = n.launch_count()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            n.attn_bwd(q, k, v, y, dy, lse, dq, dk, dv, B, S, H, Hkv, hd, dsum=dsum, dsum_ready=ready)
+            torch.cuda.synchronize()
+        names = [e.name for e in prof.events() if "attn_bwd" in e.name]
+        assert n.launch_count() - before == len(names), names
+        assert any("merge" in x for x in names) == merged and any("prep" in x for x in names) != ready
