@@ -37,27 +37,53 @@ constexpr int GQ_GROUP_SMALL = 4, GQ_GROUP_LARGE = 8;      // rows that share on
 constexpr int GQ_BLOCK = 128;
 constexpr int GQ_TILE = GQ_BLOCK * GQ_BLOCK;
 
-// sign(x) floor(|x| + 1/2). Codes are clamped to 8 bits, so larger magnitudes may stop at 1024; below 2^23 adding and
-// subtracting 2^23 with the first addition rounded down is a floor (two additions where `floorf` is a slower conversion).
-__device__ __forceinline__ float round_half_away(float x) {
-  const float t = fminf(__fadd_rn(fabsf(x), 0.5f), 1024.f);
-  return copysignf(__fsub_rn(__fadd_rd(t, 8388608.f), 8388608.f), x);
+// The code of x: sign(x) floor(|x| + 1/2) within [qmin, qmax]. The limits are whole numbers, so clamping may come first; below 2^23
+// adding and subtracting 2^23 with the first addition rounded down is a floor (two additions where `floorf` is a slower
+// conversion). NaN stays NaN: `walk_block` recognises by it what `div_rn` does not cover.
+__device__ __forceinline__ float code_of(float x, float qmin, float qmax) {
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(qmin));
+  asm("min.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(qmax));
+  return copysignf(__fsub_rn(__fadd_rd(__fadd_rn(fabsf(x), 0.5f), 8388608.f), 8388608.f), x);
 }
 
-// a / b rounded to nearest, given r = 1 / b rounded to nearest: a first quotient, its exact remainder, one correction
-// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990, theorem on division
-// with a correctly rounded reciprocal). Holds away from overflow and underflow of the quotient and the remainder.
+// a / b rounded to nearest, given r = 1 / b rounded to nearest: a first quotient, its remainder, one correction (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990). The theorem asks for a first quotient within
+// one ulp, and a * r can be 1.5 ulp off; but only significand pairs whose quotient lies within 4.5 / 2^24 ulp of the middle between
+// two floats could then round wrongly, and all 52,333,588 pairs within 9 / 2^24 were checked: none does. NaN where the first
+// quotient is infinite or b outside [2^-60, 2^60] (`short_reciprocal`). A dividend below 2^-102, whose remainder is not exact,
+// may give a quotient (below 2^-42) that is an ulp off.
 __device__ __forceinline__ float div_rn(float a, float b, float r) {
   const float q = __fmul_rn(a, r);
   return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
 }
+__device__ __forceinline__ float short_reciprocal(float b) {
+  const float m = fabsf(b);
+  return m >= 0x1p-60f && m <= 0x1p60f ? __frcp_rn(b) : __int_as_float(0x7fffffff);
+}
+
+// One row's walk over a block with the general division: what `walk_block` falls back to. The row's values are updated in place.
+__device__ __noinline__ void walk_general(const float* tile, float* w_row, int8_t* q_row, float* e_row, int lane, int nb, float s, float qmin, float qmax) {
+  for (int j = 0; j < nb; ++j) {
+    const float* u_row = tile + j * GQ_BLOCK;
+    __syncwarp();
+    const float w = w_row[j], x = __fdiv_rn(w, s);
+    const float q = fminf(fmaxf(copysignf(floorf(fabsf(x) + 0.5f), x), qmin), qmax);      // NaN: qmin
+    const float err = __fdiv_rn(__fsub_rn(w, __fmul_rn(q, s)), u_row[j]);
+    if (lane == 0) {
+      q_row[j] = (int8_t)q;
+      e_row[j] = err;
+    }
+    for (int c = j + 1 + lane; c < nb; c += 32) w_row[c] = __fsub_rn(w_row[c], __fmul_rn(err, u_row[c]));
+  }
+}
 
 // One row's walk over a block of 128 columns (`WHOLE`) or the last nb < 128 columns: without the end test of the ragged form
-// the shared-memory reads of later columns move ahead of the dependency chain.
+// the shared-memory reads of later columns move ahead of the dependency chain. A quotient that `div_rn` does not cover leaves NaN
+// in its column's error and so in every later column's: the block is then walked again.
 template <bool WHOLE>
-__device__ __forceinline__ void walk_block(const float* __restrict__ tile, const float* __restrict__ sR, const float* w_row, int8_t* q_row, float* e_row,
+__device__ __forceinline__ void walk_block(const float* __restrict__ tile, const float* __restrict__ sR, float* w_row, int8_t* q_row, float* e_row,
                                            int lane, int nb, float s, float rs, float qmin, float qmax) {
-  float reg[4];
+  float reg[4], err = 0.f;
 #pragma unroll
   for (int ii = 0; ii < 4; ++ii) {
     const int c = ii * 32 + lane;
@@ -72,8 +98,8 @@ __device__ __forceinline__ void walk_block(const float* __restrict__ tile, const
       if (!WHOLE && j >= nb) break;                                        // uniform across the warp
       const float* u_row = tile + j * GQ_BLOCK;
       const float w = __shfl_sync(0xffffffffu, reg[ii], jj);
-      const float q = fminf(fmaxf(round_half_away(div_rn(w, s, rs)), qmin), qmax);
-      const float err = div_rn(__fsub_rn(w, __fmul_rn(q, s)), u_row[j], sR[j]);
+      const float q = code_of(div_rn(w, s, rs), qmin, qmax);
+      err = div_rn(__fsub_rn(w, __fmul_rn(q, s)), u_row[j], sR[j]);
       if (lane == jj) {
         my_q = q;
         my_e = err;
@@ -92,6 +118,7 @@ __device__ __forceinline__ void walk_block(const float* __restrict__ tile, const
       e_row[c] = my_e;
     }
   }
+  if (err != err) walk_general(tile, w_row, q_row, e_row, lane, nb, s, qmin, qmax);
 }
 
 template <int BYTES>
@@ -101,8 +128,10 @@ __device__ __forceinline__ void gq_copy(float* smem_dst, const float* gmem_src, 
 }
 
 // `rows` counts (candidate, row) pairs, candidate-major; R of them per CTA (one warp each), then 12 warps for the far updates.
+// The small form's one CTA per SM may use 128 registers a thread; told only its threads, the compiler kept to 64 and spilled on the
+// chain (512 x 1536: 0.26 ms instead of 0.19).
 template <int GROUP, int MAX_THREADS, bool TWO_TILES>
-__global__ void __launch_bounds__(MAX_THREADS)
+__global__ void __launch_bounds__(MAX_THREADS, TWO_TILES ? 1 : 0)
 gptq_rows_kernel(const float* __restrict__ Wp, const float* __restrict__ U, const float* __restrict__ scales, int8_t* __restrict__ Q, int rows,
                  int weight_rows, int cols, int R, float qmin, float qmax) {
   extern __shared__ __align__(16) float sm[];
@@ -139,7 +168,7 @@ gptq_rows_kernel(const float* __restrict__ Wp, const float* __restrict__ U, cons
   };
   auto reciprocals = [&](int i1) {
     const float* tile = sU + (TWO_TILES ? ((i1 / GQ_BLOCK) & 1) * GQ_TILE : 0);
-    if (threadIdx.x < min(GQ_BLOCK, cols - i1)) sR[threadIdx.x] = __frcp_rn(tile[threadIdx.x * (GQ_BLOCK + 1)]);
+    if (threadIdx.x < min(GQ_BLOCK, cols - i1)) sR[threadIdx.x] = short_reciprocal(tile[threadIdx.x * (GQ_BLOCK + 1)]);
   };
   load_tile(0, threadIdx.x, threads);
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -147,7 +176,7 @@ gptq_rows_kernel(const float* __restrict__ Wp, const float* __restrict__ U, cons
   reciprocals(0);
   __syncthreads();
   const float s = warp < live ? scales[row0 + warp] : 1.f;
-  const float rs = __frcp_rn(s);
+  const float rs = short_reciprocal(s);
   for (int i1 = 0; i1 < cols; i1 += GQ_BLOCK) {
     const int nb = min(GQ_BLOCK, cols - i1);
     const int buf = (i1 / GQ_BLOCK) & 1;
@@ -155,7 +184,7 @@ gptq_rows_kernel(const float* __restrict__ Wp, const float* __restrict__ U, cons
       if (warp < live) {
         const float* tile = sU + (TWO_TILES ? buf * GQ_TILE : 0);
         float* e_row = sE + (buf * R + warp) * GQ_BLOCK;
-        const float* w_row = sW + warp * cols + i1;
+        float* w_row = sW + warp * cols + i1;
         int8_t* q_row = Q + (size_t)(row0 + warp) * cols + i1;
         if (nb == GQ_BLOCK) walk_block<true>(tile, sR, w_row, q_row, e_row, lane, nb, s, rs, qmin, qmax);
         else walk_block<false>(tile, sR, w_row, q_row, e_row, lane, nb, s, rs, qmin, qmax);

@@ -95,3 +95,37 @@ def test_gptq_rows_of_several_candidates_are_those_of_one_at_a_time(rows, cols):
     for k in range(5):
         want = torch.cat([n.gptq_rows(Wp[i:i + 500], U, scales[k, i:i + 500], 6) for i in range(0, rows, 500)])
         assert torch.equal(got[k], want), k
+
+
+def test_gptq_rows_outside_the_range_of_the_short_division():
+    """Infinite, overflowing, tiny and undefined quotients give the codes of the general division: the limits, zero, and the lowest code
+    for NaN, in both divisions of a column (the second through a diagonal far from one)."""
+    from parameter_golf_b200.ops import native as n
+    inf, nan = float("inf"), float("nan")
+    w = torch.tensor([inf, -inf, 3e38, -3e38, nan, 0.0, -0.0, 1e-45, 2.5, -2.5, 2.4999998], device="cuda")
+    s = torch.tensor([1.0, 1.0, 6e-8, 6e-8, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0], device="cuda")
+    for copies in (1, 80):                                                   # the small form and the large one
+        got = n.gptq_rows(w.repeat(copies)[:, None], torch.ones(1, 1, device="cuda"), s.repeat(copies), 6)
+        assert got[:, 0].reshape(copies, -1).eq(torch.tensor([31, -32, 31, -32, -32, 0, 0, 0, 3, -3, 2], dtype=torch.int8, device="cuda")).all()
+    # column 2 receives -err * u with err = 0.25 / diagonal: exact powers of two, so the code is known
+    for e in (-100, -70, -60, -59, 0, 59, 60, 61, 100):
+        U = torch.tensor([[2.0 ** e, 2.0 ** (e + 6)], [0.0, 1.0]], device="cuda")
+        got = n.gptq_rows(torch.tensor([[1.25, 0.0]], device="cuda"), U, torch.ones(1, device="cuda"), 6)
+        assert got.tolist() == [[1, -16]], e
+
+
+@pytest.mark.parametrize("bits", [5, 6, 8])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 127), (2000, 128), (500, 37)])
+def test_gptq_codes_of_one_block_are_those_of_the_float32_statement(rows, cols, bits):
+    """Without a trailing update there is no sum whose order could differ: every code equals the reference's, with weights on and
+    next to the ties of the rounding (half-precision scales, as the export has them)."""
+    from parameter_golf_b200.ops import native as n
+    from parameter_golf_b200.quant.gptq import gptq_prepare, gptq_rows_torch
+    W, H = _problem(rows, cols, rows + cols + bits)
+    perm, _, U = gptq_prepare(H)
+    Wp = W[:, perm].contiguous()
+    scale = (Wp.abs().amax(1) / ((1 << (bits - 1)) - 1)).clamp_min(6e-8).half().float().clamp_min(6e-8)
+    Wp[:, 0] = (torch.randint(-12, 12, (rows,), device="cuda") + 0.5) * scale          # a tie, and its two neighbours
+    Wp[:, 0] = torch.where(torch.arange(rows, device="cuda") % 3 == 1, torch.nextafter(Wp[:, 0], torch.zeros_like(scale)), Wp[:, 0])
+    Wp[:, 0] = torch.where(torch.arange(rows, device="cuda") % 3 == 2, torch.nextafter(Wp[:, 0], 9 * Wp[:, 0]), Wp[:, 0])
+    assert torch.equal(n.gptq_rows(Wp, U, scale, bits), gptq_rows_torch(Wp, U, scale, bits))
