@@ -98,7 +98,11 @@ def gptq_quantize(W: torch.Tensor, H: torch.Tensor, bits: int = 6, block: int = 
     if native_rows is not None and rows * len(scales) > 4 * torch.cuda.get_device_properties(W.device).multi_processor_count:
         S = torch.stack(scales)
         Q = native_rows(Wp, U, S, bits, block)
-        err = (Wp - Q.float() * S[:, :, None]).pow(2).sum(2)
+        err = torch.empty_like(S)
+        step = max(1, (1 << 23) // (len(scales) * cols))      # the fp32 temporaries of the error pass stay at 100 MB
+        for r0 in range(0, rows, step):
+            r = slice(r0, r0 + step)
+            err[:, r] = (Wp[r] - Q[:, r].float() * S[:, r, None]).pow(2).sum(2)
         err = torch.where(err < float("inf"), err, best_err)
         best_err = err.amin(0)
         order = torch.arange(len(scales), device=W.device)[:, None]

@@ -129,3 +129,25 @@ def test_gptq_codes_of_one_block_are_those_of_the_float32_statement(rows, cols, 
     Wp[:, 0] = torch.where(torch.arange(rows, device="cuda") % 3 == 1, torch.nextafter(Wp[:, 0], torch.zeros_like(scale)), Wp[:, 0])
     Wp[:, 0] = torch.where(torch.arange(rows, device="cuda") % 3 == 2, torch.nextafter(Wp[:, 0], 9 * Wp[:, 0]), Wp[:, 0])
     assert torch.equal(n.gptq_rows(Wp, U, scale, bits), gptq_rows_torch(Wp, U, scale, bits))
+
+
+@pytest.mark.parametrize("rows,cols", [(130, 200), (16000, 1100)])
+def test_gptq_of_all_candidates_at_once_needs_no_more_memory_than_one_at_a_time(rows, cols):
+    """The route with one launch (and its error pass, which takes a large matrix in pieces) picks the codes and scales of the route with
+    a launch per candidate, and a large matrix does not need more memory by it."""
+    from parameter_golf_b200.ops import native as n
+    from parameter_golf_b200.quant.gptq import gptq_quantize
+    W, H = _problem(rows, cols, rows + cols)
+    out, peak = [], []
+    for rows_fn in (n.gptq_rows, None):                       # a row function of the caller's: one candidate at a time
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        out.append(gptq_quantize(W, H, 6, rows_fn=rows_fn))
+        torch.cuda.synchronize()
+        peak.append(torch.cuda.max_memory_allocated() - before)
+    (q0, s0), (q1, s1) = out
+    same = s0 == s1                                           # two candidates' fp32 error sums can tie up to their order of summation
+    assert same.float().mean() >= 0.999 and torch.equal(q0[same], q1[same])
+    if rows > 1000:
+        assert peak[1] <= peak[0], peak
