@@ -691,3 +691,78 @@ def test_a_window_scores_the_same_alone_and_in_a_batch(S):
     whole = r.nll(ids, tgt)
     for lo, hi in ((0, 1), (11, 12), (4, 7)):
         assert torch.equal(r.nll(ids[lo:hi], tgt[lo:hi]), whole[lo:hi]), (lo, hi)
+
+
+@pytest.mark.parametrize("variant,names", [("ve", ["ve_proj"]), ("ve", ["ve_embed", "tok_emb"]), ("ve", ["ve_layer_scales", "kv_bank"]), ("ve_recurrence", ["ve_scale"]),
+                                           ("ve_lora", []), ("untied", ["lm_head"]), ("untied", ["tok_emb", "bigram_scale"]),
+                                           ("chunked", ["tok_emb"]), ("chunked", ["skip_weights", "qo_bank"]), ("chunked_untied", ["mlp_down_bank"]),
+                                           ("recurrence", ["resid_mix", "mlp_up_bank"])])
+def test_gradients_of_some_parameters_are_those_of_all_in_every_family(variant, names):
+    """The products left out by `loss_and_grads(names=...)` with value embeddings, recurrent blocks, an untied and a row-chunked
+    head, and for an adapter alone: the gradients of the full call (relative 2-norm 1e-4, the order of fp32 adds), before and after."""
+    from parameter_golf_b200.eval.ttt import init_q_lora
+    from parameter_golf_b200.models import gpt
+    from parameter_golf_b200.models.engine import EngineRunner
+    from parameter_golf_b200.ops import native
+    ov = {}
+    if "ve" in variant:
+        ov.update({"model.value_embedding.enabled": "true", "model.value_embedding.dim": 64, "model.value_embedding.layers": "[2,3]"})
+    if "recurrence" in variant:
+        ov.update({"model.recurrence.enabled": "true", "model.recurrence.start_layer": 1, "model.recurrence.repeat_layers": 2})
+    if "untied" in variant:
+        ov["model.tie_embeddings"] = "false"
+    if "chunked" in variant:
+        ov["train.logit_chunk_rows"] = 128
+    spec = small_spec(**ov)
+    params = gpt.fill_deterministic(spec.model)
+    assert set(names) <= set(params)
+    torch.manual_seed(7)
+    ids, tgt = torch.randint(0, 256, (4, 128)), torch.randint(0, 256, (4, 128))
+    eng = EngineRunner(spec, params, "cuda", batch=4)
+    if "lora" in variant:
+        eng.lora = init_q_lora(spec.model, 16, 32.0, "cuda")
+        eng.lora["b"].normal_(0.0, 0.02)
+        eng.lora["trainable"] = True
+        names = names + ["lora.a", "lora.b"]
+    full = {k: v.clone() for k, v in eng.loss_and_grads(ids, tgt)[1].items()}
+    some = {k: v.clone() for k, v in eng.loss_and_grads(ids, tgt, names=[k for k in names if k in params])[1].items()}
+    again = eng.loss_and_grads(ids, tgt)[1]
+    native.check_status()
+    assert sorted(some) == sorted(names) and all(float(full[k].norm()) > 0 for k in names)
+    for k in names:
+        assert float((some[k] - full[k]).norm()) <= 1e-4 * float(full[k].norm()), k
+    for k in full:
+        assert float((again[k] - full[k]).norm()) <= 1e-4 * float(full[k].norm()) + 1e-12, k
+
+
+@pytest.mark.parametrize("which", ["fold_scaled_grad_bf16", "fold_scaled_grad"])
+def test_a_backward_that_raised_leaves_no_product_behind(which):
+    """The staging buffers of the scaled weights' gradients are zero between uses because the fold kernel leaves them so. A call that
+    raises between the product and the fold must not add its product to the next call's gradients."""
+    from parameter_golf_b200.models import gpt
+    from parameter_golf_b200.models.engine import EngineRunner
+    spec = small_spec()
+    params = gpt.fill_deterministic(spec.model)
+    torch.manual_seed(9)
+    ids, tgt = torch.randint(0, 256, (4, 128)), torch.randint(0, 256, (4, 128))
+    eng = EngineRunner(spec, params, "cuda", batch=4)
+    full = {k: v.clone() for k, v in eng.loss_and_grads(ids, tgt)[1].items()}
+    engine = next(iter(eng.engines.values()))
+    ext = engine.C
+
+    class Raising:
+        def __getattr__(self, name):
+            if name == which:
+                def fold(*a):
+                    raise KeyboardInterrupt
+                return fold
+            return getattr(ext, name)
+
+    engine.C = Raising()
+    with pytest.raises(KeyboardInterrupt):
+        eng.loss_and_grads(ids, tgt)
+    engine.C = ext
+    assert float(sum(t.abs().sum() for t in (engine.Gd, engine.Go, engine.Gbp))) > 0           # the product is there
+    again = eng.loss_and_grads(ids, tgt)[1]
+    for k in full:
+        assert float((again[k] - full[k]).norm()) <= 1e-4 * float(full[k].norm()) + 1e-12, k
