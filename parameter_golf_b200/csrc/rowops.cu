@@ -863,12 +863,13 @@ void softcap_logits(const void* z, float* out, long long n, float cap, cudaStrea
   softcap_logits_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)z, out, n, cap, 1.f / cap);
 }
 
-static int row_grid(int rows) {
+static int sm_count() {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return std::max(1, std::min((rows + ROW_WARPS - 1) / ROW_WARPS, sms * 8));
+  return sms;
 }
+static int row_grid(int rows) { return std::max(1, std::min((rows + ROW_WARPS - 1) / ROW_WARPS, sm_count() * 8)); }
 
 #define PGB_NV_DISPATCH(d, CALL)                                        \
   do {                                                                  \
@@ -1011,12 +1012,25 @@ void embed_scatter_add(const int* ids, const void* g, float* dtable, int rows, i
     return;
   }
   const int cslices = (d + slice - 1) / slice;
-  // One CTA per SM (the tile fills its shared memory), so the chunks make one round, or two where a chunk stays long (98,304 rows, 512
-  // columns: 276 us in two rounds, 310 in one). A chunk is at least 256 rows, below which zeroing and flushing the tile is the larger
-  // part: 4,096 rows take less than 20 us in chunks of 455 and took 50 us in chunks of 2,048.
-  const int ychunks = std::max(1, std::min((rows >= 16384 ? 2 : 1) * 148 / cslices, (rows + 255) / 256));
-  const int rows_per = (rows + ychunks - 1) / ychunks;
   const size_t smem = (size_t)table_rows * slice * 4;
+  // A CTA's time is that of its rows plus zeroing and flushing its tile, which costs as much as ~400 rows, so one round of CTAs beats
+  // two unless it leaves many SMs idle: 32 column slices fill 128 of 148 SMs in one round, 288 of 296 places in two. us in one
+  // round / in two: 512 columns, table of 1,024, 16,384 rows 62 / 72, 32,768 107 / 115, 98,304 283 / 289; 128 columns, hashed table of
+  // 3,072, 32,768 rows 47 / 59; 1,024 columns, table of 1,024, 8,192 rows 66 / 70, 32,768 213 / 197. Up to four CTAs share an SM
+  // when the tile is small (256 columns, table of 256, 32,768 rows: 53 with one, 35 with four). A chunk is at least 256 rows:
+  // 4,096 rows of 512 columns take 27 us in chunks of 455 and took 66 us in chunks of 2,048.
+  const int slots = sm_count() * std::max(1, (int)std::min<size_t>(4, 227 * 1024 / (smem + 1024)));
+  int ychunks = 1;
+  double best = 0.0;
+  for (int rounds : {1, 2}) {
+    const int n = std::max(1, std::min(rounds * slots / cslices, (rows + 255) / 256));
+    const double cost = (400.0 + (double)rows / n) * ((n * cslices + slots - 1) / slots);
+    if (rounds == 1 || cost < best) {
+      ychunks = n;
+      best = cost;
+    }
+  }
+  const int rows_per = (rows + ychunks - 1) / ychunks;
   dim3 grid(cslices, ychunks);
   auto launch = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -231,3 +231,19 @@ def test_softcap_logits(shape):
     assert got.shape == z.shape and got.dtype == torch.float32
     assert bool(got[0, 2].isnan()) and int(got.isnan().sum()) == 1
     assert float((got.double() - want).nan_to_num(0.0).abs().max()) <= 30.0 * 4 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("rows,d,table,buckets", [(1, 64, 256, 0), (257, 512, 1024, 0), (16512, 512, 1024, 0), (24576, 128, 3072, 3072), (8200, 1024, 1024, 0),
+                                                  (20480, 1024, 1024, 0), (40001, 256, 256, 0), (3000, 520, 1600, 0)])
+def test_embedding_gradient_at_every_split_of_its_rows(rows, d, table, buckets):
+    """Chunks of one round and of two, several CTAs per SM, a ragged last chunk and a ragged column slice: every row is added once.
+    Integer gradients, so fp32 sums are exact in any order."""
+    from parameter_golf_b200.ops import reference as R
+    torch.manual_seed(rows)
+    ids = torch.randint(0, buckets or table, (rows,), device="cuda", dtype=torch.int32)
+    g = torch.randint(-8, 9, (rows, d), device="cuda").to(BF)
+    at = R.bigram_hash(ids.reshape(1, rows).long(), buckets).reshape(rows) if buckets else ids.long()
+    got = torch.zeros(table, d, device="cuda")
+    C().embed_scatter_add(ids, g, got, buckets, rows)
+    torch.cuda.synchronize()
+    assert torch.equal(got, torch.zeros(table, d, device="cuda").index_add_(0, at, g.float()))
