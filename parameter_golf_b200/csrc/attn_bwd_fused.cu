@@ -24,8 +24,8 @@
 // would keep a few SMs busy for a whole item; their units (plus one per key tile for loading K/V and storing dK/dV) are cut into
 // equal contiguous ranges, one per CTA, at most two of whose key tiles are shared with a neighbour. A shared tile's dK/dV go to a
 // per-CTA fp32 slot and attn_bwd_merge_kernel adds the slots in CTA order, so dK and dV stay independent of timing.
-// Longest CTA in units (H = 8, Hkv = 4, S = 2048, 148 SMs), whole items against this split: B = 1 36 / 9, B = 2 36 / 17,
-// B = 8 72 / 64, B = 48 396 / 375.
+// Longest CTA in units and key-tile loads (H = 8, Hkv = 4, S = 2048, 148 SMs), whole items against this split: B = 1 36 / 8,
+// B = 2 36 / 16, B = 8 72 / 63, B = 48 396 / 374. `split_plan` has the rule.
 //
 // The per-query terms ride on the tensor core. P^T = exp2(c S^T - lse[q]) and dS^T = P^T (dP^T - D[q]) need one lse and one
 // D per query COLUMN of the transposed tiles, i.e. every thread would need every value: broadcast loads from shared memory
@@ -709,6 +709,38 @@ static int bwd_sms() {
 }
 size_t attn_bwd_fused_part_floats() { return (size_t)bwd_sms() * 2 * 2 * 8192; }
 
+// How the items of a call are laid out over `grid` CTAs: `whole` rounds of whole items, then (rest_w > 0) the last, partly filled round
+// split evenly by weight. It is split where that shortens the longest CTA by at least SPLIT_MIN units: the slots, the merge kernel
+// and its launch cost about that much. us split / whole at H = 8, Hkv = 4 through the rotation backward: 3 units saved (17 x 1024)
+// 140 / 130, 5 (16 x 1024) 135 / 127, 8 (24 x 1024) 185 / 181, (40 x 384) 106 / 108, 9 (8 x 2048) 179 / 181, (5 x 896) 57 / 58,
+// 13 (3 x 1920) 84 / 93, 20 (2 x 2048) 69 / 91, 28 (1 x 2048) 51 / 83. One sequence of 128: 31 / 22.
+constexpr int SPLIT_MIN = 9;
+struct SplitPlan {
+  int n_pairs, n_super, w_pair, w_bk, whole, rest_base, rest_w;
+};
+static SplitPlan split_plan(int B, int S, int H, int Hkv, int grid, bool may_split) {
+  SplitPlan s;
+  const int n_qt = S / 128, group = H / Hkv;
+  s.n_pairs = (n_qt + 1) / 2;
+  s.n_super = B * Hkv * s.n_pairs;
+  s.w_pair = (n_qt + 1) * group + 2;
+  s.w_bk = s.w_pair * (s.n_pairs - 1) + (n_qt % 2 ? s.n_pairs * group + 1 : s.w_pair);
+  s.whole = (s.n_super + grid - 1) / grid;
+  s.rest_base = s.rest_w = 0;
+  const int full = s.n_super / grid * grid, longest = n_qt == 1 ? s.w_bk : s.w_pair;
+  const long long end = (long long)B * Hkv * s.w_bk, base = (long long)(full / s.n_pairs) * s.w_bk + (long long)(full % s.n_pairs) * s.w_pair;
+  if (may_split && full < s.n_super && end < 0x7fffffffll && longest - (end - base + grid - 1) / grid >= SPLIT_MIN) {
+    s.whole = full / grid;
+    s.rest_base = (int)base;
+    s.rest_w = (int)(end - base);
+  }
+  return s;
+}
+size_t attn_bwd_fused_part_floats(int B, int S, int H, int Hkv) {
+  if (B <= 0 || S < 128 || Hkv <= 0 || H < Hkv) return 0;
+  return split_plan(B, S, H, Hkv, bwd_sms(), true).rest_w ? attn_bwd_fused_part_floats() : 0;
+}
+
 int attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse, float* dsum, float* dq_acc, void* dq,
                     void* dk, void* dv, long long ldq, long long ldk, long long ldv, long long ldo, long long lddo, long long lddq, long long lddk,
                     long long lddv, int B, int S, int H, int Hkv, int hd, int accumulate_dv, int* status, cudaStream_t st, int dsum_ready, float* part,
@@ -722,8 +754,13 @@ int attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, c
   p.B = B; p.S = S; p.H = H; p.Hkv = Hkv;
   p.n_qt = S / 128;
   p.group = H / Hkv;
-  p.n_pairs = (p.n_qt + 1) / 2;
-  p.n_super = B * Hkv * p.n_pairs;
+  const int sms = bwd_sms();
+  const int grid = part ? sms : std::max(1, std::min(B * Hkv * ((p.n_qt + 1) / 2), sms));
+  const SplitPlan plan = split_plan(B, S, H, Hkv, grid, part != nullptr);
+  p.n_pairs = plan.n_pairs; p.n_super = plan.n_super;
+  p.w_pair = plan.w_pair; p.w_bk = plan.w_bk;
+  p.whole = plan.whole; p.rest_base = plan.rest_base; p.rest_w = plan.rest_w;
+  p.part = part;
   p.scale = 1.f / sqrtf((float)hd);
   p.scale_log2 = p.scale * F_LOG2E;
   p.lse = lse; p.Dsum = dsum; p.dq_acc = dq_acc;
@@ -731,24 +768,6 @@ int attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, c
   p.lddk = lddk; p.lddv = lddv;
   p.accumulate_dv = accumulate_dv;
   p.status = status;
-  const int sms = bwd_sms();
-  const int grid = part ? sms : std::min(p.n_super, sms);
-  p.part = part;
-  p.w_pair = (p.n_qt + 1) * p.group + 2;
-  p.w_bk = p.w_pair * (p.n_pairs - 1) + (p.n_qt % 2 ? p.n_pairs * p.group + 1 : p.w_pair);
-  p.whole = (p.n_super + grid - 1) / grid;
-  p.rest_base = p.rest_w = 0;
-  if (part) {
-    // Split the last, partly filled round when that shortens the longest CTA by more than two units (what the shared tiles' slots and
-    // the merge cost; a round that is nearly full is left as it is).
-    const int full = p.n_super / grid * grid;
-    const long long end = (long long)B * Hkv * p.w_bk, base = (long long)(full / p.n_pairs) * p.w_bk + (long long)(full % p.n_pairs) * p.w_pair;
-    if (full < p.n_super && end < 0x7fffffffll && (end - base) / grid + 2 < p.w_pair) {
-      p.whole = full / grid;
-      p.rest_base = (int)base;
-      p.rest_w = (int)(end - base);
-    }
-  }
   int dev = 0;
   cudaGetDevice(&dev);
   static bool configured[64] = {};          // the attribute is a per-device property of the kernel

@@ -198,5 +198,6 @@ int attn_bwd_fused(const void* q, const void* k, const void* v, const void* o, c
 // the SMs. With `qk` the accumulator goes through the backward of the per-head norm and rotation (qk_norm_rope_bwd64_acc) instead
 // of into `dq`, which may be null; qk->d_post + H * 64 must be `dk`. Returns the number of kernels launched.
 size_t attn_bwd_fused_part_floats();
+size_t attn_bwd_fused_part_floats(int B, int S, int H, int Hkv);       // the same, or 0 where a call of this shape splits nothing
 
 }  // namespace pgb

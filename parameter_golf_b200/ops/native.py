@@ -214,13 +214,15 @@ def attn_bwd(q, k, v, o, d_o, lse, dq, dk, dv, B, S, H, Hkv, hd, accumulate_dv=F
     if dq_acc is None:
         dq_acc = attn_dq_scratch(q.device, B, S, H, hd)
     load().attn_bwd_fused(q, k, v, o, d_o, lse, dsum, dq_acc, dq, dk, dv, B, S, H, Hkv, hd, accumulate_dv, status_word(q.device), dsum_ready,
-                          attn_bwd_part(q.device))
+                          attn_bwd_part(q.device, (B, S, H, Hkv)))
     return dsum
 
 
-def attn_bwd_part(device):
-    """Slots for the key tiles that two CTAs of the single-pass attention backward share (no initial value needed)."""
-    return torch.empty(load()._mod.attn_bwd_part_floats(), dtype=torch.float32, device=device)
+def attn_bwd_part(device, shape=None):
+    """Slots for the key tiles that two CTAs of the single-pass attention backward share (no initial value needed). ``shape`` =
+    (B, S, H, Hkv) of the call: None where it shares none."""
+    need = load()._mod.attn_bwd_part_floats(*(shape or ()))
+    return torch.empty(need, dtype=torch.float32, device=device) if need else None
 
 
 def softcap_logits(z, cap):
