@@ -464,7 +464,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (elect_one()) {
+    // The wide QKV product is bound by its output stage, and there the fast issue of an elected thread costs 5 % (98,304 rows: 146 us
+    // against 138 with the branch on the lane number, 24,576 rows: 50 against 48).
+    if ((EPI == EPI_QKV_NORM_ROPE && BN == 256) ? lane == 0 : elect_one()) {
       constexpr uint32_t IDESC = make_idesc_bf16(BM, BN, A_KMAJOR ? 0 : 1, B_KMAJOR ? 0 : 1);
       // operand descriptors of stage 0; a stage or K step only adds to their address field
       const uint64_t da0 = A_KMAJOR ? make_smem_desc(smem_u32(smem), 16, 1024) : make_smem_desc(smem_u32(smem), 8192, 1024);
