@@ -54,9 +54,10 @@ constexpr int F_TILE = 128 * F_HD * 2;       // 16 KB: one 128-row bf16 tile of 
 constexpr float F_LOG2E = 1.4426950408889634f;
 constexpr uint32_t F_BACKOFF_NS = 96;         // sleep between barrier polls of the single-thread roles
 constexpr int F_STAGES = 3;                  // {Q, dO, lse, D} stages
-// Two softmax warpgroups of 64 query columns each is the measured optimum at B=48, S=2048 (0.934 ms): four groups of 32
+// Two softmax warpgroups of 64 query columns each, chosen at B=48, S=2048 when that form took 0.934 ms: four groups of 32
 // columns (640 threads, 104 registers) took 1.009 ms, and two groups plus a fourth warpgroup that only drains dQ partials
-// (512 threads, softmax at 200 registers) 1.033 ms.
+// (512 threads, softmax at 200 registers) 1.033 ms. With elected issuing threads and the split last round it takes 0.834 ms; the
+// other two were not measured again since.
 #ifndef PGB_ATTN_BWD_GROUPS
 #define PGB_ATTN_BWD_GROUPS 2
 #endif

@@ -7,16 +7,14 @@
 //   * One warp per row walks a 128-column block (4 values per lane in registers, the current one broadcast with a shuffle,
 //     the rank-1 feedback reads U from a shared 128x128 tile). The two divisions of a column sit on the chain: each is a
 //     multiplication by a reciprocal and two fused corrections (`div_rn`) instead of the general routine.
-//   * The block's 128 errors must reach every column right of it. The next block needs them at once (`near`: all 16 warps,
-//     one column of one row per thread); the columns beyond are updated by the other 12 warps while the 4 row warps already
-//     walk the next block (`far`), so that phase and the fetch of the next diagonal tile are off the chain. An element of U is
-//     loaded once per CTA and used for all four rows.
-// Four rows per CTA spread 512 rows over 128 SMs. The form with eight rows per CTA, in which every warp also did the far
-// updates of its row by itself, took 2.42 ms at 512 x 1536 (6-bit); four rows with near and far update in one phase between two
-// blocks 0.53 ms; this one 0.35 ms.
-// The chain leaves most issue slots free, so when there are more than four rows per SM (five clip candidates of one matrix) a
-// larger CTA walks up to 20 rows at once, five per scheduler (`gptq_rows`); it holds one diagonal tile instead of two, which is
-// fetched during the near update. Five candidates of 512 x 1536: 1.74 ms as five launches, 0.88 ms as one.
+//   * The block's 128 errors must reach every column right of it. The next block needs them at once (`near`: all warps of the CTA,
+//     each thread a column of a row at a time); the columns beyond are updated by the 12 warps that own no row while the row warps
+//     already walk the next block (`far`), off the chain. An element of U is loaded once per group of rows (four or eight).
+// Small form: four rows and 16 warps per CTA, two diagonal tiles, of which the far warps fetch the next; 512 rows spread over 128 SMs.
+// Large form: up to 20 rows, five per scheduler, and 32 warps; one diagonal tile, fetched during the near update. It is for more rows
+// than four per SM, such as five clip candidates of one matrix, and is bound by issue slots as much as by the chain.
+// 512 x 1536, 6-bit: one candidate 0.20 ms, five in one launch 0.85 ms. Before: eight rows per CTA, every warp doing the far updates of
+// its row by itself, 2.42 ms for one; four rows with near and far update in one phase between two blocks 0.53 ms.
 // The arithmetic inside a block is written with explicitly rounded operations (no fused multiply-add) so that the
 // codes match the float32 reference except where the two summation orders of the trailing update differ.
 //
@@ -280,8 +278,10 @@ void gptq_rows(const float* Wp, const float* U, const float* scales, int8_t* Q, 
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // A CTA fills an SM in both forms and takes about as long for 20 rows as for 4 (the chain along the columns), so the count of rounds
-  // decides: four rows per CTA while those fit in one round, else as many as shared memory allows, evened out over the rounds.
+  // A CTA's time grows more slowly than its rows (one round of 1,536 columns: 4 rows 0.20 ms, 8 0.34, 12 0.52, 16 0.63, 20 0.82), so
+  // the fewest rounds win: four rows per CTA while those fit in one round, else as many as shared memory allows, evened out over the
+  // rounds. ms this way / in rounds of the small form: 1,184 rows 0.34 / 0.38, 1,776 0.53 / 0.57, 2,368 0.64 / 0.75, 2,960 0.84 / 0.93,
+  // 5,920 1.67 / 1.85. (Four rows in the large form, two CTAs per SM, measured 0.31, 0.53, 0.60, 0.80 and 1.47; not used.)
   int R = GQ_ROWS;
   if ((total + GQ_ROWS - 1) / GQ_ROWS > sms) {
     int most = GQ_MAX_ROWS;
