@@ -841,7 +841,7 @@ __global__ void __launch_bounds__(256) embed_scatter_atomic_kernel(const int* __
 }
 
 // out = cap * tanh(z / cap) in fp32 from the bf16 products of the head. Bound by DRAM (2 bytes in, 4 out per logit): 4,480 rows of 8192
-// logits take 38 us (220 MB, 5.8 TB/s); as four element-wise passes through fp32 buffers they took 285 us.
+// logits take 38 to 44 us (220 MB, 5.0 to 5.8 TB/s); as four element-wise passes through fp32 buffers they took 285 us.
 __global__ void __launch_bounds__(256) softcap_logits_kernel(const __nv_bfloat16* __restrict__ z, float* __restrict__ out, long long n, float cap,
                                                              float inv_cap) {
   const long long stride = (long long)gridDim.x * blockDim.x * 8;
