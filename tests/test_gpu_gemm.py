@@ -215,15 +215,18 @@ def test_every_tile_width_gives_the_same_product(tile_n, M, N, K):
 
 def _early_starts(fn):
     """Kernels of ``fn`` that may start before the one ahead of them has finished: programmatic edges of its captured graph."""
-    from cuda.bindings import runtime as rt
+    import ctypes
     fn()
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph):
         fn()
-    err, _, _, edges, count = rt.cudaGraphGetEdges_v2(rt.cudaGraph_t(graph.raw_cuda_graph()), 4096)
-    assert err == rt.cudaError_t.cudaSuccess
-    return sum(e.type == rt.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic for e in edges[:count])
+    # through ctypes: the list that cuda.bindings returns points into memory it has freed, whose first entries are overwritten at times
+    n, edges = 4096, (ctypes.c_uint8 * (8 * 4096))()                     # cudaGraphEdgeData: from_port, to_port, type, 5 reserved bytes
+    count, src, dst = ctypes.c_size_t(n), (ctypes.c_void_p * n)(), (ctypes.c_void_p * n)()
+    rt = ctypes.CDLL("libcudart.so.12")
+    assert rt.cudaGraphGetEdges_v2(ctypes.c_void_p(graph.raw_cuda_graph()), src, dst, edges, ctypes.byref(count)) == 0
+    return sum(edges[8 * i + 2] == 1 for i in range(count.value))        # cudaGraphDependencyTypeProgrammatic
 
 
 def test_a_product_starts_early_only_as_a_link_of_a_small_pass():
