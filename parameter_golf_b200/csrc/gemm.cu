@@ -17,6 +17,8 @@
 // accumulators (2 x BN TMEM columns) let the epilogue of tile i overlap the main loop of tile i+1.
 // Tile 128 x BN x 64, BN in {64, 128, 256} (`pick_tile`); grid = min(#tiles, #SMs); tile index = n fastest so CTAs
 // working at the same time share the rows of the large operand in L2. The 64-column form has four epilogue warps (6 warps in all).
+#include <cmath>
+
 #include "common.cuh"
 #include "launch.h"
 #include "pgb.h"
@@ -53,6 +55,7 @@ struct GemmKernelParams {
   const float* head_gain;
   int q_heads, qk_heads, rope_half, seq_len;
   float norm_eps;
+  uint32_t* signs;            // EPI_ACT_SQ_SIGN, EPI_MUL_ACTROOT
 };
 
 constexpr int STG_PITCH = 64;
@@ -60,7 +63,8 @@ constexpr int STG_WARP_BYTES = 32 * STG_PITCH;      // one 32-row x 32-column bf
 
 // Epilogue staging: two chunk-sized slots per epilogue warp. A slot first receives a chunk of the epilogue's second
 // operand (cp.async, two chunks ahead of its use), is read, then stages the output chunk in place.
-template <int BN>
+constexpr int SGN_BYTES = 32 * 4;                   // the sign words of one chunk
+template <int BN, int EPI>
 struct GemmSmem {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
@@ -68,10 +72,24 @@ struct GemmSmem {
   static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128) ? 6 : 8;
   static constexpr int TILE_BYTES = STAGES * STAGE_BYTES;
   static constexpr int STG_BYTES = epi_warps(BN) * 2 * STG_WARP_BYTES;
-  static constexpr int TOTAL = TILE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + STG_BYTES;
+  static constexpr int SGN_TOTAL = EPI == EPI_MUL_ACTROOT ? epi_warps(BN) * 2 * SGN_BYTES : 0;
+  // the declaration aligns the memory to 1024 bytes; the slack stays where there is room for it
+  static constexpr int TOTAL = TILE_BYTES + (SGN_TOTAL ? 0 : 1024) + 256 /*barriers*/ + STG_BYTES + SGN_TOTAL;
+  static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
 };
 
 __device__ __forceinline__ float act_fn(float x, float slope) { return x >= 0.f ? x : slope * x; }
+
+// epilogues that read a second [M][N] bf16 operand
+constexpr bool epi_has_aux(int epi) { return epi == EPI_AXPBY_BF16 || epi == EPI_RESID_BF16 || epi == EPI_MUL_ACTGRAD || epi == EPI_MUL_ACTROOT; }
+
+// Relative error below 2^-22; its results are rounded to bf16. Without the handling of denormal arguments (roots below 1e-19), which
+// costs the activation gradient of 98,304 x 1536 20 us.
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
 template <int EPI>
 __device__ __forceinline__ void epilogue_chunk(const GemmKernelParams& p, float alpha, float beta, int b, int m, int n0, const uint32_t (&r)[32]) {
@@ -174,8 +192,8 @@ __device__ __forceinline__ int stg_off(int row, int piece) { return row * STG_PI
 
 template <int EPI>
 __device__ __forceinline__ void epilogue_chunk_staged(const GemmKernelParams& p, float alpha, float beta, int b, int m_base, int lane, int n0, const uint32_t (&r)[32],
-                                                      const uint8_t* auxs, uint8_t* stg) {
-  constexpr bool HAS_AUX = (EPI == EPI_AXPBY_BF16 || EPI == EPI_RESID_BF16 || EPI == EPI_MUL_ACTGRAD);
+                                                      const uint8_t* auxs, uint8_t* stg, uint32_t sg) {
+  constexpr bool HAS_AUX = epi_has_aux(EPI);
   const int srow = lane >> 2, spc = lane & 3;
   float a[32];
   if constexpr (HAS_AUX) {
@@ -201,6 +219,17 @@ __device__ __forceinline__ void epilogue_chunk_staged(const GemmKernelParams& p,
       for (int i = 0; i < 32; ++i) cs[i] = p.colscale[n0 + i];
     }
   }
+  if constexpr (EPI == EPI_MUL_ACTROOT) {
+    // aux = bf16(t^2) with t = leaky_relu(h): the root, rounded to bf16, is |t| itself (t has 8 significant bits, and its square was
+    // off by at most half a unit of 8 bits, which moves the root by less than half a unit; `test_activation_root` goes through all t).
+    const float pos = 2.f, neg = -2.f * p.slope;
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+      const float2 t = unpack_bf16x2(pack_bf16x2(sqrt_approx(a[i]), sqrt_approx(a[i + 1])));
+      o[i] = __uint_as_float(r[i]) * (t.x * ((sg >> i) & 1u ? neg : pos));
+      o[i + 1] = __uint_as_float(r[i + 1]) * (t.y * ((sg >> (i + 1)) & 1u ? neg : pos));
+    }
+  }
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     const float v = __uint_as_float(r[i]);
@@ -214,6 +243,23 @@ __device__ __forceinline__ void epilogue_chunk_staged(const GemmKernelParams& p,
   }
   uint32_t pk[16], pk2[16];
   bool packed = false;
+  if constexpr (EPI == EPI_ACT_SQ_SIGN) {
+    packed = true;
+    const __nv_bfloat162 sl = __float2bfloat162_rn(p.slope);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const __nv_bfloat162 hb = __floats2bfloat162_rn(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+      const __nv_bfloat162 t = __hmax2(hb, __hmul2(hb, sl));
+      const __nv_bfloat162 sq = __hmul2(t, t);
+      pk[i] = *reinterpret_cast<const uint32_t*>(&sq);
+    }
+    if (p.signs != nullptr) {
+      uint32_t w = 0;
+#pragma unroll
+      for (int i = 31; i >= 0; --i) w = __funnelshift_l(r[i], w, 1);       // rounding to bf16 keeps the sign
+      if (m_base + lane < p.M) p.signs[(size_t)(n0 >> 5) * p.M + m_base + lane] = w;
+    }
+  }
   if constexpr (EPI == EPI_ACT_SQ) {
     // With a slope that is zero or a power of two, slope*h is exact in bf16 and the square of a bf16 value rounds
     // once either way, so the whole activation can run on packed bf16 pairs with bit-identical results.
@@ -344,10 +390,10 @@ template <int BN, bool A_KMAJOR, bool B_KMAJOR, int EPI>
 __global__ void __launch_bounds__(gemm_threads(BN), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_x, const GemmKernelParams p) {
-  using S = GemmSmem<BN>;
+  using S = GemmSmem<BN, EPI>;
   constexpr int STAGES = S::STAGES;
   constexpr uint32_t TMEM_COLS = 2 * BN;            // 128, 256 or 512: two accumulators
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::TILE_BYTES);
   uint64_t* empty_bar = full_bar + STAGES;
@@ -504,13 +550,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int quarter = warp & 3;                 // TMEM lane quarter this warp may access
     const int half = (warp - 2) >> 2;             // which half of the tile's columns
     uint8_t* slots = smem + S::TILE_BYTES + 256 + (warp - 2) * 2 * STG_WARP_BYTES;
+    uint8_t* sgn = smem + S::TILE_BYTES + 256 + S::STG_BYTES + (warp - 2) * 2 * SGN_BYTES;      // sign words beside each slot
     const bool staged_ok = (p.ldd % 8 == 0) && (p.stride_d % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.D) & 15) == 0) &&
                            (p.aux == nullptr || ((p.ld_aux % 8 == 0) && (p.stride_aux % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.aux) & 15) == 0))) &&
                            (p.D2 == nullptr || ((reinterpret_cast<uintptr_t>(p.D2) & 15) == 0));
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    constexpr bool HAS_AUX = (EPI == EPI_AXPBY_BF16 || EPI == EPI_RESID_BF16 || EPI == EPI_MUL_ACTGRAD);
+    constexpr bool HAS_AUX = epi_has_aux(EPI);
     constexpr int CH = BN / 8 / epi_warps(BN);    // 32-column chunks per epilogue warp (the warps of a quarter split the columns)
     constexpr bool BF16_OUT = !(EPI == EPI_F32 || EPI == EPI_F32_ATOMIC);
     const int c_begin = half * CH;
@@ -529,7 +576,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // shared-memory and tensor-memory traffic of those chunks, which then wait for DRAM as well. The slot is read by the
     // thread that owns the row, reused in place to stage the output chunk, and refilled once the stores have read it.
     const bool aux_async = HAS_AUX && staged_ok;
-    auto issue_aux = [&](int b, int tm, int tn, int cc, uint8_t* slot) {
+    auto issue_aux = [&](int b, int tm, int tn, int cc) {
+      uint8_t* slot = slots + (cc & 1) * STG_WARP_BYTES;
       if constexpr (HAS_AUX) {
         const int n0 = tn * BN + (c_begin + cc) * 32;
         if (n0 + 32 <= p.N) {
@@ -540,6 +588,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const int row = m_base + i * 8 + (lane >> 2);
             if (row < p.M) cp_async16(slot + stg_off(i * 8 + (lane >> 2), lane & 3), ap + (long long)row * p.ld_aux);
           }
+          if constexpr (EPI == EPI_MUL_ACTROOT) {
+            if (p.signs != nullptr && m_base + lane < p.M)
+              cp_async4(sgn + (cc & 1) * SGN_BYTES + lane * 4, p.signs + (size_t)(n0 >> 5) * p.M + m_base + lane);
+          }
         }
         cp_async_commit();          // one group per chunk, also when nothing was copied: the wait below counts groups
       }
@@ -548,8 +600,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (aux_async && blockIdx.x < total_tiles) {
       int b0, tm0, tn0;
       tile_coords(blockIdx.x, b0, tm0, tn0);
-      issue_aux(b0, tm0, tn0, 0, slots);
-      issue_aux(b0, tm0, tn0, 1, slots + STG_WARP_BYTES);
+      issue_aux(b0, tm0, tn0, 0);
+      issue_aux(b0, tm0, tn0, 1);
     }
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       int b, tm, tn;
@@ -602,7 +654,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           }
           PGB_TMEM_WAIT_LD32(rr);
           if constexpr (BF16_OUT) {
-            if (staged_ok && n0 + 32 <= p.N && (aux_async || !HAS_AUX)) epilogue_chunk_staged<EPI>(p, alpha, beta, b, m_base, lane, n0, rr, slot, slot);
+            uint32_t sg = 0;
+            if constexpr (EPI == EPI_MUL_ACTROOT) {
+              if (p.signs != nullptr) sg = *reinterpret_cast<const uint32_t*>(sgn + (cc & 1) * SGN_BYTES + lane * 4);
+            }
+            if constexpr (EPI == EPI_ACT_SQ_SIGN || EPI == EPI_MUL_ACTROOT)          // the host refuses what is not aligned
+              epilogue_chunk_staged<EPI>(p, alpha, beta, b, m_base, lane, n0, rr, slot, slot, sg);
+            else if (staged_ok && n0 + 32 <= p.N && (aux_async || !HAS_AUX)) epilogue_chunk_staged<EPI>(p, alpha, beta, b, m_base, lane, n0, rr, slot, slot, sg);
             else if (m < p.M) epilogue_chunk<EPI>(p, alpha, beta, b, m, n0, rr);
           } else {
             if (m < p.M) epilogue_chunk<EPI>(p, alpha, beta, b, m, n0, rr);
@@ -611,8 +669,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if constexpr (HAS_AUX) {
           if (aux_async) {
             __syncwarp();                         // every lane is done with this slot
-            if (cc + 2 < CH) issue_aux(b, tm, tn, cc + 2, slot);
-            else if (next < total_tiles) issue_aux(nb, ntm, ntn, cc + 2 - CH, slot);
+            if (cc + 2 < CH) issue_aux(b, tm, tn, cc + 2);
+            else if (next < total_tiles) issue_aux(nb, ntm, ntn, cc + 2 - CH);
             else cp_async_commit();
           }
         }
@@ -670,10 +728,10 @@ static void launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const C
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN, EPI>::TOTAL);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  launch_chained(chain_rows, kern, grid, gemm_threads(BN), GemmSmem<BN>::TOTAL, stream, ma, mb, mx, p);
+  launch_chained(chain_rows, kern, grid, gemm_threads(BN), GemmSmem<BN, EPI>::TOTAL, stream, ma, mb, mx, p);
 }
 
 template <int BN, int EPI>
@@ -705,6 +763,14 @@ static void launch_epi(const GemmArgs& a, const CUtensorMap& ma, const CUtensorM
     case EPI_QKV_NORM_ROPE:
       if (!(a.a_kmajor && a.b_kmajor)) throw std::runtime_error("gemm: the QKV epilogue takes row-major activations and [N][K] weights");
       launch_variant<BN, true, true, EPI_QKV_NORM_ROPE>(ma, mb, mx, p, grid, a.chain_rows, stream);
+      break;
+    case EPI_ACT_SQ_SIGN:
+      if (!(a.a_kmajor && a.b_kmajor)) throw std::runtime_error("gemm: the activation with signs takes row-major activations and [N][K] weights");
+      launch_variant<BN, true, true, EPI_ACT_SQ_SIGN>(ma, mb, mx, p, grid, a.chain_rows, stream);
+      break;
+    case EPI_MUL_ACTROOT:
+      if (!(a.a_kmajor && !a.b_kmajor)) throw std::runtime_error("gemm: the activation gradient from the root takes row-major gradients and [K][N] weights");
+      launch_variant<BN, true, false, EPI_MUL_ACTROOT>(ma, mb, mx, p, grid, a.chain_rows, stream);
       break;
     default: throw std::runtime_error("gemm: unknown epilogue");
   }
@@ -789,6 +855,14 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   p.rope_half = a.rope_dims / 2;
   p.seq_len = a.seq_len;
   p.norm_eps = a.norm_eps;
+  p.signs = a.signs;
+  if (a.epi == EPI_ACT_SQ_SIGN || a.epi == EPI_MUL_ACTROOT) {
+    int e = 0;
+    const bool slope_ok = a.slope == 0.f || (a.slope > 0.f && a.slope < 1.f && std::frexp(a.slope, &e) == 0.5f);
+    if (a.batch != 1 || a.N % 32 || (a.ldd % 8) || (reinterpret_cast<uintptr_t>(a.D) & 15) || !slope_ok ||
+        (a.epi == EPI_MUL_ACTROOT && (a.aux == nullptr || (a.ld_aux % 8) || (reinterpret_cast<uintptr_t>(a.aux) & 15) || (a.slope > 0.f && !a.signs))))
+      throw std::runtime_error("gemm: the activation with signs needs 16-byte aligned rows, N a multiple of 32 and a slope of 0 or a power of two below 1");
+  }
   if (a.epi == EPI_QKV_NORM_ROPE) {
     const bool rope_ok = a.rope_dims == 0 || ((a.rope_dims == 16 || a.rope_dims == 32 || a.rope_dims == 64) && a.rope_cos && a.rope_sin &&
                                               (reinterpret_cast<uintptr_t>(a.rope_cos) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.rope_sin) & 15) == 0);
@@ -801,7 +875,7 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   const int total = p.tiles_m * p.tiles_n * p.splits * a.batch;
   const int grid = std::min(total, num_sms());
   // L2 prefetch of the epilogue's second operand ([batch][M][N] bf16, row pitch ld_aux) one tile ahead of its readers
-  const bool has_aux = a.aux != nullptr && (a.epi == EPI_AXPBY_BF16 || a.epi == EPI_MUL_ACTGRAD);
+  const bool has_aux = a.aux != nullptr && (a.epi == EPI_AXPBY_BF16 || a.epi == EPI_MUL_ACTGRAD || a.epi == EPI_MUL_ACTROOT);
   p.aux_l2_prefetch = (has_aux && a.ld_aux % 8 == 0 && (a.batch == 1 || a.stride_aux % 8 == 0) &&
                        (reinterpret_cast<uintptr_t>(a.aux) & 15) == 0 && total > grid) ? 1 : 0;
   const CUtensorMap mx = p.aux_l2_prefetch ? operand_map(a.aux, true, a.M, a.N, a.ld_aux, a.stride_aux, a.batch, BM) : ma;

@@ -20,6 +20,8 @@ enum GemmEpilogue : int {
   EPI_MUL_ACTGRAD = 6,  // D = bf16(acc * d/dh leaky_relu(h, slope)^2), h = aux
   EPI_QKV_NORM_ROPE = 7,  // D = bf16(acc) and, for the query and key heads (64 columns each), D2 = gain_h * rope(rms_norm(D)):
                           // the QKV projection with per-head RMSNorm, partial RoPE and the query gain in its output stage
+  EPI_ACT_SQ_SIGN = 8,  // D = bf16(leaky_relu(h, slope)^2) of h = bf16(acc), and (optional) the sign bits of h in `signs`
+  EPI_MUL_ACTROOT = 9,  // EPI_MUL_ACTGRAD with h taken back from the activation: aux = what EPI_ACT_SQ_SIGN wrote, and its `signs`
 };
 
 struct GemmArgs {
@@ -55,6 +57,9 @@ struct GemmArgs {
   const float* head_gain = nullptr;
   int q_heads = 0, kv_heads = 0, rope_dims = 0, seq_len = 0;
   float norm_eps = 0.f;
+  // EPI_ACT_SQ_SIGN / EPI_MUL_ACTROOT: [N / 32][M] words, bit i of word (c, m) = sign of h[m][32 c + i]. May be null where nobody
+  // reads them (a forward without a backward) or, with slope 0, where they make no difference. The slope is 0 or a power of two below 1.
+  uint32_t* signs = nullptr;
 };
 
 void gemm_bf16(const GemmArgs& args, cudaStream_t stream);

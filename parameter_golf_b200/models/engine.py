@@ -10,8 +10,9 @@ one execution path per op and the element-wise work folded into GEMM epilogues a
 * O and MLP-down projections carry the residual add in their epilogue; their per-feature output
   scales (``attn_scale``, ``mlp_scale``) are folded into the bf16 weight copies at cast time, and the
   scale gradients are recovered from the un-scaled weight gradient (``d_scale[n] = sum_k W[n,k] G[n,k]``);
-* MLP-up stores the pre-activation and ``leaky_relu(.)^2`` from one accumulator read; the
-  down-projection's dX GEMM multiplies by the activation derivative in its epilogue;
+* MLP-up stores ``leaky_relu(.)^2`` and, for a backward, one sign bit per value; the down-projection's dX GEMM
+  multiplies by the activation derivative in its epilogue, with the pre-activation taken back as the signed root
+  (exact for a slope of 0 or a power of two below 1; other slopes store the pre-activation beside the activation);
 * tied-embedding logits are produced in bf16 and overwritten in place by their gradient in the
   soft-capped cross-entropy kernel.
 
@@ -85,6 +86,8 @@ class CudaEngine:
         self.n, self.d, self.kv, self.mlp, self.H, self.Hkv, self.hd = m.num_layers, m.model_dim, m.kv_dim, m.mlp_dim, m.num_heads, m.num_kv_heads, m.head_dim
         self.qkvw = self.d + 2 * self.kv
         self.slope = m.leaky_slope if m.activation == "leaky_relu_sq" else 0.0
+        # the backward can take the pre-activation from the activation's root and a sign bit (none needed for relu^2)
+        self.act_root = N.act_root_supported(self.slope)
         self.enc = self.n // 2
         self.sched = gpt.layer_schedule(m)                     # (layer, pass) per activation slot
         self.nslots = len(self.sched)
@@ -140,6 +143,7 @@ class CudaEngine:
         # for per-layer gradient reduction overlapped with the rest of the backward (role of `GpuBackwardLayerObserver`,
         # pg-model/src/gpu.rs:517-525).
         self.backward_observer = None
+        self.want_grad = False           # whether the pass under way has a backward (set by `forward`)
         self.want = None                 # names whose gradients the backward has to produce (None: every parameter)
         self.adam_t = 0
         self.layer_flags = None          # set by the sharded optimizer: per-layer weight-ready counters
@@ -318,7 +322,11 @@ class CudaEngine:
         self.yg = [[buf(T, d) for _ in range(L)] for _ in self.gates]          # gated attention outputs, one list per gate
         self.gv = [[torch.empty(T, self.H, dtype=torch.float32, device=dev) for _ in range(L)] for _ in self.gates]
         self.zz = [None] * L                 # what the output projection consumed in each slot
-        self.hu, self.a = per_layer(T, self.mlp), per_layer(T, self.mlp)
+        self.a = per_layer(T, self.mlp)
+        self.hu = None if self.act_root else per_layer(T, self.mlp)
+        self.signs = [None] * L
+        if self.act_root and self.slope > 0 and self.train:
+            self.signs = [buf(self.mlp // 32, T, dtype=torch.int32) for _ in range(L)]
         self.x_out = [buf(T, d) for _ in range(self.nslots)]
         self.lse = [None] * L
         self.hf = buf(T, d)
@@ -563,7 +571,10 @@ class CudaEngine:
         self.gemm(zz, Wo, self.x_mid[li], epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_in[li])
         if not self.parallel:
             C.mix_norm_fwd(self.x_mid[li], None, None, None, None, None, self.mm[li], s_l, self.eps)
-        self.gemm(self.mm[li], Wup, self.hu[li], epi=N.EPI_ACT_SQ, slope=self.slope, D2=self.a[li])
+        if self.act_root:
+            C.gemm_act(self.mm[li], Wup, self.a[li], self.signs[li] if self.want_grad else None, self.slope, N.status_word(self.dev), self.T)
+        else:
+            self.gemm(self.mm[li], Wup, self.hu[li], epi=N.EPI_ACT_SQ, slope=self.slope, D2=self.a[li])
         xo = self.x_out[j]
         if not recompute:
             self.gemm(self.a[li], Wd, xo, epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_mid[li])
@@ -578,6 +589,7 @@ class CudaEngine:
         if self.cast_generation != self.param_generation:
             raise RuntimeError(f"stale bf16 weights: parameters are at generation {self.param_generation}, the compute copies at "
                                f"{self.cast_generation}; call cast_weights() after changing parameters")
+        self.want_grad = want_grad
         if self.lora is not None:
             self._lora_refresh()
         if ids is not None:                       # otherwise self.ids / self.tgt were filled by `load_span`
@@ -678,7 +690,10 @@ class CudaEngine:
             # ---- MLP
             if self._wants("mlp_down_bank", "mlp_scale"):
                 self._dw_folded(self.dx, self.a[aj], self.Gd, C.fold_scaled_grad_bf16, *view["down"])
-            self.gemm(self.dx, Wd, self.d_hu, True, False, N.EPI_MUL_ACTGRAD, slope=self.slope, aux=self.hu[aj])
+            if self.act_root:
+                C.gemm_actgrad(self.dx, Wd, self.d_hu, self.a[aj], self.signs[aj], self.slope, N.status_word(self.dev), self.T)
+            else:
+                self.gemm(self.dx, Wd, self.d_hu, True, False, N.EPI_MUL_ACTGRAD, slope=self.slope, aux=self.hu[aj])
             if self._wants("mlp_up_bank"):
                 self._dw(self.d_hu, self.mm[aj], view["up"])
             self.gemm(self.d_hu, Wup, self.d_m, True, False)

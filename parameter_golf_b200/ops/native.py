@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import importlib
 import importlib.util
+import math
 import os
 
 import torch
@@ -170,6 +171,11 @@ def gemm_qkv_norm_rope(h, W, pre, post, cos, sin, gain, H, Hkv, rope_dims, seq_l
 
 def qkv_epilogue_supported(hd, rope_dims):
     return hd == 64 and rope_dims in (0, 16, 32, 64)
+
+
+def act_root_supported(slope):
+    """Whether `gemm_act` / `gemm_actgrad` take this slope: 0, or a power of two below 1 (slope * h is then exact in bf16)."""
+    return slope == 0.0 or (0.0 < slope < 1.0 and math.frexp(slope)[0] == 0.5)
 
 
 def attn_fwd(q, k, v, y, B, S, H, Hkv, hd, lse=None, z=None, xsa_eps=1e-8):
