@@ -15,8 +15,8 @@
 // CTA = 10 warps: warp 0 issues TMA loads, warp 1 owns TMEM and issues the MMAs (one elected lane),
 // warps 2..9 read the accumulator back (tcgen05.ld, one row per thread) and run the epilogue. Two
 // accumulators (2 x BN TMEM columns) let the epilogue of tile i overlap the main loop of tile i+1.
-// Tile 128 x BN x 64, BN in {64, 128, 256} (`pick_tile`); grid = min(#tiles, #SMs); tile index = n fastest so CTAs
-// working at the same time share the rows of the large operand in L2. The 64-column form has four epilogue warps (6 warps in all).
+// Tile 128 x BN x 64, BN in {64, 128, 256} (`pick_tile`), 256 x 256 by a pair of CTAs in most of the 256-column forms (`tile_ctas`);
+// grid = min(#tiles, #SMs); tile index = n fastest so CTAs working at the same time share the rows of the large operand in L2. The 64-column form has four epilogue warps (6 warps in all).
 #include <cmath>
 
 #include "common.cuh"
@@ -31,6 +31,12 @@ constexpr int BK = 64;
 // TMA warp, MMA warp, epilogue warps: two per TMEM lane quarter (one for 64 columns, so that a warp still owns whole heads)
 constexpr int epi_warps(int bn) { return bn == 64 ? 4 : 8; }
 constexpr int gemm_threads(int bn) { return 64 + 32 * epi_warps(bn); }
+// 256-column tiles are computed by two CTAs on neighbouring SMs: 256 rows, 128 in each one's tensor memory, each holding its own rows of A
+// and half of B's columns in shared memory. A K step then pulls 32 KB through L2 per CTA instead of 48, which is what bounds the
+// large products (98,304 x 1536 x 512: 1.8 GB of operands). us alone / in pairs, 98,304 rows: 512 columns from 1536 125 / 111, with
+// the residual 139 / 127, 512 from 1024 94 / 82; weight gradients of 512 x 1536 119 / 109. Not where a short sum meets a second operand:
+// the output stage is then the longer part, and a pair's two have to wait for each other (activation gradient from 512 195 / 217).
+constexpr int tile_ctas(int bn, int epi) { return bn == 256 && epi != EPI_RESID_BF16 && epi != EPI_MUL_ACTGRAD && epi != EPI_MUL_ACTROOT ? 2 : 1; }
 
 struct GemmKernelParams {
   int M, N, K, batch;
@@ -47,6 +53,7 @@ struct GemmKernelParams {
   int wait_value;
   int seg_rows[2];        // fp32 epilogues: rows >= seg_rows[k] (> 0) are written to seg_D[k] as row m - seg_rows[k]
   float* seg_D[2];
+  int aligned;             // rows of the bf16 outputs and of the second operand start on 16-byte boundaries
   int aux_l2_prefetch;     // the producer warp pulls the next tile's second operand into L2 through `map_x`
   const float* batch_sumsq;   // optional: alpha and beta of batch b are multiplied by 1 / (sqrt(batch_sumsq[b]) + 1e-7) ^ sumsq_pow
   int sumsq_pow;
@@ -61,20 +68,25 @@ struct GemmKernelParams {
 constexpr int STG_PITCH = 64;
 constexpr int STG_WARP_BYTES = 32 * STG_PITCH;      // one 32-row x 32-column bf16 chunk
 
-// Epilogue staging: two chunk-sized slots per epilogue warp. A slot first receives a chunk of the epilogue's second
-// operand (cp.async, two chunks ahead of its use), is read, then stages the output chunk in place.
+// Epilogue staging: two chunk-sized slots per epilogue warp, first behind the operand stages so that they start on the 512 bytes their
+// swizzle repeats after. Without a second operand they hold outputs on their way out, in turn. With one, a slot first receives a
+// chunk of it (cp.async, two chunks ahead of its use), is read, then stages the output chunk in place.
 constexpr int SGN_BYTES = 32 * 4;                   // the sign words of one chunk
 template <int BN, int EPI>
 struct GemmSmem {
   static constexpr int A_BYTES = BM * BK * 2;
-  static constexpr int B_BYTES = BN * BK * 2;
+  static constexpr int CTAS = tile_ctas(BN, EPI);
+  static constexpr int B_ROWS = BN / CTAS;
+  static constexpr int B_BYTES = B_ROWS * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128) ? 6 : 8;
+  static constexpr int STAGES = BN == 64 ? 8 : BN == 128 || CTAS == 2 ? 6 : 4;     // pairs with five and four slots: 512 columns from 1536 118 us, not 111
   static constexpr int TILE_BYTES = STAGES * STAGE_BYTES;
   static constexpr int STG_BYTES = epi_warps(BN) * 2 * STG_WARP_BYTES;
   static constexpr int SGN_TOTAL = EPI == EPI_MUL_ACTROOT ? epi_warps(BN) * 2 * SGN_BYTES : 0;
-  // the declaration aligns the memory to 1024 bytes; the slack stays where there is room for it
-  static constexpr int TOTAL = TILE_BYTES + (SGN_TOTAL ? 0 : 1024) + 256 /*barriers*/ + STG_BYTES + SGN_TOTAL;
+  static constexpr int BAR_BYTES = 256;             // 2 per stage, 4 for the accumulators, two words
+  // the declaration aligns the memory to 1024 bytes; slack for it stays where there is room
+  static constexpr int TOTAL = TILE_BYTES + STG_BYTES + BAR_BYTES + SGN_TOTAL + (SGN_TOTAL ? 0 : 1024);
+  static_assert(8 * (2 * STAGES + 4) + 8 <= BAR_BYTES, "barriers");
   static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
 };
 
@@ -181,28 +193,26 @@ __device__ __forceinline__ void epilogue_chunk(const GemmKernelParams& p, float 
   }
 }
 
-// Aligned bf16 epilogue with coalesced global traffic. A thread owns one accumulator row, but 16-byte accesses of 32
-// different rows per instruction touch half a sector each; here rows are exchanged through a per-warp shared-memory
-// tile (32 rows x 64 B) so that every global load/store instruction covers 8 rows x 64 contiguous bytes.
-// `auxs` is this chunk of the second operand, already in shared memory in the same swizzled layout (cp.async wrote it).
-// The tile is XOR-swizzled: the 16-byte piece p of row r sits at piece p ^ ((r >> 1) & 3). Both access patterns are
-// then free of bank conflicts (8 consecutive rows x one piece, and 2 consecutive rows x 4 pieces, each cover all 32
-// banks once); a padded pitch can only satisfy one of the two.
+// Aligned bf16 epilogue. A thread owns one accumulator row, but 16-byte accesses of 32 different rows per instruction touch half a
+// sector each, so chunks of 32 rows x 64 bytes go through shared memory. An output without a second operand leaves by a TMA store:
+// one thread asks, and the warp neither computes addresses nor waits (98,304 rows: QKV 138 us with loads and stores of its own, 125 so;
+// 1,024 columns 98 and 92). With a second operand the warp copies by itself, 8 rows x 64 contiguous bytes per instruction: the
+// operand's, the output's and the prefetch's boxes of 64-byte rows are more than the TMA has time for beside the main loop's (the
+// activation gradient took 211 us that way, 195 so).
+// The chunk is XOR-swizzled: the 16-byte piece p of row r sits at piece p ^ ((r >> 1) & 3), the 64-byte swizzle of the tensor maps,
+// under which all these access patterns (8 consecutive rows x one piece, 2 rows x 4 pieces, the TMA's) are free of bank conflicts.
 __device__ __forceinline__ int stg_off(int row, int piece) { return row * STG_PITCH + ((piece ^ ((row >> 1) & 3)) << 4); }
 
+// Outputs of one chunk: this thread's row of 32 values, packed. `ax` is the row of the second operand, `sg` its sign word.
 template <int EPI>
-__device__ __forceinline__ void epilogue_chunk_staged(const GemmKernelParams& p, float alpha, float beta, int b, int m_base, int lane, int n0, const uint32_t (&r)[32],
-                                                      const uint8_t* auxs, uint8_t* stg, uint32_t sg) {
-  constexpr bool HAS_AUX = epi_has_aux(EPI);
-  const int srow = lane >> 2, spc = lane & 3;
+__device__ __forceinline__ void epilogue_math(const GemmKernelParams& p, float alpha, float beta, int m_base, int lane, int n0, const uint32_t (&r)[32],
+                                              const uint32_t (&ax)[16], uint32_t sg, uint32_t (&pk)[16], uint32_t (&pk2)[16]) {
   float a[32];
-  if constexpr (HAS_AUX) {
+  if constexpr (epi_has_aux(EPI)) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint4 q = *reinterpret_cast<const uint4*>(auxs + stg_off(lane, i));
-      const float2 f0 = unpack_bf16x2(q.x), f1 = unpack_bf16x2(q.y), f2 = unpack_bf16x2(q.z), f3 = unpack_bf16x2(q.w);
-      a[8 * i] = f0.x; a[8 * i + 1] = f0.y; a[8 * i + 2] = f1.x; a[8 * i + 3] = f1.y;
-      a[8 * i + 4] = f2.x; a[8 * i + 5] = f2.y; a[8 * i + 6] = f3.x; a[8 * i + 7] = f3.y;
+    for (int i = 0; i < 16; ++i) {
+      const float2 f = unpack_bf16x2(ax[i]);
+      a[2 * i] = f.x; a[2 * i + 1] = f.y;
     }
   }
   float o[32], o2[32];
@@ -241,7 +251,6 @@ __device__ __forceinline__ void epilogue_chunk_staged(const GemmKernelParams& p,
       o[i] = v * 2.f * act_fn(h, p.slope) * (h >= 0.f ? 1.f : p.slope);
     }
   }
-  uint32_t pk[16], pk2[16];
   bool packed = false;
   if constexpr (EPI == EPI_ACT_SQ_SIGN) {
     packed = true;
@@ -292,21 +301,6 @@ __device__ __forceinline__ void epilogue_chunk_staged(const GemmKernelParams& p,
       if constexpr (EPI == EPI_ACT_SQ) pk2[i] = pack_bf16x2(o2[2 * i], o2[2 * i + 1]);
     }
   }
-  auto put = [&](const uint32_t (&x)[16], void* base) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      *reinterpret_cast<uint4*>(stg + stg_off(lane, i)) = make_uint4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
-    __syncwarp();
-    __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(base) + (long long)b * p.stride_d + n0 + spc * 8;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = m_base + i * 8 + srow;
-      if (row < p.M) *reinterpret_cast<uint4*>(d + (long long)row * p.ldd) = *reinterpret_cast<const uint4*>(stg + stg_off(i * 8 + srow, spc));
-    }
-    __syncwarp();
-  };
-  put(pk, p.D);
-  if constexpr (EPI == EPI_ACT_SQ) put(pk2, p.D2);
 }
 
 // Half-split rotary on the first 2*HALF of a head's 64 values, tables [seq_len][HALF] (the layout of `qk_norm_rope_fwd`).
@@ -333,30 +327,17 @@ __device__ __forceinline__ void rope_head(float (&x)[64], const float* __restric
 // RMS-normalised, rotated and (queries) gain-scaled head goes to D2. The norm is taken of the bf16-rounded projection, the
 // values the backward recomputes it from. Replaces a pass over the projection (`qk_norm_rope_fwd`, kept for the LoRA path);
 // same math as the reference's fused QK kernels (parameter-golf-rs/crates/pg-kernels/src/gpu_kernels.rs:2640-2822).
-__device__ __forceinline__ void epilogue_qkv_head_staged(const GemmKernelParams& p, int b, int m_base, int lane, int n0, const uint32_t (&ra)[32],
-                                                         const uint32_t (&rb)[32], uint8_t* stg) {
-  const int srow = lane >> 2, spc = lane & 3;
-  auto put = [&](const uint32_t* x, void* base, int col0) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      *reinterpret_cast<uint4*>(stg + stg_off(lane, i)) = make_uint4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
-    __syncwarp();
-    __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(base) + (long long)b * p.stride_d + col0 + spc * 8;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = m_base + i * 8 + srow;
-      if (row < p.M) *reinterpret_cast<uint4*>(d + (long long)row * p.ldd) = *reinterpret_cast<const uint4*>(stg + stg_off(i * 8 + srow, spc));
-    }
-    __syncwarp();
-  };
+template <typename Put>
+__device__ __forceinline__ void epilogue_qkv_head(const GemmKernelParams& p, int m_base, int lane, int n0, const uint32_t (&ra)[32],
+                                                  const uint32_t (&rb)[32], Put put) {
   uint32_t pk[32];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     pk[i] = pack_bf16x2(__uint_as_float(ra[2 * i]) * p.alpha, __uint_as_float(ra[2 * i + 1]) * p.alpha);
     pk[16 + i] = pack_bf16x2(__uint_as_float(rb[2 * i]) * p.alpha, __uint_as_float(rb[2 * i + 1]) * p.alpha);
   }
-  put(pk, p.D, n0);
-  put(pk + 16, p.D, n0 + 32);
+  put(pk, 0, n0);
+  put(pk + 16, 0, n0 + 32);
   const int head = n0 >> 6;
   if (head >= p.qk_heads) return;                  // value heads: the projection as it is (warp-uniform)
   float x[64];
@@ -382,20 +363,25 @@ __device__ __forceinline__ void epilogue_qkv_head_staged(const GemmKernelParams&
   const float g = (head < p.q_heads && p.head_gain != nullptr) ? p.head_gain[head] : 1.f;
 #pragma unroll
   for (int i = 0; i < 32; ++i) pk[i] = pack_bf16x2(x[2 * i] * g, x[2 * i + 1] * g);     // one rounding, at the store
-  put(pk, p.D2, n0);
-  put(pk + 16, p.D2, n0 + 32);
+  put(pk, 1, n0);
+  put(pk + 16, 1, n0 + 32);
 }
 
 template <int BN, bool A_KMAJOR, bool B_KMAJOR, int EPI>
 __global__ void __launch_bounds__(gemm_threads(BN), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    const __grid_constant__ CUtensorMap map_x, const GemmKernelParams p) {
+                    const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_d2,
+                    const GemmKernelParams p) {
   using S = GemmSmem<BN, EPI>;
   constexpr int STAGES = S::STAGES;
   constexpr uint32_t TMEM_COLS = 2 * BN;            // 128, 256 or 512: two accumulators
+  constexpr bool PAIR = S::CTAS == 2;
+  constexpr int TILE_M = BM * S::CTAS;
+  const int rank = PAIR ? (int)(blockIdx.x & 1) : 0;          // which CTA of the pair; the first one issues the MMAs of both
+  const int first_tile = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, tile_step = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::TILE_BYTES);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::TILE_BYTES + S::STG_BYTES);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tfull_bar = empty_bar + STAGES;
   uint64_t* tempty_bar = tfull_bar + 2;
@@ -412,21 +398,22 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 32 * epi_warps(BN));
+      mbar_init(&tempty_bar[a], S::CTAS * epi_warps(BN));       // one arrival per epilogue warp, of both CTAs
     }
     *abort_flag = 0;
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
-    tmem_relinquish();
+    tmem_alloc<PAIR>(tmem_slot, TMEM_COLS);
+    tmem_relinquish<PAIR>();
   }
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&map_a);
     tma_prefetch_desc(&map_b);
   }
   tc_fence_before();
-  __syncthreads();
+  if constexpr (PAIR) cluster_sync();               // the other CTA's barriers are set up before anything arrives on them
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   chain_next();
@@ -462,58 +449,63 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         asm volatile("fence.proxy.async.global;" ::: "memory");
       }
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+      for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
         const int b = tile / tiles_per_batch;
         int r = tile - b * tiles_per_batch;
         const int split = r / (p.tiles_m * p.tiles_n);
         r -= split * p.tiles_m * p.tiles_n;
         const int tm = r / p.tiles_n, tn = r - tm * p.tiles_n;
-        const int m0 = tm * BM, n0 = tn * BN;
+        const int m0 = tm * TILE_M + rank * BM, n0 = tn * BN + rank * S::B_ROWS;
         const int kb0 = split * p.kb_per_split;
         const int kb1 = min(kb0 + p.kb_per_split, p.kb_total);
-        if (p.aux_l2_prefetch && tile + (int)gridDim.x < total_tiles) {
+        if (p.aux_l2_prefetch && tile + tile_step < total_tiles) {
           // The epilogue warps read the second operand of this CTA's NEXT tile while they finish this one; ask for it now
           // so that those reads find it in L2.
-          const int nt = tile + gridDim.x;
+          const int nt = tile + tile_step;
           const int pb = nt / tiles_per_batch;
           int pr = nt - pb * tiles_per_batch;
           pr -= (pr / (p.tiles_m * p.tiles_n)) * p.tiles_m * p.tiles_n;
           const int ptm = pr / p.tiles_n, ptn = pr - ptm * p.tiles_n;
 #pragma unroll
           for (int j = 0; j < BN / 64; ++j)
-            if (ptn * BN + 64 * j < p.N) tma_prefetch_l2_3d(&map_x, ptn * BN + 64 * j, ptm * BM, pb);
+            if (ptn * BN + 64 * j < p.N) tma_prefetch_l2_3d(&map_x, ptn * BN + 64 * j, ptm * TILE_M + rank * BM, pb);
         }
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, ST_WAIT_EMPTY, kb)) { ok = false; break; }
           uint8_t* sa = smem + stage * S::STAGE_BYTES;
           uint8_t* sb = sa + S::A_BYTES;
-          mbar_expect_tx(&full_bar[stage], S::STAGE_BYTES);
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], S::CTAS * S::STAGE_BYTES);      // the bytes of both CTAs' loads
           if constexpr (A_KMAJOR) {
-            tma_load_3d(sa, &map_a, &full_bar[stage], kb * BK, m0, b);
+            tma_load_3d<PAIR>(sa, &map_a, &full_bar[stage], kb * BK, m0, b);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_3d(sa + j * 8192, &map_a, &full_bar[stage], m0 + 64 * j, kb * BK, b);
+            for (int j = 0; j < BM / 64; ++j) tma_load_3d<PAIR>(sa + j * 8192, &map_a, &full_bar[stage], m0 + 64 * j, kb * BK, b);
           }
           if constexpr (B_KMAJOR) {
-            tma_load_3d(sb, &map_b, &full_bar[stage], kb * BK, n0, b);
+            tma_load_3d<PAIR>(sb, &map_b, &full_bar[stage], kb * BK, n0, b);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j) tma_load_3d(sb + j * 8192, &map_b, &full_bar[stage], n0 + 64 * j, kb * BK, b);
+            for (int j = 0; j < S::B_ROWS / 64; ++j) tma_load_3d<PAIR>(sb + j * 8192, &map_b, &full_bar[stage], n0 + 64 * j, kb * BK, b);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
       if (!ok) {
-        // drain: every stage whose load may still be in flight
-        for (int s = 0; s < STAGES; ++s) mbar_drain(&full_bar[s], (s < stage) ? phase : (phase ^ 1));
+        // drain: every stage whose load may still be in flight (a pair's loads all report to the first CTA, which the other outlives)
+        if (rank == 0)
+          for (int s = 0; s < STAGES; ++s) mbar_drain(&full_bar[s], (s < stage) ? phase : (phase ^ 1));
+      } else if constexpr (PAIR) {
+        // the last arrivals of the other CTA's MMA thread on this CTA's barriers are in before it leaves
+        for (int i = 0; i < STAGES; ++i) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, ST_WAIT_EMPTY, -1)) break;
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    // The wide QKV product is bound by its output stage, and there the fast issue of an elected thread costs 5 % (98,304 rows: 146 us
-    // against 138 with the branch on the lane number, 24,576 rows: 50 against 48).
-    if ((EPI == EPI_QKV_NORM_ROPE && BN == 256) ? lane == 0 : elect_one()) {
-      constexpr uint32_t IDESC = make_idesc_bf16(BM, BN, A_KMAJOR ? 0 : 1, B_KMAJOR ? 0 : 1);
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t IDESC = make_idesc_bf16(TILE_M, BN, A_KMAJOR ? 0 : 1, B_KMAJOR ? 0 : 1);
       // operand descriptors of stage 0; a stage or K step only adds to their address field
       const uint64_t da0 = A_KMAJOR ? make_smem_desc(smem_u32(smem), 16, 1024) : make_smem_desc(smem_u32(smem), 8192, 1024);
       const uint64_t db0 = B_KMAJOR ? make_smem_desc(smem_u32(smem) + S::A_BYTES, 16, 1024) : make_smem_desc(smem_u32(smem) + S::A_BYTES, 8192, 1024);
@@ -523,7 +515,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+      for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
         int r = tile % tiles_per_batch;
         const int split = r / (p.tiles_m * p.tiles_n);
         const int kb0 = split * p.kb_per_split;
@@ -536,12 +528,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           tc_fence_after();
           const uint32_t at = (uint32_t)stage * (S::STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) umma_ss(tmem_d, da0 + at + k * A_STEP, db0 + at + k * B_STEP, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
-          umma_commit(&empty_bar[stage]);
+          for (int k = 0; k < BK / 16; ++k) umma_ss<PAIR>(tmem_d, da0 + at + k * A_STEP, db0 + at + k * B_STEP, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
+          umma_commit<PAIR>(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit(&tfull_bar[acc]);
+        umma_commit<PAIR>(&tfull_bar[acc]);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
@@ -549,11 +541,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // ------------------------------------------------------------------ epilogue (warps 2..9; 2..5 for 64 columns)
     const int quarter = warp & 3;                 // TMEM lane quarter this warp may access
     const int half = (warp - 2) >> 2;             // which half of the tile's columns
-    uint8_t* slots = smem + S::TILE_BYTES + 256 + (warp - 2) * 2 * STG_WARP_BYTES;
-    uint8_t* sgn = smem + S::TILE_BYTES + 256 + S::STG_BYTES + (warp - 2) * 2 * SGN_BYTES;      // sign words beside each slot
-    const bool staged_ok = (p.ldd % 8 == 0) && (p.stride_d % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.D) & 15) == 0) &&
-                           (p.aux == nullptr || ((p.ld_aux % 8 == 0) && (p.stride_aux % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.aux) & 15) == 0))) &&
-                           (p.D2 == nullptr || ((reinterpret_cast<uintptr_t>(p.D2) & 15) == 0));
+    uint8_t* slots = smem + S::TILE_BYTES + (warp - 2) * 2 * STG_WARP_BYTES;
+    uint8_t* sgn = smem + S::TILE_BYTES + S::STG_BYTES + S::BAR_BYTES + (warp - 2) * 2 * SGN_BYTES;      // sign words beside each slot
+    const bool leader = elect_one();              // issues this warp's stores and waits for them
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
@@ -569,19 +559,38 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       tm = r / p.tiles_n;
       tn = r - tm * p.tiles_n;
     };
+    auto fill = [&](uint8_t* slot, const uint32_t* x) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(slot + stg_off(lane, i)) = make_uint4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+    };
+    // A chunk of output by TMA: into a slot once the store that last left it has read it, then out.
+    int out = 1;
+    auto put = [&](const uint32_t* x, int second, int b, int m_base, int col) {
+      out ^= 1;
+      uint8_t* slot = slots + out * STG_WARP_BYTES;
+      if (leader) bulk_wait_read<1>();                     // the latest store is the other slot's
+      __syncwarp();
+      fill(slot, x);
+      fence_proxy_async();
+      __syncwarp();
+      if (leader) {
+        if (m_base < p.M) tma_store_3d(second ? &map_d2 : &map_d, slot, col, m_base, b);
+        bulk_commit();                                     // also of nothing: the wait above counts groups
+      }
+    };
     // Second operand: a 32-row x 32-column chunk goes into one of this warp's two staging slots with 16-byte asynchronous
     // copies (8 rows x 64 contiguous bytes per instruction), one commit group per chunk, two chunks ahead of its use
     // (across the tile boundary too), so its DRAM latency hides behind the chunks processed meanwhile. cp.async is used
     // rather than loads into registers because pending register loads share the warp's few scoreboard counters with the
     // shared-memory and tensor-memory traffic of those chunks, which then wait for DRAM as well. The slot is read by the
     // thread that owns the row, reused in place to stage the output chunk, and refilled once the stores have read it.
-    const bool aux_async = HAS_AUX && staged_ok;
+    const bool aux_async = HAS_AUX && p.aligned;
+    auto whole = [&](int tn, int cc) { return tn * BN + (c_begin + cc) * 32 + 32 <= p.N; };
     auto issue_aux = [&](int b, int tm, int tn, int cc) {
-      uint8_t* slot = slots + (cc & 1) * STG_WARP_BYTES;
       if constexpr (HAS_AUX) {
-        const int n0 = tn * BN + (c_begin + cc) * 32;
-        if (n0 + 32 <= p.N) {
-          const int m_base = tm * BM + quarter * 32;
+        if (whole(tn, cc)) {
+          const int n0 = tn * BN + (c_begin + cc) * 32, m_base = tm * TILE_M + rank * BM + quarter * 32;
+          uint8_t* slot = slots + (cc & 1) * STG_WARP_BYTES;
           const __nv_bfloat16* ap = reinterpret_cast<const __nv_bfloat16*>(p.aux) + (long long)b * p.stride_aux + n0 + (lane & 3) * 8;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -597,21 +606,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
     };
     static_assert(CH % 2 == 0, "slot parity follows the chunk index within the tile");
-    if (aux_async && blockIdx.x < total_tiles) {
+    if (aux_async && first_tile < total_tiles) {
       int b0, tm0, tn0;
-      tile_coords(blockIdx.x, b0, tm0, tn0);
+      tile_coords(first_tile, b0, tm0, tn0);
       issue_aux(b0, tm0, tn0, 0);
       issue_aux(b0, tm0, tn0, 1);
     }
-    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+    for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
       int b, tm, tn;
       tile_coords(tile, b, tm, tn);
-      const int next = tile + gridDim.x;
+      const int next = tile + tile_step;
       int nb = 0, ntm = 0, ntn = 0;
       if (next < total_tiles) tile_coords(next, nb, ntm, ntn);
-      const int m = tm * BM + quarter * 32 + lane;
+      const int m_base = tm * TILE_M + rank * BM + quarter * 32, m = m_base + lane;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
-      const int m_base = tm * BM + quarter * 32;
       float alpha = p.alpha, beta = p.beta;
       if (p.batch_sumsq != nullptr) {
         // Newton-Schulz on an un-normalised input: the matrix norm enters as a per-matrix factor of the whole output
@@ -634,7 +642,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             PGB_TMEM_LD32(taddr + c * 32 + 32, rb);
             PGB_TMEM_WAIT_LD32(ra);
             PGB_TMEM_WAIT_LD32(rb);
-            epilogue_qkv_head_staged(p, b, m_base, lane, n0, ra, rb, slots);
+            epilogue_qkv_head(p, m_base, lane, n0, ra, rb, [&](const uint32_t* x, int second, int col) { put(x, second, b, m_base, col); });
           }
         }
       } else {
@@ -642,7 +650,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       for (int cc = 0; cc < CH; ++cc) {
         const int c = c_begin + cc;
         const int n0 = tn * BN + c * 32;
-        uint8_t* slot = slots + (cc & 1) * STG_WARP_BYTES;
         if (n0 < p.N) {                           // warp-uniform
           uint32_t rr[32];
           PGB_TMEM_LD32(taddr + c * 32, rr);
@@ -653,17 +660,40 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
           }
           PGB_TMEM_WAIT_LD32(rr);
+          bool done = false;
           if constexpr (BF16_OUT) {
-            uint32_t sg = 0;
-            if constexpr (EPI == EPI_MUL_ACTROOT) {
-              if (p.signs != nullptr) sg = *reinterpret_cast<const uint32_t*>(sgn + (cc & 1) * SGN_BYTES + lane * 4);
+            if (p.aligned && whole(tn, cc)) {
+              uint32_t ax[16], pk[16], pk2[16];
+              uint32_t sg = 0;
+              if constexpr (HAS_AUX) {
+                uint8_t* slot = slots + (cc & 1) * STG_WARP_BYTES;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const uint4 q = *reinterpret_cast<const uint4*>(slot + stg_off(lane, i));
+                  ax[4 * i] = q.x; ax[4 * i + 1] = q.y; ax[4 * i + 2] = q.z; ax[4 * i + 3] = q.w;
+                }
+                if constexpr (EPI == EPI_MUL_ACTROOT) {
+                  if (p.signs != nullptr) sg = *reinterpret_cast<const uint32_t*>(sgn + (cc & 1) * SGN_BYTES + lane * 4);
+                }
+                epilogue_math<EPI>(p, alpha, beta, m_base, lane, n0, rr, ax, sg, pk, pk2);
+                fill(slot, pk);
+                __syncwarp();
+                __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + (long long)b * p.stride_d + n0 + (lane & 3) * 8;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const int lr = i * 8 + (lane >> 2);
+                  if (m_base + lr < p.M) *reinterpret_cast<uint4*>(d + (long long)(m_base + lr) * p.ldd) = *reinterpret_cast<const uint4*>(slot + stg_off(lr, lane & 3));
+                }
+              } else {
+                epilogue_math<EPI>(p, alpha, beta, m_base, lane, n0, rr, ax, sg, pk, pk2);
+                put(pk, 0, b, m_base, n0);
+                if constexpr (EPI == EPI_ACT_SQ) put(pk2, 1, b, m_base, n0);
+              }
+              done = true;
             }
-            if constexpr (EPI == EPI_ACT_SQ_SIGN || EPI == EPI_MUL_ACTROOT)          // the host refuses what is not aligned
-              epilogue_chunk_staged<EPI>(p, alpha, beta, b, m_base, lane, n0, rr, slot, slot, sg);
-            else if (staged_ok && n0 + 32 <= p.N && (aux_async || !HAS_AUX)) epilogue_chunk_staged<EPI>(p, alpha, beta, b, m_base, lane, n0, rr, slot, slot, sg);
-            else if (m < p.M) epilogue_chunk<EPI>(p, alpha, beta, b, m, n0, rr);
-          } else {
-            if (m < p.M) epilogue_chunk<EPI>(p, alpha, beta, b, m, n0, rr);
+          }
+          if constexpr (EPI != EPI_ACT_SQ_SIGN && EPI != EPI_MUL_ACTROOT) {      // the host refuses what is not aligned
+            if (!done && m < p.M) epilogue_chunk<EPI>(p, alpha, beta, b, m, n0, rr);
           }
         }
         if constexpr (HAS_AUX) {
@@ -677,16 +707,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
       }
       tc_fence_before();
-      mbar_arrive(&tempty_bar[acc]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive_first<PAIR>(&tempty_bar[acc]);
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
+    if (leader) bulk_wait_all();                  // the stores have read their slots, and their writes are complete
   }
 
   tc_fence_before();
-  __syncthreads();
+  if constexpr (PAIR) cluster_sync();               // neither CTA's shared or tensor memory is used by the other any more
+  else __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc<PAIR>(tmem_base, TMEM_COLS);
   }
 }
 
@@ -720,9 +753,20 @@ static CUtensorMap operand_map(const void* ptr, bool kmajor, int rows, int K, lo
   return make_tmap_bf16(ptr, 3, dims, strides, box);
 }
 
+struct GemmMaps {
+  CUtensorMap a, b, x, d, d2;      // operands, second operand of the epilogue (prefetch only), outputs
+};
+
+// [batch][M][N] bf16 in chunks of 32 x 32, the unit in which an epilogue warp writes
+static CUtensorMap chunk_map(const void* ptr, const GemmArgs& a, long long ld, long long batch_stride) {
+  const uint64_t dims[3] = {(uint64_t)a.N, (uint64_t)a.M, (uint64_t)a.batch};
+  const uint64_t strides[2] = {(uint64_t)ld * 2, (uint64_t)(a.batch > 1 ? batch_stride : (long long)a.M * ld) * 2};
+  const uint32_t box[3] = {32, 32, 1};
+  return make_tmap_bf16(ptr, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
 template <int BN, bool AK, bool BKM, int EPI>
-static void launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mx, const GemmKernelParams& p, int grid,
-                           long long chain_rows, cudaStream_t stream) {
+static void launch_variant(const GemmMaps& m, const GemmKernelParams& p, int grid, long long chain_rows, cudaStream_t stream) {
   auto kern = gemm_tcgen05_kernel<BN, AK, BKM, EPI>;
   static bool configured[64] = {};          // the attribute is a per-device property of the kernel
   int dev = 0;
@@ -731,46 +775,46 @@ static void launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const C
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN, EPI>::TOTAL);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  launch_chained(chain_rows, kern, grid, gemm_threads(BN), GemmSmem<BN, EPI>::TOTAL, stream, ma, mb, mx, p);
+  launch_chained_clusters(chain_rows, tile_ctas(BN, EPI), kern, grid, gemm_threads(BN), GemmSmem<BN, EPI>::TOTAL, stream, m.a, m.b, m.x, m.d, m.d2, p);
 }
 
 template <int BN, int EPI>
-static void launch_major(const GemmArgs& a, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mx, const GemmKernelParams& p, int grid,
+static void launch_major(const GemmArgs& a, const GemmMaps& m, const GemmKernelParams& p, int grid,
                          cudaStream_t stream) {
-  if (a.a_kmajor && a.b_kmajor) launch_variant<BN, true, true, EPI>(ma, mb, mx, p, grid, a.chain_rows, stream);
-  else if (a.a_kmajor && !a.b_kmajor) launch_variant<BN, true, false, EPI>(ma, mb, mx, p, grid, a.chain_rows, stream);
+  if (a.a_kmajor && a.b_kmajor) launch_variant<BN, true, true, EPI>(m, p, grid, a.chain_rows, stream);
+  else if (a.a_kmajor && !a.b_kmajor) launch_variant<BN, true, false, EPI>(m, p, grid, a.chain_rows, stream);
   else if constexpr (BN == 64) throw std::runtime_error("gemm: 64-column tiles take row-major activations");
-  else if (!a.a_kmajor && a.b_kmajor) launch_variant<BN, false, true, EPI>(ma, mb, mx, p, grid, a.chain_rows, stream);
-  else launch_variant<BN, false, false, EPI>(ma, mb, mx, p, grid, a.chain_rows, stream);
+  else if (!a.a_kmajor && a.b_kmajor) launch_variant<BN, false, true, EPI>(m, p, grid, a.chain_rows, stream);
+  else launch_variant<BN, false, false, EPI>(m, p, grid, a.chain_rows, stream);
 }
 
 template <int BN>
-static void launch_epi(const GemmArgs& a, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mx, const GemmKernelParams& p, int grid,
+static void launch_epi(const GemmArgs& a, const GemmMaps& m, const GemmKernelParams& p, int grid,
                        cudaStream_t stream) {
   if constexpr (BN != 64) {
     switch (a.epi) {
-      case EPI_F32: launch_major<BN, EPI_F32>(a, ma, mb, mx, p, grid, stream); return;
-      case EPI_F32_ATOMIC: launch_major<BN, EPI_F32_ATOMIC>(a, ma, mb, mx, p, grid, stream); return;
-      case EPI_RESID_BF16: launch_major<BN, EPI_RESID_BF16>(a, ma, mb, mx, p, grid, stream); return;
+      case EPI_F32: launch_major<BN, EPI_F32>(a, m, p, grid, stream); return;
+      case EPI_F32_ATOMIC: launch_major<BN, EPI_F32_ATOMIC>(a, m, p, grid, stream); return;
+      case EPI_RESID_BF16: launch_major<BN, EPI_RESID_BF16>(a, m, p, grid, stream); return;
       default: break;
     }
   }
   switch (a.epi) {
-    case EPI_BF16: launch_major<BN, EPI_BF16>(a, ma, mb, mx, p, grid, stream); break;
-    case EPI_AXPBY_BF16: launch_major<BN, EPI_AXPBY_BF16>(a, ma, mb, mx, p, grid, stream); break;
-    case EPI_ACT_SQ: launch_major<BN, EPI_ACT_SQ>(a, ma, mb, mx, p, grid, stream); break;
-    case EPI_MUL_ACTGRAD: launch_major<BN, EPI_MUL_ACTGRAD>(a, ma, mb, mx, p, grid, stream); break;
+    case EPI_BF16: launch_major<BN, EPI_BF16>(a, m, p, grid, stream); break;
+    case EPI_AXPBY_BF16: launch_major<BN, EPI_AXPBY_BF16>(a, m, p, grid, stream); break;
+    case EPI_ACT_SQ: launch_major<BN, EPI_ACT_SQ>(a, m, p, grid, stream); break;
+    case EPI_MUL_ACTGRAD: launch_major<BN, EPI_MUL_ACTGRAD>(a, m, p, grid, stream); break;
     case EPI_QKV_NORM_ROPE:
       if (!(a.a_kmajor && a.b_kmajor)) throw std::runtime_error("gemm: the QKV epilogue takes row-major activations and [N][K] weights");
-      launch_variant<BN, true, true, EPI_QKV_NORM_ROPE>(ma, mb, mx, p, grid, a.chain_rows, stream);
+      launch_variant<BN, true, true, EPI_QKV_NORM_ROPE>(m, p, grid, a.chain_rows, stream);
       break;
     case EPI_ACT_SQ_SIGN:
       if (!(a.a_kmajor && a.b_kmajor)) throw std::runtime_error("gemm: the activation with signs takes row-major activations and [N][K] weights");
-      launch_variant<BN, true, true, EPI_ACT_SQ_SIGN>(ma, mb, mx, p, grid, a.chain_rows, stream);
+      launch_variant<BN, true, true, EPI_ACT_SQ_SIGN>(m, p, grid, a.chain_rows, stream);
       break;
     case EPI_MUL_ACTROOT:
       if (!(a.a_kmajor && !a.b_kmajor)) throw std::runtime_error("gemm: the activation gradient from the root takes row-major gradients and [K][N] weights");
-      launch_variant<BN, true, false, EPI_MUL_ACTROOT>(ma, mb, mx, p, grid, a.chain_rows, stream);
+      launch_variant<BN, true, false, EPI_MUL_ACTROOT>(m, p, grid, a.chain_rows, stream);
       break;
     default: throw std::runtime_error("gemm: unknown epilogue");
   }
@@ -782,15 +826,22 @@ struct TilePlan {
 
 // Tile width and number of K splits by estimated time, in SM clocks. An item (one tile, one K split) costs 540 / 285 / 245 clocks
 // per 64-deep K step of a 256 / 128 / 64 column tile (a 64-column MMA is bound by its operand reads) plus an epilogue; a round of
-// items beyond the first costs 0.8 of that, since a main loop overlaps the epilogue before it. The constants were fitted to
-// products of 1024 to 98,304 rows on the model's sites and order the widths as measured there (us, 256 / 128 / 64 columns):
-//   M = 2048,  N = 512,  K = 512   7.7 / 5.6 / 5.0       M = 4096, N = 512, K = 1536   12.5 / 8.9 / 11.0
-//   M = 5760,  N = 512,  K = 1536  12.8 / 13.5 / 14.3    M = 98304, N = 1024, K = 512  99 / 111 / 134
+// items beyond the first costs 0.8 of that, since a main loop overlaps the epilogue before it. A pair's items are twice as tall and
+// there are half as many places for them. The constants were fitted to products of 1024 to 98,304 rows on the model's sites and order the
+// widths as measured there (us with launch, cold caches, 256 / 128 / 64 columns):
+//   M = 2048,  N = 512,  K = 512   14 / 11 / 10          M = 4096, N = 512, K = 1536   20 / 16 / 18
+//   M = 16384, N = 512,  K = 1536  35 / 37 / 41          M = 98304, N = 512, K = 1024  80 / 100
+// With a second operand (AXPBY) a pair's output stage is the longer part unless the sum is long: M = 98304, N = 512: K = 512 84 / 72,
+// K = 1536 123 / 145; M = 16384, K = 512 24 / 23.
 // A narrower tile has to win by 8 %: it reads the activations from L2 more often than the model counts.
 // Weight gradients (fp32 adds): every split adds a whole tile to the output in L2 (~52 clocks per column), so one round with as many
-// splits as fill the SMs beats two rounds (512x1536 from 4096 rows: 3 splits of 128-column tiles 10.4 us, 6 splits 12.3; from
-// 98,304 rows 6 splits of 256 columns 118 us, 12 splits 122), and narrow tiles win while the sum is short.
-static TilePlan pick_tile(const GemmArgs& a, int tiles_m, int kb_total, int sms) {
+// splits as fill the SMs beats two rounds (512x1536 from 4096 rows: 3 splits of 128-column tiles 10.4 us, 6 splits 12.3), and narrow tiles win while the sum is short.
+static int tile_count(const GemmArgs& a, int bn) {
+  const int rows = BM * tile_ctas(bn, a.epi);
+  return ((a.M + rows - 1) / rows) * ((a.N + bn - 1) / bn) * a.batch;
+}
+
+static TilePlan pick_tile(const GemmArgs& a, int kb_total, int sms) {
   TilePlan best{0, 1};
   double best_cost = 0.0;
   const bool atomic = a.epi == EPI_F32_ATOMIC;
@@ -798,16 +849,16 @@ static TilePlan pick_tile(const GemmArgs& a, int tiles_m, int kb_total, int sms)
     if (a.tile_n > 0 && bn != a.tile_n) continue;
     if (a.tile_n <= 0 && bn == 256 && a.N <= 128) continue;
     if (bn == 64 && (!a.a_kmajor || a.epi == EPI_F32 || a.epi == EPI_RESID_BF16 || atomic)) continue;
-    const int base = tiles_m * ((a.N + bn - 1) / bn) * a.batch;
+    const int base = tile_count(a, bn), units = sms / tile_ctas(bn, a.epi);
     const double step = bn == 256 ? 540.0 : bn == 128 ? 285.0 : 245.0;
-    const double epi = atomic ? 52.0 * bn : bn == 256 ? 4900.0 : bn == 128 ? 2900.0 : 2000.0;
+    const double epi = atomic ? 52.0 * bn : bn == 256 ? (a.epi == EPI_AXPBY_BF16 ? 7500.0 : 4900.0) : bn == 128 ? 2900.0 : 2000.0;
     int last = 0;
     for (int waves : {1, 2, 3}) {
       int splits = std::max(1, a.splits);
-      if (atomic && a.splits <= 0) splits = std::min(std::max(1, kb_total / 4), std::max(1, waves * sms / base));
+      if (atomic && a.splits <= 0) splits = std::min(std::max(1, kb_total / 4), std::max(1, waves * units / base));
       if (splits == last) continue;
       last = splits;
-      const int rounds = (base * splits + sms - 1) / sms;
+      const int rounds = (base * splits + units - 1) / units;
       const double cost = (step * ((kb_total + splits - 1) / splits) + epi) * (1.0 + 0.8 * (rounds - 1));
       if (best.bn == 0 || cost < 0.92 * best_cost) {
         best = {bn, splits};
@@ -824,10 +875,10 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   if ((a.lda % 8) || (a.ldb % 8)) throw std::runtime_error("gemm: leading dimensions must be multiples of 8 elements");
   GemmKernelParams p;
   p.M = a.M; p.N = a.N; p.K = a.K; p.batch = a.batch;
-  p.tiles_m = (a.M + BM - 1) / BM;
   p.kb_total = (a.K + BK - 1) / BK;
-  const TilePlan plan = pick_tile(a, p.tiles_m, p.kb_total, num_sms());
+  const TilePlan plan = pick_tile(a, p.kb_total, num_sms());
   const int bn = plan.bn, splits = plan.splits;
+  p.tiles_m = (a.M + BM * tile_ctas(bn, a.epi) - 1) / (BM * tile_ctas(bn, a.epi));
   p.tiles_n = (a.N + bn - 1) / bn;
   if (splits > 1 && a.epi != EPI_F32_ATOMIC) throw std::runtime_error("gemm: split-K needs the atomic fp32 epilogue");
   p.kb_per_split = (p.kb_total + splits - 1) / splits;
@@ -870,18 +921,25 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
         (reinterpret_cast<uintptr_t>(a.D) & 15) || (reinterpret_cast<uintptr_t>(a.D2) & 15))
       throw std::runtime_error("gemm: the QKV epilogue needs heads of 64, rope_dims in {0,16,32,64}, 16-byte aligned outputs of one row pitch and a sequence length");
   }
-  const CUtensorMap ma = operand_map(a.A, a.a_kmajor, a.M, a.K, a.lda, a.stride_a, a.batch, BM);
-  const CUtensorMap mb = operand_map(a.B, a.b_kmajor, a.N, a.K, a.ldb, a.stride_b, a.batch, bn);
+  GemmMaps m;
+  m.a = operand_map(a.A, a.a_kmajor, a.M, a.K, a.lda, a.stride_a, a.batch, BM);
+  m.b = operand_map(a.B, a.b_kmajor, a.N, a.K, a.ldb, a.stride_b, a.batch, bn / tile_ctas(bn, a.epi));
   const int total = p.tiles_m * p.tiles_n * p.splits * a.batch;
-  const int grid = std::min(total, num_sms());
+  const int grid = std::min(total, num_sms() / tile_ctas(bn, a.epi)) * tile_ctas(bn, a.epi);
+  auto rows_ok = [&](const void* ptr, long long ld, long long stride) {
+    return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0 && ld % 8 == 0 && (a.batch == 1 || stride % 8 == 0);
+  };
+  const bool aux = a.aux != nullptr && epi_has_aux(a.epi), two = a.D2 != nullptr && (a.epi == EPI_ACT_SQ || a.epi == EPI_QKV_NORM_ROPE);
+  p.aligned = rows_ok(a.D, a.ldd, a.stride_d) && (!two || rows_ok(a.D2, a.ldd, a.stride_d)) && (!aux || rows_ok(a.aux, a.ld_aux, a.stride_aux));
+  const bool stores = p.aligned && !aux && a.epi != EPI_F32 && a.epi != EPI_F32_ATOMIC;
+  m.d = stores ? chunk_map(a.D, a, a.ldd, a.stride_d) : m.a;
+  m.d2 = stores && two ? chunk_map(a.D2, a, a.ldd, a.stride_d) : m.a;
   // L2 prefetch of the epilogue's second operand ([batch][M][N] bf16, row pitch ld_aux) one tile ahead of its readers
-  const bool has_aux = a.aux != nullptr && (a.epi == EPI_AXPBY_BF16 || a.epi == EPI_MUL_ACTGRAD || a.epi == EPI_MUL_ACTROOT);
-  p.aux_l2_prefetch = (has_aux && a.ld_aux % 8 == 0 && (a.batch == 1 || a.stride_aux % 8 == 0) &&
-                       (reinterpret_cast<uintptr_t>(a.aux) & 15) == 0 && total > grid) ? 1 : 0;
-  const CUtensorMap mx = p.aux_l2_prefetch ? operand_map(a.aux, true, a.M, a.N, a.ld_aux, a.stride_aux, a.batch, BM) : ma;
-  if (bn == 256) launch_epi<256>(a, ma, mb, mx, p, grid, stream);
-  else if (bn == 128) launch_epi<128>(a, ma, mb, mx, p, grid, stream);
-  else launch_epi<64>(a, ma, mb, mx, p, grid, stream);
+  p.aux_l2_prefetch = p.aligned && aux && total > grid / tile_ctas(bn, a.epi) ? 1 : 0;
+  m.x = p.aux_l2_prefetch ? operand_map(a.aux, true, a.M, a.N, a.ld_aux, a.stride_aux, a.batch, BM) : m.a;
+  if (bn == 256) launch_epi<256>(a, m, p, grid, stream);
+  else if (bn == 128) launch_epi<128>(a, m, p, grid, stream);
+  else launch_epi<64>(a, m, p, grid, stream);
 }
 
 }  // namespace pgb

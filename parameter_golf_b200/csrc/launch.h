@@ -13,18 +13,32 @@ namespace pgb {
 constexpr long long CHAIN_ROWS = 16384;
 
 template <typename... P, typename... A>
-inline void launch_chained(long long rows, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+inline void launch_chained_clusters(long long rows, int ctas, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (rows > 0 && rows <= CHAIN_ROWS) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (ctas > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = ctas;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = rows > 0 && rows <= CHAIN_ROWS ? 1 : 0;
+  cfg.numAttrs = n;
   cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+template <typename... P, typename... A>
+inline void launch_chained(long long rows, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  launch_chained_clusters(rows, 1, kern, grid, block, smem, st, static_cast<A&&>(args)...);
 }
 
 }  // namespace pgb

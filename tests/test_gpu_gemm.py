@@ -213,6 +213,33 @@ def test_every_tile_width_gives_the_same_product(tile_n, M, N, K):
             n.gemm(A, W, torch.empty(M, N, device="cuda"), epi=n.EPI_F32, tile_n=64)
 
 
+@pytest.mark.parametrize("M,N,K,batch", [(1, 256, 64, 1), (128, 264, 72, 2), (257, 512, 512, 1), (255, 320, 200, 3), (5000, 1000, 136, 1)])
+def test_tiles_of_a_cta_pair_are_those_of_one_cta(M, N, K, batch):
+    """256-column tiles (two CTAs) against 128-column tiles (one): the same sums in the same order, so the same bits; all majors, second
+    CTAs without rows or columns, batches, outputs whose rows are not aligned (these leave by plain stores) and an operand in place."""
+    n = _n()
+    torch.manual_seed(M + N)
+    shape = lambda *s: (batch, *s) if batch > 1 else s
+    K8 = K // 8 * 8
+    for ak in (True, False):
+        for bk in (True, False):
+            m = M if ak else (M + 7) // 8 * 8                       # row strides are multiples of 8 elements
+            A = _rand(*shape(m, K8) if ak else shape(K8, m))
+            W = _rand(*shape(N, K8) if bk else shape(K8, N), scale=K ** -0.5)
+            for pad in (0, 1):
+                out = []
+                for tile in (128, 256):
+                    Y = torch.full(shape(m, N + 8), 3.0, device="cuda", dtype=torch.bfloat16)
+                    D, Z = Y[..., pad:N + pad], torch.full(shape(m, N), 2.0, device="cuda")
+                    n.gemm(A, W, D, ak, bk, tile_n=tile)
+                    n.gemm(A, W, D, ak, bk, n.EPI_AXPBY_BF16, alpha=0.5, beta=0.5, aux=D, tile_n=tile)
+                    n.gemm(A, W, Z, ak, bk, n.EPI_F32, tile_n=tile)
+                    n.gemm(A, W, Z, ak, bk, n.EPI_F32_ATOMIC, splits=1, tile_n=tile)
+                    out.append((Y, Z))
+                assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]), (ak, bk, pad)
+    n.check_status()
+
+
 def _early_starts(fn):
     """Kernels of ``fn`` that may start before the one ahead of them has finished: programmatic edges of its captured graph."""
     import ctypes
