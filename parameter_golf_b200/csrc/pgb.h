@@ -179,6 +179,11 @@ void expand_span_u16(const void* span, int* ids, int* targets, int n, cudaStream
 // ---- post-training quantisation (gptq.cu) --------------------------------------------------------------------------------
 // GPTQ with fixed per-row scales: Wp [rows, cols] fp32 (columns already in activation order), U [cols, cols] upper
 // Cholesky factor of the inverse Hessian, scales [candidates, rows], Q int8 codes [candidates, rows, cols] out. Column blocks of 128.
+// U [c][c] (fp32, upper) with inv(P H P^T) = U^T U, P H P^T being H [c][c] with rows and columns in the REVERSE of `order`. `work` has
+// gptq_factor_work_doubles(c) doubles; info[0] (of two ints) becomes 0, the order of the leading minor that is not positive, or -1 where
+// a bounded wait ran out. One cooperative launch.
+size_t gptq_factor_work_doubles(int c);
+void gptq_factor(const float* H, const long long* order, double* work, float* U, int* info, int c, cudaStream_t st);
 void gptq_rows(const float* Wp, const float* U, const float* scales, int8_t* Q, int candidates, int rows, int cols, int bits, cudaStream_t st);
 
 // ---- attention (attn_fwd.cu, attn_bwd.cu): causal, grouped KV heads, head_dim 64, bf16 ----------------------------------

@@ -238,6 +238,25 @@ def softcap_logits(z, cap):
     return out
 
 
+def gptq_factor(H, order):
+    """Upper ``U`` with ``inv(H[p][:, p]) = U^T U``, ``p`` being ``order`` reversed, and the int32 word that says whether ``H`` was positive
+    definite (`gptq_factor_check`; asked after the work behind this call has been queued, it costs no idle time). Not counted by
+    `launch_count`: a call of `quant.gptq.gptq_quantize` counts its row kernels."""
+    U = torch.empty_like(H)
+    info = torch.empty(2, dtype=torch.int32, device=H.device)
+    load_raw().gptq_factor(H, order, U, info)
+    return U, info
+
+
+def gptq_factor_check(info):
+    k = int(info[0])
+    if k > 0:
+        raise torch.linalg.LinAlgError("linalg.cholesky: The factorization could not be completed because the input is not positive-definite "
+                                       f"(the leading minor of order {k} is not positive-definite).")
+    if k < 0:
+        raise RuntimeError("gptq_factor: a wait inside the kernel ran out")
+
+
 def gptq_rows(Wp, U, scales, bits, block=128):
     """GPTQ row kernel: int8 codes for the permuted rows ``Wp`` given the Cholesky factor ``U``; ``scales`` is [rows] (one clip
     candidate) or [candidates, rows], which gives codes [candidates, rows, cols] from one launch."""

@@ -33,16 +33,28 @@ def damp_hessian(H: torch.Tensor, damping: float = 0.01) -> torch.Tensor:
 
 def gptq_prepare(H: torch.Tensor, damping: float = 0.01):
     """Return (perm, inv_perm, U) with ``U`` the upper Cholesky factor of ``inv(H[perm][:, perm])``."""
-    Hd = damp_hessian(H, damping)
+    perm, inv_perm, U, check = _prepare(H, damping)
+    check()
+    return perm, inv_perm, U
+
+
+def _prepare(H: torch.Tensor, damping: float):
+    """`gptq_prepare` and a function that raises if ``H`` was not positive definite: it waits for the device, so it is called last."""
+    Hd = damp_hessian(H, damping).contiguous()
     perm = torch.argsort(torch.diagonal(Hd), descending=True)
     # inv(H) = U^T U with U upper means H = R R^T with R = inv(U) upper, and R is the Cholesky factor of H with its rows and
     # columns in reverse order, reversed back. So one factorisation and one triangular inverse give the (unique) factor; neither
     # inv(H) nor its own factorisation is needed.
     rev = perm.flip(0)
+    if Hd.is_cuda:
+        from ..ops import native
+        U, info = native.gptq_factor(Hd, rev)
+        inv_perm = torch.empty_like(perm).scatter_(0, perm, torch.arange(perm.numel(), device=perm.device))
+        return perm, inv_perm, U, lambda: native.gptq_factor_check(info)
     L = torch.linalg.cholesky(Hd[rev][:, rev].double())
     eye = torch.eye(L.shape[0], dtype=L.dtype, device=L.device)
     U = torch.linalg.solve_triangular(L, eye, upper=False).flip(0, 1).float()
-    return perm, torch.argsort(perm), U
+    return perm, torch.argsort(perm), U, lambda: None
 
 
 def gptq_rows_torch(Wp: torch.Tensor, U: torch.Tensor, scales: torch.Tensor, bits: int, block: int = 128) -> torch.Tensor:
@@ -75,7 +87,7 @@ def gptq_quantize(W: torch.Tensor, H: torch.Tensor, bits: int = 6, block: int = 
     W = W.float()
     rows, cols = W.shape
     qmin, qmax = qrange(bits)
-    perm, inv_perm, U = gptq_prepare(H.to(W.device), damping)
+    perm, inv_perm, U, check = _prepare(H.to(W.device), damping)
     Wp = W[:, perm].contiguous()
     srt = W.abs().sort(dim=1).values
     native_rows = None
@@ -85,11 +97,9 @@ def gptq_quantize(W: torch.Tensor, H: torch.Tensor, bits: int = 6, block: int = 
             rows_fn = native_rows = native.gptq_rows
         else:
             rows_fn = gptq_rows_torch
-    scales = []
-    for p in CLIP_PERCENTILES:
-        idx = min(int(cols * p), cols - 1)
-        scale = (srt[:, idx].clamp_min(1e-8) / qmax).clamp_min(1e-8)
-        scales.append(scale.half().float().clamp_min(6e-8))   # what de-quantisation will multiply by
+    S = torch.stack([srt[:, min(int(cols * p), cols - 1)] for p in CLIP_PERCENTILES])
+    S = (S.clamp_min(1e-8) / qmax).clamp_min(1e-8).half().float().clamp_min(6e-8)         # what de-quantisation will multiply by
+    scales = list(S.unbind(0))
     best_err = torch.full((rows,), float("inf"), device=W.device)
     best_q = torch.zeros_like(Wp, dtype=torch.int8)
     best_s = torch.ones(rows, device=W.device)
@@ -97,7 +107,6 @@ def gptq_quantize(W: torch.Tensor, H: torch.Tensor, bits: int = 6, block: int = 
     # takes 0.85 ms instead of five times 0.20. Fewer rows keep a launch per candidate, which is slower than one would be (five
     # chains one after the other): the number of launches of such a call is part of its tests. The first of the least errors wins.
     if native_rows is not None and rows * len(scales) > 4 * torch.cuda.get_device_properties(W.device).multi_processor_count:
-        S = torch.stack(scales)
         Q = native_rows(Wp, U, S, bits, block)
         err = torch.empty_like(S)
         step = max(1, (1 << 23) // (len(scales) * cols))      # the fp32 temporaries of the error pass stay at 100 MB
@@ -111,6 +120,7 @@ def gptq_quantize(W: torch.Tensor, H: torch.Tensor, bits: int = 6, block: int = 
         found = best_err < float("inf")
         best_s = torch.where(found, S.gather(0, k[None])[0], best_s)
         best_q = torch.where(found[:, None], Q[k, torch.arange(rows, device=W.device)], best_q)
+        check()
         return best_q[:, inv_perm].contiguous(), best_s
     for scale in scales:
         Q = rows_fn(Wp, U, scale, bits, block)
@@ -119,6 +129,7 @@ def gptq_quantize(W: torch.Tensor, H: torch.Tensor, bits: int = 6, block: int = 
         best_err = torch.where(better, err, best_err)
         best_s = torch.where(better, scale, best_s)
         best_q = torch.where(better[:, None], Q, best_q)
+    check()
     return best_q[:, inv_perm].contiguous(), best_s
 
 

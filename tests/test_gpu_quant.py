@@ -151,3 +151,29 @@ def test_gptq_of_all_candidates_at_once_needs_no_more_memory_than_one_at_a_time(
     assert same.float().mean() >= 0.999 and torch.equal(q0[same], q1[same])
     if rows > 1000:
         assert peak[1] <= peak[0], peak
+
+
+@pytest.mark.parametrize("c", [1, 63, 64, 65, 130, 200, 513])
+def test_gptq_factor_around_its_tiles(c):
+    """The factor from the kernel against fp64 torch, at sizes around the 64-column tiles: both are fp64 sums rounded to fp32 once, so they
+    may differ by an ulp where a rounding is close."""
+    from parameter_golf_b200.quant.gptq import damp_hessian, gptq_prepare
+    x = torch.randn(2 * c, c, device="cuda", generator=torch.Generator(device="cuda").manual_seed(c)) * torch.linspace(0.3, 2.0, c, device="cuda")
+    H = x.t() @ x / (2 * c)
+    perm, inv_perm, U = gptq_prepare(H)
+    Hp = damp_hessian(H)[perm][:, perm].double()
+    want = torch.linalg.cholesky(torch.linalg.inv(Hp), upper=True)
+    assert (U.double() - want).norm() <= 1e-6 * want.norm()
+    assert torch.equal(U, U.triu()) and torch.equal(perm[inv_perm], torch.arange(c, device="cuda"))
+
+
+@pytest.mark.parametrize("c,bad", [(5, 2), (100, 70)])
+def test_gptq_factor_refuses_what_is_not_positive_definite(c, bad):
+    from parameter_golf_b200.quant.gptq import gptq_prepare, gptq_quantize
+    for value in (-3.0, float("nan")):
+        H = torch.eye(c, device="cuda")
+        H[bad, bad] = value
+        with pytest.raises(torch.linalg.LinAlgError, match="not positive-definite"):
+            gptq_prepare(H)
+        with pytest.raises(torch.linalg.LinAlgError, match="not positive-definite"):
+            gptq_quantize(torch.randn(3, c, device="cuda"), H)
