@@ -29,7 +29,7 @@ void gemm(torch::Tensor A, torch::Tensor B, torch::Tensor D, bool a_kmajor, bool
           double slope, c10::optional<torch::Tensor> aux, c10::optional<torch::Tensor> colscale, c10::optional<torch::Tensor> D2,
           int64_t splits, c10::optional<torch::Tensor> status, c10::optional<torch::Tensor> wait_flag, int64_t wait_value,
           int64_t seg_row0, c10::optional<torch::Tensor> seg_D0, int64_t seg_row1, c10::optional<torch::Tensor> seg_D1,
-          c10::optional<torch::Tensor> batch_sumsq, int64_t sumsq_pow, int64_t tile_n, int64_t chain_rows) {
+          c10::optional<torch::Tensor> batch_sumsq, int64_t sumsq_pow, int64_t tile_n, int64_t chain_rows, c10::optional<torch::Tensor> row_part) {
   check_bf16(A, "A");
   check_bf16(B, "B");
   TORCH_CHECK(A.dim() == B.dim() && A.dim() == D.dim() && (A.dim() == 2 || A.dim() == 3), "gemm: operands must all be 2-D or all 3-D");
@@ -115,6 +115,12 @@ void gemm(torch::Tensor A, torch::Tensor B, torch::Tensor D, bool a_kmajor, bool
                 "gemm: batch_sumsq must be fp32[batch] (power 1 or 2) with a bf16 epilogue");
     g.batch_sumsq = batch_sumsq->data_ptr<float>();
     g.sumsq_pow = (int)sumsq_pow;
+  }
+  if (row_part.has_value()) {
+    TORCH_CHECK(row_part->is_cuda() && row_part->scalar_type() == torch::kFloat32 && row_part->is_contiguous() && row_part->dim() == 2 &&
+                    row_part->size(0) == g.N / 64 && row_part->size(1) == g.M,
+                "gemm: row_part must be a contiguous fp32 CUDA tensor [N / 64, M]");
+    g.row_part = row_part->data_ptr<float>();
   }
   pgb::gemm_bf16(g, cur_stream());
 }

@@ -63,6 +63,10 @@ struct GemmKernelParams {
   int q_heads, qk_heads, rope_half, seq_len;
   float norm_eps;
   uint32_t* signs;            // EPI_ACT_SQ_SIGN, EPI_MUL_ACTROOT
+  float* row_part;            // EPI_AXPBY_BF16: sums of squares out; EPI_ACT_SQ_SIGN: in (norm_parts per row)
+  float* row_factor;          // EPI_ACT_SQ_SIGN: out; EPI_MUL_ACTROOT: in
+  int norm_parts;
+  float norm_scale;
 };
 
 constexpr int STG_PITCH = 64;
@@ -206,7 +210,7 @@ __device__ __forceinline__ int stg_off(int row, int piece) { return row * STG_PI
 // Outputs of one chunk: this thread's row of 32 values, packed. `ax` is the row of the second operand, `sg` its sign word.
 template <int EPI>
 __device__ __forceinline__ void epilogue_math(const GemmKernelParams& p, float alpha, float beta, int m_base, int lane, int n0, const uint32_t (&r)[32],
-                                              const uint32_t (&ax)[16], uint32_t sg, uint32_t (&pk)[16], uint32_t (&pk2)[16]) {
+                                              const uint32_t (&ax)[16], uint32_t sg, float rf, uint32_t (&pk)[16], uint32_t (&pk2)[16]) {
   float a[32];
   if constexpr (epi_has_aux(EPI)) {
 #pragma unroll
@@ -236,8 +240,8 @@ __device__ __forceinline__ void epilogue_math(const GemmKernelParams& p, float a
 #pragma unroll
     for (int i = 0; i < 32; i += 2) {
       const float2 t = unpack_bf16x2(pack_bf16x2(sqrt_approx(a[i]), sqrt_approx(a[i + 1])));
-      o[i] = __uint_as_float(r[i]) * (t.x * ((sg >> i) & 1u ? neg : pos));
-      o[i + 1] = __uint_as_float(r[i + 1]) * (t.y * ((sg >> (i + 1)) & 1u ? neg : pos));
+      o[i] = __uint_as_float(r[i]) * rf * (t.x * ((sg >> i) & 1u ? neg : pos));
+      o[i + 1] = __uint_as_float(r[i + 1]) * rf * (t.y * ((sg >> (i + 1)) & 1u ? neg : pos));
     }
   }
 #pragma unroll
@@ -257,7 +261,7 @@ __device__ __forceinline__ void epilogue_math(const GemmKernelParams& p, float a
     const __nv_bfloat162 sl = __float2bfloat162_rn(p.slope);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const __nv_bfloat162 hb = __floats2bfloat162_rn(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+      const __nv_bfloat162 hb = __floats2bfloat162_rn(__uint_as_float(r[2 * i]) * rf, __uint_as_float(r[2 * i + 1]) * rf);
       const __nv_bfloat162 t = __hmax2(hb, __hmul2(hb, sl));
       const __nv_bfloat162 sq = __hmul2(t, t);
       pk[i] = *reinterpret_cast<const uint32_t*>(&sq);
@@ -265,7 +269,7 @@ __device__ __forceinline__ void epilogue_math(const GemmKernelParams& p, float a
     if (p.signs != nullptr) {
       uint32_t w = 0;
 #pragma unroll
-      for (int i = 31; i >= 0; --i) w = __funnelshift_l(r[i], w, 1);       // rounding to bf16 keeps the sign
+      for (int i = 31; i >= 0; --i) w = __funnelshift_l(r[i], w, 1);       // the factor and rounding to bf16 keep the sign
       if (m_base + lane < p.M) p.signs[(size_t)(n0 >> 5) * p.M + m_base + lane] = w;
     }
   }
@@ -605,7 +609,38 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         cp_async_commit();          // one group per chunk, also when nothing was copied: the wait below counts groups
       }
     };
-    static_assert(CH % 2 == 0, "slot parity follows the chunk index within the tile");
+    static_assert(CH % 2 == 0, "slot parity and the halves of a 64-column sum of squares follow the chunk index within the tile");
+    // The factor of this thread's row. For the next tile it is asked for before the last chunk of this one and used after it.
+    constexpr bool ROW_FACTOR = EPI == EPI_ACT_SQ_SIGN || EPI == EPI_MUL_ACTROOT;
+    constexpr int PARTS = EPI == EPI_ACT_SQ_SIGN ? 8 : 1;       // read in one go; wider rows are summed in further rounds
+    auto ask_factor = [&](int m, float (&q)[PARTS]) {
+      if constexpr (ROW_FACTOR) {
+        const int mm = min(m, p.M - 1);
+        if constexpr (EPI == EPI_MUL_ACTROOT) q[0] = p.row_factor ? __ldcg(p.row_factor + mm) : 1.f;
+        else if (p.row_part) {
+#pragma unroll
+          for (int k = 0; k < PARTS; ++k) q[k] = k < p.norm_parts ? __ldcg(p.row_part + (size_t)k * p.M + mm) : 0.f;
+        }
+      }
+    };
+    auto take_factor = [&](int m, const float (&q)[PARTS]) {
+      if constexpr (EPI == EPI_MUL_ACTROOT) return q[0];
+      if (!ROW_FACTOR || !p.row_part) return 1.f;
+      float s = 0.f;
+#pragma unroll
+      for (int k = 0; k < PARTS; ++k) s += q[k];
+      for (int k = PARTS; k < p.norm_parts; ++k) s += __ldcg(p.row_part + (size_t)k * p.M + min(m, p.M - 1));
+      return p.norm_scale * rsqrtf(s / p.K + p.norm_eps);
+    };
+    float asked[PARTS] = {};
+    if constexpr (ROW_FACTOR) {
+      if (first_tile < total_tiles) {
+        int b0, tm0, tn0;
+        tile_coords(first_tile, b0, tm0, tn0);
+        ask_factor(tm0 * TILE_M + rank * BM + quarter * 32 + lane, asked);
+      }
+    }
+    float sumsq = 0.f;                            // of this thread's row in the 64 columns under way (AXPBY with `row_part`)
     if (aux_async && first_tile < total_tiles) {
       int b0, tm0, tn0;
       tile_coords(first_tile, b0, tm0, tn0);
@@ -627,6 +662,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const float f = p.sumsq_pow == 2 ? inv * inv : inv;
         alpha *= f;
         beta *= f;
+      }
+      const float rf = take_factor(m, asked);
+      if constexpr (EPI == EPI_ACT_SQ_SIGN) {
+        if (p.row_factor && tn == 0 && half == 0 && m < p.M) p.row_factor[m] = rf;
       }
       if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, p.status, ST_WAIT_TMEM_FULL, tile)) { ok = false; break; }
       tc_fence_after();
@@ -650,6 +689,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       for (int cc = 0; cc < CH; ++cc) {
         const int c = c_begin + cc;
         const int n0 = tn * BN + c * 32;
+        if constexpr (ROW_FACTOR) {
+          if (cc == CH - 1 && next < total_tiles) ask_factor(ntm * TILE_M + rank * BM + quarter * 32 + lane, asked);
+        }
         if (n0 < p.N) {                           // warp-uniform
           uint32_t rr[32];
           PGB_TMEM_LD32(taddr + c * 32, rr);
@@ -675,7 +717,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if constexpr (EPI == EPI_MUL_ACTROOT) {
                   if (p.signs != nullptr) sg = *reinterpret_cast<const uint32_t*>(sgn + (cc & 1) * SGN_BYTES + lane * 4);
                 }
-                epilogue_math<EPI>(p, alpha, beta, m_base, lane, n0, rr, ax, sg, pk, pk2);
+                epilogue_math<EPI>(p, alpha, beta, m_base, lane, n0, rr, ax, sg, rf, pk, pk2);
+                if constexpr (EPI == EPI_AXPBY_BF16) {
+                  if (p.row_part) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                      const float2 f = unpack_bf16x2(pk[i]);
+                      sumsq = fmaf(f.x, f.x, fmaf(f.y, f.y, sumsq));
+                    }
+                    if (cc & 1) {
+                      if (m < p.M) p.row_part[(size_t)(n0 >> 6) * p.M + m] = sumsq;
+                      sumsq = 0.f;
+                    }
+                  }
+                }
                 fill(slot, pk);
                 __syncwarp();
                 __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + (long long)b * p.stride_d + n0 + (lane & 3) * 8;
@@ -685,7 +740,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                   if (m_base + lr < p.M) *reinterpret_cast<uint4*>(d + (long long)(m_base + lr) * p.ldd) = *reinterpret_cast<const uint4*>(slot + stg_off(lr, lane & 3));
                 }
               } else {
-                epilogue_math<EPI>(p, alpha, beta, m_base, lane, n0, rr, ax, sg, pk, pk2);
+                epilogue_math<EPI>(p, alpha, beta, m_base, lane, n0, rr, ax, sg, rf, pk, pk2);
                 put(pk, 0, b, m_base, n0);
                 if constexpr (EPI == EPI_ACT_SQ) put(pk2, 1, b, m_base, n0);
               }
@@ -907,6 +962,13 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   p.seq_len = a.seq_len;
   p.norm_eps = a.norm_eps;
   p.signs = a.signs;
+  p.row_part = a.epi == EPI_ACT_SQ_SIGN ? const_cast<float*>(a.norm_part) : a.row_part;
+  p.row_factor = a.row_factor;
+  p.norm_parts = a.K / 64;
+  p.norm_scale = a.norm_scale;
+  if ((a.row_part && (a.epi != EPI_AXPBY_BF16 || a.N % 64 || a.batch != 1)) || (a.norm_part && (a.epi != EPI_ACT_SQ_SIGN || a.K % 64)) ||
+      (a.row_factor && !(a.epi == EPI_MUL_ACTROOT || (a.epi == EPI_ACT_SQ_SIGN && a.norm_part))))
+    throw std::runtime_error("gemm: row sums and factors go with un-batched products of a multiple of 64 columns and their own epilogues");
   if (a.epi == EPI_ACT_SQ_SIGN || a.epi == EPI_MUL_ACTROOT) {
     int e = 0;
     const bool slope_ok = a.slope == 0.f || (a.slope > 0.f && a.slope < 1.f && std::frexp(a.slope, &e) == 0.5f);
@@ -931,6 +993,7 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   };
   const bool aux = a.aux != nullptr && epi_has_aux(a.epi), two = a.D2 != nullptr && (a.epi == EPI_ACT_SQ || a.epi == EPI_QKV_NORM_ROPE);
   p.aligned = rows_ok(a.D, a.ldd, a.stride_d) && (!two || rows_ok(a.D2, a.ldd, a.stride_d)) && (!aux || rows_ok(a.aux, a.ld_aux, a.stride_aux));
+  if (a.row_part && !p.aligned) throw std::runtime_error("gemm: row sums need 16-byte aligned rows");
   const bool stores = p.aligned && !aux && a.epi != EPI_F32 && a.epi != EPI_F32_ATOMIC;
   m.d = stores ? chunk_map(a.D, a, a.ldd, a.stride_d) : m.a;
   m.d2 = stores && two ? chunk_map(a.D2, a, a.ldd, a.stride_d) : m.a;

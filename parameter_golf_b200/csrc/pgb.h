@@ -60,6 +60,14 @@ struct GemmArgs {
   // EPI_ACT_SQ_SIGN / EPI_MUL_ACTROOT: [N / 32][M] words, bit i of word (c, m) = sign of h[m][32 c + i]. May be null where nobody
   // reads them (a forward without a backward) or, with slope 0, where they make no difference. The slope is 0 or a power of two below 1.
   uint32_t* signs = nullptr;
+  // RMSNorm without a pass of its own. A product with an AXPBY epilogue can leave the sums of squares of its (rounded) outputs in `row_part`
+  // ([N / 64][M], one per row and 64 columns, summed in a fixed order whatever the tile). EPI_ACT_SQ_SIGN, given those of its own A in
+  // `norm_part` ([K / 64][M]), multiplies its row m by f = norm_scale / sqrt(sum / K + norm_eps), which is the product of the normed row, and
+  // writes f to `row_factor` [M] (optional); EPI_MUL_ACTROOT multiplies its row m by row_factor[m] (optional).
+  float* row_part = nullptr;
+  const float* norm_part = nullptr;
+  float norm_scale = 1.f;
+  float* row_factor = nullptr;
 };
 
 void gemm_bf16(const GemmArgs& args, cudaStream_t stream);
@@ -67,6 +75,7 @@ void gemm_bf16(const GemmArgs& args, cudaStream_t stream);
 // ---- row kernels (rowops.cu); activations bf16, parameters fp32 ------------------------------------------------
 void mix_norm_fwd(const void* x, const void* x0, const void* skip, const float* sw, const float* mix, void* x_in, void* h, int rows, int d, float s,
                   float eps, cudaStream_t st);
+// s < 0: d_h already carries the forward's row factor s / rms (see GemmArgs::row_factor)
 void mix_norm_bwd(const void* d_h, const void* d_res, const void* x_in, const void* x, const void* x0, const void* skip, const float* sw,
                   const float* mix, const void* add_grad, void* d_x, void* d_x0, void* d_skip, float* d_mix, float* d_sw, int skip_to_dx, int rows,
                   int d, float s, float eps, cudaStream_t st);

@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(ROW_THREADS) mix_norm_bwd_kernel(const __nv_bf
     dot = warp_sum(dot);
     const float ms = ss / d + eps;
     const float inv = rsqrtf(ms);
-    const float k1 = s * inv, k2 = dot / (ms * d);
+    const float k1 = s < 0.f ? 1.f : s * inv, k2 = dot / (ms * d);
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int c = (j * 32 + lane) * 8;

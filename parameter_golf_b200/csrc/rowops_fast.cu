@@ -117,7 +117,7 @@ mix_norm_bwd2_kernel(const __nv_bfloat16* d_h, const __nv_bfloat16* d_res, const
     ss = warp_sum(ss);
     dot = warp_sum(dot);
     const float ms = ss / d + eps;
-    const float k1 = s * rsqrtf(ms), k2 = dot / (ms * d);
+    const float k1 = s < 0.f ? 1.f : s * rsqrtf(ms), k2 = dot / (ms * d);
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       const int c = (j * 32 + lane) * 8;

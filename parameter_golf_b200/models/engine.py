@@ -88,6 +88,10 @@ class CudaEngine:
         self.slope = m.leaky_slope if m.activation == "leaky_relu_sq" else 0.0
         # the backward can take the pre-activation from the activation's root and a sign bit (none needed for relu^2)
         self.act_root = N.act_root_supported(self.slope)
+        # The norm in front of the MLP has no pass of its own: the output projection leaves the sums of squares of its rows, the up
+        # projection runs on the un-normed rows and multiplies its outputs by the row's factor, and so does the activation gradient
+        # (whose rows are what both the weight gradient and the input gradient take).
+        self.fold_norm = self.act_root and not m.parallel
         self.enc = self.n // 2
         self.sched = gpt.layer_schedule(m)                     # (layer, pass) per activation slot
         self.nslots = len(self.sched)
@@ -316,7 +320,10 @@ class CudaEngine:
         self.k_cols = [t[:, d:d + self.kv] for t in self.qk_post]
         self.v_cols = [t[:, d + self.kv:] for t in self.qkv_pre]
         self.y, self.x_mid = per_layer(T, d), per_layer(T, d)
-        self.mm = self.h if self.parallel else per_layer(T, d)      # parallel residual: the MLP reads the attention branch's normed input
+        # what the MLP reads: the un-normed residual, in a parallel residual the attention branch's normed input, else a normed copy
+        self.mm = self.x_mid if self.fold_norm else self.h if self.parallel else per_layer(T, d)
+        self.row_part = buf(d // 64, T, dtype=torch.float32) if self.fold_norm else None
+        self.row_factor = [buf(T, dtype=torch.float32) for _ in range(L)] if self.fold_norm else [None] * L
         xsa_sets = {self.act_slot[j] for j, (l, _) in enumerate(self.sched) if l in m.xsa_layers()} if self.train else ({0} if m.xsa_last_n > 0 else set())
         self.z = [buf(T, d) if i in xsa_sets else None for i in range(L)]
         self.yg = [[buf(T, d) for _ in range(L)] for _ in self.gates]          # gated attention outputs, one list per gate
@@ -568,11 +575,12 @@ class CudaEngine:
             C.head_gate_fwd(zz, self.h[li], p[wname][l], p[bname][l] if bname else None, out, self.gv[gi][li], self.H, self.hd, gscale_, gmult)
             zz = out
         self.zz[li] = zz
-        self.gemm(zz, Wo, self.x_mid[li], epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_in[li])
-        if not self.parallel:
+        self.gemm(zz, Wo, self.x_mid[li], epi=N.EPI_AXPBY_BF16, alpha=1.0, beta=1.0, aux=self.x_in[li], row_part=self.row_part)
+        if not self.parallel and not self.fold_norm:
             C.mix_norm_fwd(self.x_mid[li], None, None, None, None, None, self.mm[li], s_l, self.eps)
         if self.act_root:
-            C.gemm_act(self.mm[li], Wup, self.a[li], self.signs[li] if self.want_grad else None, self.slope, N.status_word(self.dev), self.T)
+            C.gemm_act(self.mm[li], Wup, self.a[li], self.signs[li] if self.want_grad else None, self.slope, N.status_word(self.dev), self.T, 0,
+                       self.row_part, s_l, self.eps, self.row_factor[li])
         else:
             self.gemm(self.mm[li], Wup, self.hu[li], epi=N.EPI_ACT_SQ, slope=self.slope, D2=self.a[li])
         xo = self.x_out[j]
@@ -691,7 +699,7 @@ class CudaEngine:
             if self._wants("mlp_down_bank", "mlp_scale"):
                 self._dw_folded(self.dx, self.a[aj], self.Gd, C.fold_scaled_grad_bf16, *view["down"])
             if self.act_root:
-                C.gemm_actgrad(self.dx, Wd, self.d_hu, self.a[aj], self.signs[aj], self.slope, N.status_word(self.dev), self.T)
+                C.gemm_actgrad(self.dx, Wd, self.d_hu, self.a[aj], self.signs[aj], self.slope, N.status_word(self.dev), self.T, 0, self.row_factor[aj])
             else:
                 self.gemm(self.dx, Wd, self.d_hu, True, False, N.EPI_MUL_ACTGRAD, slope=self.slope, aux=self.hu[aj])
             if self._wants("mlp_up_bank"):
@@ -701,7 +709,8 @@ class CudaEngine:
                 dx_mid, dx_next = self.dx, self.dx_mid      # no norm between x_mid and the MLP: the residual gradient passes through
                 d_hx = self.d_m                             # and the MLP-input gradient joins the QKV-input gradient below
             else:
-                C.mix_norm_bwd(self.d_m, self.dx, self.x_mid[aj], None, None, None, None, None, None, self.dx_mid, None, None, None, None, False, s_l, self.eps)
+                C.mix_norm_bwd(self.d_m, self.dx, self.x_mid[aj], None, None, None, None, None, None, self.dx_mid, None, None, None, None, False,
+                               -1.0 if self.fold_norm else s_l, self.eps)
                 dx_mid, dx_next = self.dx_mid, self.dx
                 d_hx = self.d_hx if self.gates else None
             # ---- attention output projection

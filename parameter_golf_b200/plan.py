@@ -188,16 +188,18 @@ def estimate_engine_memory(spec: RunSpec, micro_batch_tokens: int, train: bool =
         saved = saved_slots(sched, t.save_layer_acts)
         nact = sum(saved) + (0 if all(saved) else 1)
     gates = int(m.attn_out_gate.enabled) + int(m.sparse_attn_gate.enabled)
-    # per activation set: x_in, h, y, x_mid (+ mm unless parallel residual), qkv_pre, qk_post, a, lse, gate outputs, and for the
+    # per activation set: x_in, h, y, x_mid (+ mm, see below), qkv_pre, qk_post, a, lse, gate outputs, and for the
     # activation's backward one sign bit per value (none for relu^2) or, with a slope that is no power of two, the pre-activation
     slope = m.leaky_slope if m.activation == "leaky_relu_sq" else 0.0
-    per_set = 2 * T * d * (4 + (0 if m.parallel else 1)) + 2 * 2 * T * qkvw + 2 * T * mlp + 4 * T * H
+    # per activation set the norm in front of the MLP has either a normed copy or one factor per row
+    fold_norm = act_root_supported(slope) and not m.parallel
+    per_set = 2 * T * d * (4 + (0 if m.parallel or fold_norm else 1)) + 2 * 2 * T * qkvw + 2 * T * mlp + 4 * T * H + (4 * T if fold_norm else 0)
     if not act_root_supported(slope):
         per_set += 2 * T * mlp
     elif slope > 0 and train:
         per_set += T * mlp // 8
     per_set += gates * (2 * T * d + 4 * T * H)
-    act = nact * per_set
+    act = nact * per_set + (4 * T * (d // 64) if fold_norm else 0)
     if train:
         xsa_sets = {(j if saved[j] else -1) for j, (l, _) in enumerate(sched) if l in m.xsa_layers()}
         act += len(xsa_sets) * 2 * T * d
