@@ -79,6 +79,11 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 constexpr int A1_THREADS = 256;
 constexpr int A1_KST = 2, A1_VST = 2;
 constexpr int A1_SMEM = (2 + A1_KST + A1_VST) * AT_TILE_BYTES + 1024 + 256;
+// Shared memory asked for when there are no more items than SMs: more than half of an SM's, so that every CTA gets an SM for itself. A
+// kernel that starts before its predecessor has finished would otherwise put two CTAs on each SM that is free first, where both run
+// slower: one sequence of 2,048 took 31 us in a chain and 23.5 alone.
+constexpr int A1_SMEM_ALONE = 120 * 1024;
+static_assert(A1_SMEM_ALONE >= A1_SMEM && 2 * (A1_SMEM_ALONE + 1024) > 228 * 1024, "one CTA per SM");
 // Register budget: 2 CTAs x 256 threads => 128 registers per thread at launch. `setmaxnreg.inc` can only take what the
 // role warps released; a request for more never completes, so the two sides must balance exactly.
 constexpr int A1_REG_LAUNCH = 128, A1_REG_ROLE = 40, A1_REG_SOFTMAX = 216;
@@ -508,7 +513,7 @@ void attn_fwd(const void* q, const void* k, const void* v, void* y, float* lse, 
   cudaGetDevice(&dev);
   const bool cached = dev >= 0 && dev < 64;
   if (!cached || !configured[dev]) {
-    cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, A1_SMEM);
+    cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, A1_SMEM_ALONE);
     cudaFuncAttributes fa;
     // the register hand-over inside the kernel is balanced for exactly this launch allocation; anything else would never complete
     if (cudaFuncGetAttributes(&fa, attn_fwd_kernel) != cudaSuccess || fa.numRegs != A1_REG_LAUNCH)
@@ -526,8 +531,8 @@ void attn_fwd(const void* q, const void* k, const void* v, void* y, float* lse, 
     }
   }
   p.sched = base + 2 * (sched_next.fetch_add(1, std::memory_order_relaxed) % A1_SCHED_SLOTS);
-  const int grid = std::min(p.n_qt * B * H, 2 * sms);
-  launch_chained(T, attn_fwd_kernel, grid, A1_THREADS, A1_SMEM, st, mq, mk, mv, p);
+  const int items = p.n_qt * B * H, grid = std::min(items, 2 * sms);
+  launch_chained(T, attn_fwd_kernel, grid, A1_THREADS, items <= sms ? A1_SMEM_ALONE : A1_SMEM, st, mq, mk, mv, p);
 }
 
 }  // namespace pgb
