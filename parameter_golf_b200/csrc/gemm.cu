@@ -60,7 +60,7 @@ struct GemmKernelParams {
   const float* rope_cos;      // EPI_QKV_NORM_ROPE
   const float* rope_sin;
   const float* head_gain;
-  int q_heads, qk_heads, rope_half, seq_len;
+  int q_heads, qk_heads, rope_half, seq_len, raw_qk;
   float norm_eps;
   uint32_t* signs;            // EPI_ACT_SQ_SIGN, EPI_MUL_ACTROOT
   float* row_part;            // EPI_AXPBY_BF16: sums of squares out; EPI_ACT_SQ_SIGN: in (norm_parts per row)
@@ -340,9 +340,11 @@ __device__ __forceinline__ void epilogue_qkv_head(const GemmKernelParams& p, int
     pk[i] = pack_bf16x2(__uint_as_float(ra[2 * i]) * p.alpha, __uint_as_float(ra[2 * i + 1]) * p.alpha);
     pk[16 + i] = pack_bf16x2(__uint_as_float(rb[2 * i]) * p.alpha, __uint_as_float(rb[2 * i + 1]) * p.alpha);
   }
-  put(pk, 0, n0);
-  put(pk + 16, 0, n0 + 32);
   const int head = n0 >> 6;
+  if (p.raw_qk || head >= p.qk_heads) {
+    put(pk, 0, n0);
+    put(pk + 16, 0, n0 + 32);
+  }
   if (head >= p.qk_heads) return;                  // value heads: the projection as it is (warp-uniform)
   float x[64];
   float ss = 0.f;
@@ -960,6 +962,7 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   p.qk_heads = a.q_heads + a.kv_heads;
   p.rope_half = a.rope_dims / 2;
   p.seq_len = a.seq_len;
+  p.raw_qk = a.raw_qk;
   p.norm_eps = a.norm_eps;
   p.signs = a.signs;
   p.row_part = a.epi == EPI_ACT_SQ_SIGN ? const_cast<float*>(a.norm_part) : a.row_part;

@@ -56,6 +56,7 @@ struct GemmArgs {
   const float* rope_sin = nullptr;
   const float* head_gain = nullptr;
   int q_heads = 0, kv_heads = 0, rope_dims = 0, seq_len = 0;
+  bool raw_qk = true;        // false: the raw query and key heads are not written (nothing but a backward reads them)
   float norm_eps = 0.f;
   // EPI_ACT_SQ_SIGN / EPI_MUL_ACTROOT: [N / 32][M] words, bit i of word (c, m) = sign of h[m][32 c + i]. May be null where nobody
   // reads them (a forward without a backward) or, with slope 0, where they make no difference. The slope is 0 or a power of two below 1.

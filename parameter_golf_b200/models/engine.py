@@ -557,7 +557,7 @@ class CudaEngine:
             wait = dict(wait_flag=self.layer_flags[l:l + 1], wait_value=self.layer_flag_value)
         if fused_qk:
             N.gemm_qkv_norm_rope(self.h[li], Wqkv, self.qkv_pre[li], self.qk_post[li], self.cos, self.sin, gain, self.H, self.Hkv,
-                                 m.rope_dims, S, self.eps, **wait)
+                                 m.rope_dims, S, self.eps, raw_qk=self.want_grad, **wait)
         else:
             self.gemm(self.h[li], Wqkv, self.qkv_pre[li], **wait)
         if m.value_embedding.enabled and l in m.value_embedding.layers:

@@ -162,11 +162,12 @@ def gemm(A, B, D, a_kmajor=True, b_kmajor=True, epi=EPI_BF16, alpha=1.0, beta=0.
     return D
 
 
-def gemm_qkv_norm_rope(h, W, pre, post, cos, sin, gain, H, Hkv, rope_dims, seq_len, eps, wait_flag=None, wait_value=0):
+def gemm_qkv_norm_rope(h, W, pre, post, cos, sin, gain, H, Hkv, rope_dims, seq_len, eps, wait_flag=None, wait_value=0, raw_qk=True):
     """QKV projection whose output stage also applies the per-head RMSNorm, the partial RoPE and the query gain: ``pre`` = h W^T
     for all heads (the backward of the norm and the attention read it), ``post`` = the normalised, rotated, gain-scaled query
-    and key heads. Heads of 64; ``rope_dims`` in {0, 16, 32, 64}."""
-    load().gemm_qkv_norm_rope(h, W, pre, post, cos, sin, gain, H, Hkv, rope_dims, seq_len, eps, status_word(h.device), wait_flag, wait_value)
+    and key heads. Heads of 64; ``rope_dims`` in {0, 16, 32, 64}. ``raw_qk=False`` leaves the query and key columns of ``pre`` alone, which
+    only a backward reads."""
+    load().gemm_qkv_norm_rope(h, W, pre, post, cos, sin, gain, H, Hkv, rope_dims, seq_len, eps, status_word(h.device), wait_flag, wait_value, raw_qk)
     return post
 
 

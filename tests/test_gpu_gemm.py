@@ -213,6 +213,25 @@ def test_every_tile_width_gives_the_same_product(tile_n, M, N, K):
             n.gemm(A, W, torch.empty(M, N, device="cuda"), epi=n.EPI_F32, tile_n=64)
 
 
+@pytest.mark.parametrize("B,S", [(1, 128), (3, 640)])
+def test_qkv_product_without_the_raw_heads(B, S):
+    """What a forward without a backward leaves out is only the raw query and key columns."""
+    n = _n()
+    from parameter_golf_b200.ops import reference as R
+    H, Hkv, d, T = 8, 4, 512, B * S
+    h, W = _rand(T, d), _rand((H + 2 * Hkv) * 64, d, scale=d ** -0.5)
+    cos, sin = (t.contiguous() for t in R.rope_tables(S, 16, 10000.0, device="cuda"))
+    out = []
+    for raw in (True, False):
+        pre, post = (torch.full((T, W.shape[0]), 9.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        n.gemm_qkv_norm_rope(h, W, pre, post, cos, sin, torch.ones(H, device="cuda"), H, Hkv, 16, S, 1e-6, raw_qk=raw)
+        out.append((pre, post))
+    n.check_status()
+    qk = (H + Hkv) * 64
+    assert torch.equal(out[0][1], out[1][1]) and torch.equal(out[0][0][:, qk:], out[1][0][:, qk:])
+    assert (out[1][0][:, :qk] == 9.0).all() and not (out[0][0][:, :qk] == 9.0).all()
+
+
 @pytest.mark.parametrize("M,N,K,batch", [(1, 256, 64, 1), (128, 264, 72, 2), (257, 512, 512, 1), (255, 320, 200, 3), (5000, 1000, 136, 1)])
 def test_tiles_of_a_cta_pair_are_those_of_one_cta(M, N, K, batch):
     """256-column tiles (two CTAs) against 128-column tiles (one): the same sums in the same order, so the same bits; all majors, second
