@@ -886,8 +886,10 @@ struct TilePlan {
 // items beyond the first costs 0.8 of that, since a main loop overlaps the epilogue before it. A pair's items are twice as tall and
 // there are half as many places for them. The constants were fitted to products of 1024 to 98,304 rows on the model's sites and order the
 // widths as measured there (us with launch, cold caches, 256 / 128 / 64 columns):
-//   M = 2048,  N = 512,  K = 512   14 / 11 / 10          M = 4096, N = 512, K = 1536   20 / 16 / 18
+//   M = 2048,  N = 1536, K = 512   14 / 12 / 14          M = 4096, N = 512, K = 1536   20 / 16 / 18
 //   M = 16384, N = 512,  K = 1536  35 / 37 / 41          M = 98304, N = 512, K = 1024  80 / 100
+// The output stages of the activation and the QKV product are longer than the plain one: with the same figure for all, 2,048 rows of the up
+// projection and 4,480 of the QKV product took pairs (one scored window 799 us, now 773; logits of 5 x 896 1,007 and 955).
 // With a second operand (AXPBY) a pair's output stage is the longer part unless the sum is long: M = 98304, N = 512: K = 512 84 / 72,
 // K = 1536 123 / 145; M = 16384, K = 512 24 / 23.
 // A narrower tile has to win by 8 %: it reads the activations from L2 more often than the model counts.
@@ -908,7 +910,9 @@ static TilePlan pick_tile(const GemmArgs& a, int kb_total, int sms) {
     if (bn == 64 && (!a.a_kmajor || a.epi == EPI_F32 || a.epi == EPI_RESID_BF16 || atomic)) continue;
     const int base = tile_count(a, bn), units = sms / tile_ctas(bn, a.epi);
     const double step = bn == 256 ? 540.0 : bn == 128 ? 285.0 : 245.0;
-    const double epi = atomic ? 52.0 * bn : bn == 256 ? (a.epi == EPI_AXPBY_BF16 ? 7500.0 : 4900.0) : bn == 128 ? 2900.0 : 2000.0;
+    const bool busy = a.epi == EPI_ACT_SQ_SIGN || a.epi == EPI_QKV_NORM_ROPE;
+    const double wide = a.epi == EPI_AXPBY_BF16 ? 7500.0 : busy ? 6000.0 : 4900.0;
+    const double epi = atomic ? 52.0 * bn : bn == 256 ? wide : bn == 128 ? 2900.0 : 2000.0;
     int last = 0;
     for (int waves : {1, 2, 3}) {
       int splits = std::max(1, a.splits);
